@@ -526,8 +526,14 @@ template <typename T> void grow(T **p, size_t &cap, size_t bytes, const char *wh
   cap = bytes;
 }
 
-// `height` rows of row_bytes, contiguous at device address `src` (256-byte
-// aligned), to `dst` at `pitch`, in the widest words that divide both.
+template <int E> void configure_decoder() {
+  check(cudaFuncSetAttribute(decode_blocks<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kDecodeWarps * kWarpSmemMax)),
+        "cudaFuncSetAttribute");
+}
+
+} // namespace
+
 void repitch(const uint8_t *src, size_t height, size_t row_bytes, void *dst, size_t pitch,
              cudaStream_t s) {
   const unsigned grid = static_cast<unsigned>(
@@ -551,14 +557,6 @@ void repitch(const uint8_t *src, size_t height, size_t row_bytes, void *dst, siz
     repitch_rows<uint8_t><<<grid, 256, 0, s>>>(src, row_bytes, d, pitch, height);
   check(cudaGetLastError(), "launching the frame copy");
 }
-
-template <int E> void configure_decoder() {
-  check(cudaFuncSetAttribute(decode_blocks<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kDecodeWarps * kWarpSmemMax)),
-        "cudaFuncSetAttribute");
-}
-
-} // namespace
 
 DeviceChunkDecoder::~DeviceChunkDecoder() {
   // the owner has drained the stream the decodes ran on; cudaFree waits

@@ -74,6 +74,12 @@ cudaError_t launch_place(const PlaceLaunch &L, cudaStream_t stream);
 cudaError_t launch_stamp_mask(void *base, int elem_bytes, const uint64_t *offsets, uint64_t n,
                               cudaStream_t s);
 
+// `height` rows of row_bytes, contiguous at device address `src` (256-byte
+// aligned), to `dst` at `pitch`, in the widest words that divide both
+// (decode.cu).
+void repitch(const uint8_t *src, size_t height, size_t row_bytes, void *dst, size_t pitch,
+             cudaStream_t s);
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
 // library needs no link against libcuda.
 void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes,
@@ -111,7 +117,10 @@ public:
   // the placement, so the two can be timed apart.
   void enqueue(int slot, cudaStream_t stream, cudaEvent_t mid = nullptr);
 
-  // Copy a host frame (row-major, height x width) into frame f of a slot.
+  // Copy a frame (row-major, height x width; host, device or managed memory)
+  // into frame f of a slot. Frames of kLinearUpload bytes and more go through
+  // a contiguous device copy that the plan keeps from the first such upload
+  // (as large as its largest frame), so uploads of one plan share a stream.
   void upload(int slot, int f, const void *host, cudaStream_t stream);
   // Copy a device frame (row-major, pitch in bytes) into frame f of a slot.
   void upload_device(int slot, int f, const void *device, size_t pitch_bytes,
@@ -148,6 +157,7 @@ private:
   };
 
   void release();
+  bool linear_copy(); // whether linear_ is there
 
   int elem_bytes_;
   std::vector<Shape> shapes_;
@@ -167,6 +177,7 @@ private:
   SignalPixel *pool_ = nullptr;
   uint32_t *pool_next_ = nullptr;
   uint32_t *block_sums_ = nullptr;
+  uint8_t *linear_ = nullptr; // upload()'s contiguous copy
 };
 
 // The cost model's task height (plan.cu) for these shapes at `wpc` warps per
