@@ -61,6 +61,8 @@ size_t g_filled_h[kMaxDevices] = {}, g_filled_w[kMaxDevices] = {};
 
 uint64_t align_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 
+uint64_t place_groups(uint64_t ntiles) { return (ntiles + kPlaceTiles - 1) / kPlaceTiles; }
+
 // Where each buffer sits in the scratch for one frame shape.
 struct Layout {
   FrameDesc frame;
@@ -68,7 +70,7 @@ struct Layout {
   uint32_t ntasks = 0, pool_cap = 0;
   int max_blocks = 0;
   uint64_t frame_at = 0, tile_count_at = 0, tile_start_at = 0, pool_at = 0, pool_next_at = 0,
-           block_sums_at = 0, arena_at = 0, out_at = 0, prefix_at = 0, count_at = 0;
+           block_sums_at = 0, arena_at = 0, out_at = 0, run_at = 0, count_at = 0;
   uint64_t arena_bytes = 0, total = 0;
 };
 
@@ -120,7 +122,6 @@ Layout plan_layout(uint64_t height, uint64_t width) {
   const uint64_t chunks =
       (cap + (kChunkRecords - kMaxStaged) - 1) / (kChunkRecords - kMaxStaged) + warps + 1;
   const uint64_t pool_records = chunks * kChunkRecords;
-  const uint64_t place_blocks = (L.ntiles + kPlaceTiles - 1) / kPlaceTiles;
   L.arena_bytes = L.pitch * L.rows * sizeof(uint16_t);
 
   uint64_t at = 0;
@@ -133,8 +134,8 @@ Layout plan_layout(uint64_t height, uint64_t width) {
   L.tile_count_at = take(L.ntiles * 4);
   L.tile_start_at = take(L.ntiles * 4);
   L.pool_next_at = take(16);
-  L.block_sums_at = take(std::max<uint64_t>(place_blocks, 1) * 4);
-  L.prefix_at = take(2 * 4);
+  L.block_sums_at = take(place_groups(L.ntiles) * 4);
+  L.run_at = take(2 * 4); // the threshold's status word
   L.count_at = take(2 * 4); // the frame's count, then the status word
   L.arena_at = take(L.arena_bytes);
   L.out_at = take(cap * sizeof(SignalPixel));
@@ -184,7 +185,7 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   auto *pool = reinterpret_cast<SignalPixel *>(base + L.pool_at);
   auto *pool_next = reinterpret_cast<uint32_t *>(base + L.pool_next_at);
   auto *block_sums = reinterpret_cast<uint32_t *>(base + L.block_sums_at);
-  auto *prefix = reinterpret_cast<uint32_t *>(base + L.prefix_at);
+  int *run_status = reinterpret_cast<int *>(base + L.run_at);
   auto *count = reinterpret_cast<uint32_t *>(base + L.count_at);
   int *status = reinterpret_cast<int *>(count + 1);
   void *arena = base + L.arena_at;
@@ -200,7 +201,8 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
         "uploading the frame descriptor");
   check(cudaMemsetAsync(tile_count, 0, L.ntiles * 4, s), "clearing tile counts");
   check(cudaMemsetAsync(pool_next, 0, 16, s), "clearing the pool cursor");
-  check(cudaMemsetAsync(count, 0, 2 * 4, s), "clearing the count and status");
+  check(cudaMemsetAsync(block_sums, 0, place_groups(L.ntiles) * 4, s), "clearing the tile sums");
+  check(cudaMemsetAsync(run_status, 0, 4, s), "clearing the status");
   // Off-frame pixels read as masked: every byte of the arena that the frame
   // does not cover is 0xFF. The layout is a function of the shape and only
   // the frame's own pixels are written below, so after a completed call with
@@ -226,10 +228,11 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   T.ntasks = L.ntasks;
   T.tile_count = tile_count;
   T.tile_start = tile_start;
+  T.block_sums = block_sums;
   T.pool = pool;
   T.pool_next = pool_next;
   T.pool_cap = L.pool_cap;
-  T.status = status;
+  T.status = run_status;
   T.wait_limit = 1u << 22;
   T.warps_per_block = kWarpsPerBlock;
   T.max_blocks = L.max_blocks;
@@ -238,14 +241,16 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   PlaceLaunch P;
   P.frames = frames;
   P.nframes = 1;
+  P.sms = device_sm_count();
   P.ntiles = L.ntiles;
   P.tile_count = tile_count;
   P.tile_start = tile_start;
+  P.block_sums = block_sums;
   P.pool = pool;
   P.out = list;
-  P.block_sums = block_sums;
-  P.frame_prefix = prefix;
   P.frame_count = count;
+  P.run_status = run_status;
+  P.status = status;
   check(launch_place(P, s), "launching the placement");
 
   uint32_t host_words[2] = {0, 0};

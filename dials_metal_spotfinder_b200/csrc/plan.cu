@@ -141,7 +141,8 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
   if (occ < 1)
     throw DeviceError("the threshold kernel does not fit on this device");
   const int per_sm = tuning_.blocks_per_sm > 0 ? std::min(tuning_.blocks_per_sm, occ) : occ;
-  max_blocks_ = device_sm_count() * per_sm;
+  sms_ = device_sm_count();
+  max_blocks_ = sms_ * per_sm;
   if (tuning_.seg_rows <= 0)
     tuning_.seg_rows = choose_seg_rows(shapes, static_cast<uint64_t>(max_blocks_) * wpc);
 
@@ -157,6 +158,7 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     d.seg_rows = std::min(tuning_.seg_rows, s.height);
     d.segments = (s.height + d.seg_rows - 1) / d.seg_rows;
     d.task_begin = task;
+    tile = round_up(tile, kPlaceTiles);
     d.tile_base = tile;
     d.out_base = out;
     // The reference's list capacity: the frame's own bytes, 16 to an entry
@@ -199,20 +201,19 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     check(cudaMemcpy(frames_, host_frames_.data(), nf * sizeof(FrameDesc),
                      cudaMemcpyHostToDevice),
           "uploading frame descriptors");
-    alloc(reinterpret_cast<void **>(&tile_count_), ntiles_ * 4, "cudaMalloc tile counts");
+    cleared_bytes_ = (ntiles_ + nblocks + 2) * 4;
+    alloc(reinterpret_cast<void **>(&tile_count_), cleared_bytes_, "cudaMalloc tile counts");
+    block_sums_ = tile_count_ + ntiles_;
+    pool_next_ = block_sums_ + nblocks;
+    run_status_ = reinterpret_cast<int *>(pool_next_ + 1);
     alloc(reinterpret_cast<void **>(&tile_start_), ntiles_ * 4, "cudaMalloc tile starts");
     alloc(reinterpret_cast<void **>(&pool_), pool_records * sizeof(SignalPixel),
           "cudaMalloc staging pool");
-    alloc(reinterpret_cast<void **>(&pool_next_), 16, "cudaMalloc pool cursor");
-    alloc(reinterpret_cast<void **>(&block_sums_), std::max<uint64_t>(nblocks, 1) * 4,
-          "cudaMalloc block sums");
     for (Slot &sl : slots_) {
       alloc(&sl.arena, arena_bytes, "cudaMalloc arena");
       check(cudaMemset(sl.arena, 0xff, arena_bytes), "filling the arena");
       alloc(reinterpret_cast<void **>(&sl.out), total_capacity_ * sizeof(SignalPixel),
             "cudaMalloc output lists");
-      alloc(reinterpret_cast<void **>(&sl.frame_prefix), (nf + 1) * 4,
-            "cudaMalloc frame prefix");
       alloc(reinterpret_cast<void **>(&sl.frame_count), (nf + 1) * 4,
             "cudaMalloc frame counts");
       sl.status = reinterpret_cast<int *>(sl.frame_count + nf);
@@ -234,7 +235,6 @@ void ThresholdPlan::release() {
   for (Slot &sl : slots_) {
     cudaFree(sl.arena);
     cudaFree(sl.out);
-    cudaFree(sl.frame_prefix);
     cudaFree(sl.frame_count);
     sl = Slot();
   }
@@ -242,14 +242,13 @@ void ThresholdPlan::release() {
   cudaFree(tile_count_);
   cudaFree(tile_start_);
   cudaFree(pool_);
-  cudaFree(pool_next_);
-  cudaFree(block_sums_);
   cudaFree(linear_);
   linear_ = nullptr;
   frames_ = nullptr;
   tile_count_ = tile_start_ = nullptr;
   pool_ = nullptr;
   pool_next_ = block_sums_ = nullptr;
+  run_status_ = nullptr;
 }
 
 void *ThresholdPlan::frame_origin(int slot, int f) const {
@@ -297,20 +296,18 @@ void ThresholdPlan::upload_device(int slot, int f, const void *device, size_t pi
 
 void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid) {
   Slot &sl = slots_.at(slot);
-  check(cudaMemsetAsync(tile_count_, 0, ntiles_ * sizeof(uint32_t), stream),
-        "clearing tile counts");
-  check(cudaMemsetAsync(pool_next_, 0, sizeof(uint32_t), stream), "clearing the pool");
-  check(cudaMemsetAsync(sl.status, 0, sizeof(int), stream), "clearing the status");
+  check(cudaMemsetAsync(tile_count_, 0, cleared_bytes_, stream), "clearing tile counts");
   ThresholdLaunch L;
   L.frames = frames_;
   L.nframes = static_cast<int32_t>(host_frames_.size());
   L.ntasks = ntasks_;
   L.tile_count = tile_count_;
   L.tile_start = tile_start_;
+  L.block_sums = block_sums_;
   L.pool = pool_;
   L.pool_next = pool_next_;
   L.pool_cap = pool_cap_;
-  L.status = sl.status;
+  L.status = run_status_;
   L.wait_limit = 1u << 22;
   L.warps_per_block = tuning_.warps_per_block;
   L.max_blocks = max_blocks_;
@@ -324,14 +321,16 @@ void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid) {
   PlaceLaunch P;
   P.frames = frames_;
   P.nframes = L.nframes;
+  P.sms = sms_;
   P.ntiles = ntiles_;
   P.tile_count = tile_count_;
   P.tile_start = tile_start_;
+  P.block_sums = block_sums_;
   P.pool = pool_;
   P.out = sl.out;
-  P.block_sums = block_sums_;
-  P.frame_prefix = sl.frame_prefix;
   P.frame_count = sl.frame_count;
+  P.run_status = run_status_;
+  P.status = sl.status;
   check(launch_place(P, stream), "launching the placement");
 }
 

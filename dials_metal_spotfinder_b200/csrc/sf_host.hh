@@ -36,6 +36,7 @@ struct ThresholdLaunch {
   uint32_t ntasks;
   uint32_t *tile_count;
   uint32_t *tile_start;
+  uint32_t *block_sums; // the counts' sums over each kPlaceTiles tiles
   SignalPixel *pool;
   uint32_t *pool_next;
   uint32_t pool_cap;
@@ -51,22 +52,25 @@ cudaError_t launch_threshold(const CUtensorMap &map, const ThresholdLaunch &L,
 template <typename T> size_t threshold_smem_bytes(int wpc);
 template <typename T> int threshold_occupancy(int wpc);
 
-// Ordered compaction of the staged records (place.cu).
+// Ordered compaction of the staged records (place.cu). Every frame's
+// tile_base is a multiple of kPlaceTiles.
 struct PlaceLaunch {
   const FrameDesc *frames;
   int32_t nframes;
+  int sms; // of the device
   uint64_t ntiles;
   const uint32_t *tile_count;
   const uint32_t *tile_start;
+  const uint32_t *block_sums; // per kPlaceTiles tiles
   const SignalPixel *pool;
   SignalPixel *out;
-  uint32_t *block_sums;   // ceil(ntiles / kPlaceTiles)
-  uint32_t *frame_prefix; // nframes + 1
-  uint32_t *frame_count;  // nframes
+  uint32_t *frame_count; // nframes
+  const int *run_status; // the threshold's status, copied to *status
+  int *status;
 };
 constexpr int kPlaceThreads = 256;
-constexpr int kPlaceItems = 4;
-constexpr int kPlaceTiles = kPlaceThreads * kPlaceItems;
+constexpr int kPlaceTiles = 1024;
+constexpr uint32_t kPlaceSlices = 4; // blocks that may share a group of tiles
 
 cudaError_t launch_place(const PlaceLaunch &L, cudaStream_t stream);
 
@@ -151,7 +155,6 @@ private:
     void *arena = nullptr;
     CUtensorMap map;
     SignalPixel *out = nullptr;
-    uint32_t *frame_prefix = nullptr;
     uint32_t *frame_count = nullptr; // followed by the status word
     int *status = nullptr;
   };
@@ -167,16 +170,20 @@ private:
   uint32_t ntasks_ = 0;
   uint64_t ntiles_ = 0, total_capacity_ = 0;
   uint32_t pool_cap_ = 0;
-  int max_blocks_ = 0, grid_blocks_ = 0;
+  int max_blocks_ = 0, grid_blocks_ = 0, sms_ = 0;
   uint64_t device_bytes_ = 0;
 
   std::vector<Slot> slots_;
   FrameDesc *frames_ = nullptr;
+  // One allocation, cleared by one memset before each run: the tiles'
+  // counts, their sums per kPlaceTiles, the pool's cursor and the run's
+  // status.
   uint32_t *tile_count_ = nullptr;
+  uint64_t cleared_bytes_ = 0;
+  uint32_t *block_sums_ = nullptr, *pool_next_ = nullptr;
+  int *run_status_ = nullptr;
   uint32_t *tile_start_ = nullptr;
   SignalPixel *pool_ = nullptr;
-  uint32_t *pool_next_ = nullptr;
-  uint32_t *block_sums_ = nullptr;
   uint8_t *linear_ = nullptr; // upload()'s contiguous copy
 };
 

@@ -310,6 +310,7 @@ struct ThresholdArgs {
   uint32_t ntasks;
   uint32_t *tile_count; // zeroed before the launch
   uint32_t *tile_start;
+  uint32_t *block_sums; // per kPlaceTiles tiles; zeroed too
   SignalPixel *pool;
   uint32_t *pool_next;
   uint32_t pool_cap; // records
@@ -772,6 +773,13 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
             args.tile_count[tile + fd.strips] = foundB;
             args.tile_start[tile + fd.strips] = chunk == kNoChunk ? 0u : start + foundA;
           }
+          // the placement's sums over groups of tiles
+          const uint64_t ga = tile / kPlaceTiles, gb = (tile + fd.strips) / kPlaceTiles;
+          const uint32_t na = ga == gb ? foundA + foundB : foundA;
+          if (na > 0)
+            atomicAdd(&args.block_sums[ga], na);
+          if (ga != gb && foundB > 0)
+            atomicAdd(&args.block_sums[gb], foundB);
         }
         fill += foundA + foundB;
         __syncwarp();
@@ -847,6 +855,7 @@ static cudaError_t launch_wpc(const CUtensorMap &map, const ThresholdLaunch &L,
   a.ntasks = L.ntasks;
   a.tile_count = L.tile_count;
   a.tile_start = L.tile_start;
+  a.block_sums = L.block_sums;
   a.pool = L.pool;
   a.pool_next = L.pool_next;
   a.pool_cap = L.pool_cap;
