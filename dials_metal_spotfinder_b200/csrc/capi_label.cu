@@ -96,7 +96,7 @@ struct HostLabeller {
       check(cudaMalloc(&list, std::max<size_t>(n, 1024) * sizeof(SignalPixel)), "cudaMalloc list");
       list_cap = std::max<size_t>(n, 1024);
     }
-    dev->reserve(std::max<uint64_t>(n, 1), 1, carry + 1);
+    dev->reserve(std::max<uint64_t>(n, 1), 1, carry + 1, true);
     if (n)
       check(cudaMemcpyAsync(list, sig, n * sizeof(SignalPixel), cudaMemcpyHostToDevice, stream),
             "copying the signal list");
@@ -112,7 +112,7 @@ struct HostLabeller {
   void finish() {
     if (!started)
       return;
-    dev->reserve(1, 1, carry + 1);
+    dev->reserve(1, 1, carry + 1, true);
     dev->enqueue(0, list, offs, meta, nullptr, meta + 1, true, stream);
     collect();
   }

@@ -58,6 +58,8 @@ constexpr int kThreads = 256;
 // launches with larger buffers.
 constexpr uint32_t kSmallCap = 256;
 constexpr uint32_t kMidCap = 512;
+// The least a growing labeller makes room for: 16 Ki pixels, 3 MB.
+constexpr uint64_t kRoomPixels = 16384;
 
 // Quotients by one divisor fixed for a whole launch (the frame width), by a
 // multiply-high and two shifts: Granlund and Montgomery, "Division by
@@ -1560,18 +1562,10 @@ DeviceLabeller::~DeviceLabeller() {
 }
 
 void DeviceLabeller::release() {
-  for (Live &l : live_) {
-    cudaFree(l.frame);
-    cudaFree(l.index);
-    cudaFree(l.value);
-    cudaFree(l.parent);
+  cudaFree(arena_);
+  arena_ = nullptr;
+  for (Live &l : live_)
     l = Live();
-  }
-  void *ptrs[] = {root_, size_, rank_of_root_, cursor_, lastz_, bits_, bcnt_, flist_, comp_root_,
-                  msize_, mpk_, runs_, run_starts_, spot_tmp_, pix_tmp_, members_, pack_, obits_, ocnt_, spots_out_, kept_out_, seg_start_,
-                  seg_count_, seg_z_, tab_, big_, mid_};
-  for (void *p : ptrs)
-    cudaFree(p);
   tab_ = nullptr;
   root_ = size_ = rank_of_root_ = cursor_ = nullptr;
   lastz_ = nullptr;
@@ -1587,14 +1581,14 @@ void DeviceLabeller::release() {
   seg_z_ = nullptr;
 }
 
-void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t carry_pixels) {
+void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t carry_pixels,
+                             bool room) {
   if (batch_pixels <= batch_cap_ && max_frames <= frame_cap_ && carry_pixels <= carry_cap_)
     return;
   const uint64_t bc = std::max(batch_pixels, batch_cap_);
   const int fc = std::max(max_frames, frame_cap_);
   const uint64_t cc = std::max(carry_pixels, carry_cap_);
-  const uint64_t live = bc + cc;
-  if (live >= 0x7fffffffull)
+  if (bc + cc >= 0x7fffffffull)
     throw std::invalid_argument("labelling batch too large");
   // Growing keeps the carry: copy it across after reallocating.
   check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
@@ -1610,55 +1604,20 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
     check(cudaMemcpy(par.data(), c.parent, host.carry_n * 4, cudaMemcpyDeviceToHost), "carry");
   }
   release();
-  const uint64_t nwmax = live / 32 + 1;
-  const uint64_t spot_cap = live / opt_.min_spot_size + 1;
-  try {
-    auto alloc = [](auto **p, uint64_t count, const char *what) {
-      check(cudaMalloc(reinterpret_cast<void **>(p), std::max<uint64_t>(count, 1) * sizeof(**p)),
-            what);
-    };
-    for (Live &l : live_) {
-      alloc(&l.frame, live, "live frames");
-      alloc(&l.index, live, "live indices");
-      alloc(&l.value, live, "live values");
-      alloc(&l.parent, live, "live parents");
-    }
-    alloc(&root_, live, "roots");
-    alloc(&size_, live, "sizes");
-    alloc(&rank_of_root_, live, "ranks");
-    alloc(&cursor_, live, "cursors");
-    alloc(&lastz_, live, "last frames");
-    alloc(&bits_, nwmax, "finished-root bitmap");
-    alloc(&bcnt_, (fc + 1) * nwmax, "bucket counts");
-    alloc(&flist_, live, "finished roots");
-    alloc(&comp_root_, live, "components");
-    alloc(&msize_, live, "member sizes");
-    alloc(&mpk_, live, "member offsets");
-    alloc(&runs_, live, "run list");
-    alloc(&run_starts_, live / 32 + 1, "run starts");
-    alloc(&members_, live, "members");
-    alloc(&pack_, live, "spot offsets");
-    alloc(&obits_, nwmax, "open bitmap");
-    alloc(&ocnt_, nwmax, "open counts");
-    alloc(&big_, live / (kMidCap + 1) + 1, "large components");
-    alloc(&mid_, live / (kSmallCap + 1) + 1, "middle-sized components");
-    alloc(&spots_out_, spot_cap, "spots");
-    alloc(&spot_tmp_, spot_cap, "spot scratch");
-    alloc(&pix_tmp_, live, "spot pixel scratch");
-    alloc(&kept_out_, live, "spot pixels");
-    alloc(&seg_start_, fc + 1, "segments");
-    alloc(&seg_count_, fc + 1, "segments");
-    alloc(&seg_z_, fc + 1, "segments");
-    alloc(&tab_, static_cast<uint64_t>(fc) * nblk_, "block tables");
-    scan32_.reserve((fc + 1) * nwmax);
-    scan32_.reserve(live);
-    scan64_.reserve(live);
-  } catch (...) {
-    release();
-    batch_cap_ = carry_cap_ = live_cap_ = spot_cap_ = 0;
-    frame_cap_ = 0;
-    throw;
+  batch_cap_ = carry_cap_ = live_cap_ = spot_cap_ = 0;
+  frame_cap_ = 0;
+  // With room: half as much again for the batch, a few such batches for the
+  // carry, and at least kRoomPixels, where that fits.
+  bool done = false;
+  if (room) {
+    const uint64_t rb = std::max<uint64_t>(
+        bc, std::min(std::max(bc + bc / 2, kRoomPixels),
+                     static_cast<uint64_t>(height_) * static_cast<uint64_t>(width_)));
+    const uint64_t rc = std::max(2 * cc, 4 * rb);
+    done = rb + rc < 0x7fffffffull && allocate(rb, fc, rc);
   }
+  if (!done && !allocate(bc, fc, cc))
+    throw DeviceError("CUDA: cudaMalloc labeller buffers: out of memory");
   if (host.carry_n) {
     const Live &c = live_[cur_];
     check(cudaMemcpy(c.frame, fr.data(), host.carry_n * 4, cudaMemcpyHostToDevice), "carry");
@@ -1666,11 +1625,82 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
     check(cudaMemcpy(c.value, val.data(), host.carry_n * 4, cudaMemcpyHostToDevice), "carry");
     check(cudaMemcpy(c.parent, par.data(), host.carry_n * 4, cudaMemcpyHostToDevice), "carry");
   }
+}
+
+// The buffers for these capacities, in one allocation; false (and nothing
+// held) where it does not fit.
+bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
+  const uint64_t live = bc + cc;
+  const uint64_t nwmax = live / 32 + 1;
+  const uint64_t spot_cap = live / opt_.min_spot_size + 1;
+  struct Part {
+    void **p;
+    uint64_t bytes;
+  };
+  std::vector<Part> parts;
+  auto part = [&](auto **p, uint64_t count) {
+    parts.push_back({reinterpret_cast<void **>(p), std::max<uint64_t>(count, 1) * sizeof(**p)});
+  };
+  for (Live &l : live_) {
+    part(&l.frame, live);
+    part(&l.index, live);
+    part(&l.value, live);
+    part(&l.parent, live);
+  }
+  part(&root_, live);
+  part(&size_, live);
+  part(&rank_of_root_, live);
+  part(&cursor_, live);
+  part(&lastz_, live);
+  part(&bits_, nwmax);                                // finished-root bitmap
+  part(&bcnt_, static_cast<uint64_t>(fc + 1) * nwmax); // bucket counts
+  part(&flist_, live);                                // finished roots
+  part(&comp_root_, live);
+  part(&msize_, live);
+  part(&mpk_, live);
+  part(&runs_, live);
+  part(&run_starts_, live / 32 + 1);
+  part(&members_, live);
+  part(&pack_, live);
+  part(&obits_, nwmax);
+  part(&ocnt_, nwmax);
+  part(&big_, live / (kMidCap + 1) + 1);
+  part(&mid_, live / (kSmallCap + 1) + 1);
+  part(&spots_out_, spot_cap);
+  part(&spot_tmp_, spot_cap);
+  part(&pix_tmp_, live);
+  part(&kept_out_, live);
+  part(&seg_start_, static_cast<uint64_t>(fc) + 1);
+  part(&seg_count_, static_cast<uint64_t>(fc) + 1);
+  part(&seg_z_, static_cast<uint64_t>(fc) + 1);
+  part(&tab_, static_cast<uint64_t>(fc) * nblk_); // block tables
+  uint64_t total = 0;
+  for (const Part &q : parts)
+    total += (q.bytes + 255) / 256 * 256;
+  if (cudaMalloc(reinterpret_cast<void **>(&arena_), total) != cudaSuccess) {
+    cudaGetLastError();
+    arena_ = nullptr;
+    return false;
+  }
+  uint64_t at = 0;
+  for (const Part &q : parts) {
+    *q.p = arena_ + at;
+    at += (q.bytes + 255) / 256 * 256;
+  }
+  try {
+    scan32_.reserve((fc + 1) * nwmax);
+    scan32_.reserve(live);
+    scan64_.reserve(live);
+  } catch (const DeviceError &) {
+    release();
+    return false;
+  }
   batch_cap_ = bc;
   frame_cap_ = fc;
   carry_cap_ = cc;
   live_cap_ = live;
   spot_cap_ = spot_cap;
+  return true;
 }
 
 void DeviceLabeller::set_next_frame(int64_t z, cudaStream_t s) {

@@ -84,8 +84,12 @@ public:
   // Buffers for batches of up to `batch_pixels` new signal pixels over up to
   // `max_frames` frames, with up to `carry_pixels` carried between batches.
   // Grows (synchronising the device) only when asked for more; call before
-  // any graph capture.
-  void reserve(uint64_t batch_pixels, int max_frames, uint64_t carry_pixels);
+  // any graph capture. With `room`, for a caller that learns the sizes frame
+  // by frame, it grows by more than it was asked where that fits: the carry
+  // grows by about a frame's pixels with each of the first frames, and
+  // reallocating on every one of them was 67 of the 85 ms that four
+  // 2162 x 2068 frames took.
+  void reserve(uint64_t batch_pixels, int max_frames, uint64_t carry_pixels, bool room = false);
 
   // Enqueue one batch of `nframes` consecutive frames numbered from the
   // device-side batch_z0, which the batch then advances by nframes. Frame
@@ -119,9 +123,12 @@ public:
 
 private:
   void release();
+  bool allocate(uint64_t batch_pixels, int frames, uint64_t carry_pixels);
 
   int height_, width_;
   GroupOptions opt_;
+
+  unsigned char *arena_ = nullptr; // every buffer below but the scalars and the carry's table
 
   uint64_t batch_cap_ = 0, carry_cap_ = 0, live_cap_ = 0, spot_cap_ = 0;
   int frame_cap_ = 0;
