@@ -14,26 +14,45 @@
 namespace sf {
 namespace {
 
-constexpr int kDecodeWarps = 4;
+constexpr int kDecodeWarps = 2; // per block of threads; the warps are independent
 constexpr unsigned kFull = 0xffffffffu;
-// Compressed bytes a warp stages in shared memory; a longer block (nearly
-// incompressible, so few sequences) is parsed from global memory instead.
-constexpr uint32_t kStageCap = 4096;
-// Shared memory a warp may own: the decoded block, its staged compressed
-// bytes, and the list of its sequence starts (a sequence other than the last
-// spans at least three bytes).
-__host__ __device__ constexpr uint32_t list_bytes_for(uint32_t stage_bytes) {
-  return ((stage_bytes / 3 + 2) * 2 + 15) & ~15u;
-}
-constexpr uint32_t kWarpSmemMax = static_cast<uint32_t>(kMaxBlockBytes) + kStageCap + 16 +
-                                  list_bytes_for(kStageCap + 16);
+// Compressed bytes a warp stages in shared memory: every block of up to
+// 8 KB that any coder made shorter. A longer one (nearly incompressible, so
+// few sequences) is parsed from global memory instead.
+constexpr uint32_t kStageCap = 8192;
 constexpr uint16_t kSeqEnd = 0xffff, kSeqBad = 0xfffe;
+// Sequences a lane parses at a time, and a warp's records at a time.
+constexpr uint32_t kLaneSeqs = 4;
+constexpr uint32_t kGroupSeqs = 32 * kLaneSeqs;
+// 32-byte pieces of the output whose references a warp looks up at a time.
+constexpr uint32_t kSegments = 4;
 
-// lane % d and 32 % d for match offsets d < 32, shared by a block's warps.
-struct ModTable {
-  uint8_t lane_mod[32][32];
-  uint8_t step[32];
+// What a warp owns of the shared memory. `next` (two bytes per compressed
+// byte) lies over the output, which is written only once it is dead, and
+// `extra` is what it needs beyond that; everything after the output is dead
+// once the block is decoded and then holds `bounce` (see store_planes).
+struct WarpLayout {
+  uint32_t out, extra, stage, list, ends, starts, total;
 };
+__host__ __device__ constexpr uint32_t up16(uint32_t x) { return (x + 15) & ~15u; }
+__host__ __device__ constexpr WarpLayout warp_layout(uint32_t out_bytes, uint32_t stage_bytes,
+                                                     uint32_t elem) {
+  WarpLayout w{};
+  w.out = out_bytes;
+  w.extra = up16(2 * stage_bytes) > out_bytes ? up16(2 * stage_bytes) - out_bytes : 0;
+  w.stage = stage_bytes;
+  // every fourth sequence start; a sequence spans at least three bytes
+  w.list = up16((stage_bytes / (3 * kLaneSeqs) + 3) * 2);
+  // a bit per compressed byte, and two words past the last
+  w.ends = up16((stage_bytes / 32 + 3) * 4);
+  // a bit per output byte, and a step's words past the last
+  w.starts = up16((out_bytes / 32 + 1 + kSegments) * 4);
+  const uint32_t rest =
+      w.extra + w.stage + w.list + w.ends + w.starts + kGroupSeqs * static_cast<uint32_t>(sizeof(uint2));
+  const uint32_t bounce = 1024 * elem;
+  w.total = w.out + (rest > bounce ? rest : bounce);
+  return w;
+}
 
 struct BlockDesc {
   uint64_t in;  // the LZ4 data, in the chunk
@@ -47,6 +66,7 @@ struct FrameDst {
   uint8_t *base;
   uint64_t pitch;
   uint64_t row_bytes;
+  uint32_t word; // 4, 2 or 1: divides the base, the pitch, the rows and every block's offset
 };
 
 size_t round16(size_t x) { return (x + 15) & ~static_cast<size_t>(15); }
@@ -151,176 +171,312 @@ __device__ bool warp_lz4(const uint8_t *src, uint32_t cs, uint8_t *dst, uint32_t
   return op == n;
 }
 
-// The same decode with the sequence parsing spread over the warp, for a
-// block whose L compressed bytes sit in shared memory at `in`:
+// A length continued past its four bits at byte q of the L compressed bytes:
+// adds the run of 255s and the byte that ends it, and moves q past them.
+// `ends` has a bit per byte that is not 255, set from L on; false where the
+// length runs past the end. (Byte by byte, the warp would wait for its
+// longest run at every step.)
+__device__ __forceinline__ bool add_length(const uint8_t *in, uint32_t L, const uint32_t *ends,
+                                           uint32_t *q, uint32_t *length) {
+  if (*q >= L)
+    return false;
+  uint32_t word = *q >> 5;
+  uint32_t w = ends[word] & (0xffffffffu << (*q & 31));
+  while (w == 0) // ends with the word after the last byte's
+    w = ends[++word];
+  const uint32_t r = 32 * word + __ffs(w) - 1;
+  if (r >= L)
+    return false;
+  *length += 255 * (r - *q) + in[r];
+  *q = r + 1;
+  return true;
+}
+
+// The LZ4 sequence at byte p < L, every read bounds-checked: its literals
+// (count, start), its match (offset, length; 0 of the last sequence), and
+// the byte after it -- L where no last sequence follows, kSeqEnd where its
+// literals end the block, kSeqBad where it runs past the end.
+struct Seq {
+  uint32_t lit, start, off, len;
+};
+__device__ __forceinline__ uint32_t parse_seq(const uint8_t *in, uint32_t L,
+                                              const uint32_t *ends, uint32_t p, Seq *s) {
+  const uint32_t t = in[p];
+  uint32_t q = p + 1;
+  bool ok = true;
+  *s = Seq{t >> 4, 0, 0, 0};
+  if (s->lit == 15)
+    ok = add_length(in, L, ends, &q, &s->lit);
+  ok = ok && s->lit <= L - q;
+  s->start = q;
+  q += s->lit;
+  const bool last = ok && q == L;
+  ok = ok && (last || L - q >= 2);
+  if (ok && !last) {
+    s->off = in[q] | (static_cast<uint32_t>(in[q + 1]) << 8);
+    s->len = (t & 15) + 4;
+    q += 2;
+    if (s->len == 19)
+      ok = add_length(in, L, ends, &q, &s->len);
+  }
+  return !ok ? kSeqBad : last ? kSeqEnd : q;
+}
+
+// The same decode spread over the warp, for a block whose L compressed bytes
+// sit in shared memory, `in_at` bytes after the output `dst`:
 //  1. every lane parses a sequence at each of its byte positions p as if a
-//     token started there, and records where the next one would start
-//     (next[p]; kSeqEnd when its literals end the block, kSeqBad when it
-//     runs past the end);
-//  2. lane 0 follows next[] from byte 0, listing the real sequence starts;
-//  3. 32 sequences at a time, one a lane: parse, an exclusive scan of the
-//     output lengths for each sequence's output position, the bounds
-//     checks, the literal copies (short ones by their own lane, long ones by
-//     the warp), then the matches in order, each by the warp as in
-//     warp_lz4 (byte i of a match of offset d is byte i mod d of the d bytes
-//     before it; the phases come from the table).
-// `next` (2L bytes) may share `dst`: it is dead before any output is
-// written. `list` holds L / 3 + 2 entries. Returns false on a malformed
-// block, having written nothing past n.
-__device__ bool warp_lz4_parallel(const uint8_t *in, uint32_t L, uint16_t *next, uint16_t *list,
-                                  uint8_t *dst, uint32_t n, int lane, const ModTable &mt) {
-  for (uint32_t p = lane; p < L; p += 32) {
-    uint32_t q = p;
-    const uint32_t t = in[q++];
-    uint32_t lit = t >> 4, nx = kSeqBad;
-    bool ok = true;
-    if (lit == 15) {
-      uint32_t v;
-      do {
-        if (q >= L) {
-          ok = false;
-          break;
-        }
-        v = in[q++];
-        lit += v;
-      } while (v == 255);
-    }
-    if (ok && lit <= L - q) {
-      q += lit;
-      if (q == L) {
-        nx = kSeqEnd;
-      } else if (L - q >= 2) {
-        q += 2;
-        if ((t & 15) == 15) {
-          uint32_t v;
-          do {
-            if (q >= L) {
-              ok = false;
-              break;
-            }
-            v = in[q++];
-          } while (v == 255);
-        }
-        if (ok)
-          nx = q; // q == L: no final sequence, refused by the walk
-      }
-    }
-    next[p] = static_cast<uint16_t>(nx);
+//     token started there: next[p] is where the next one would start;
+//  2. two doublings in place (next[p] > p, and a warp's reads go before its
+//     writes, so entries above p still hold the single step) make next[p]
+//     the start four sequences on;
+//  3. lane 0 follows next[] from byte 0, listing every fourth real start;
+//  4. 128 sequences at a time, four a lane: parse, a warp scan of the output
+//     lengths, the bounds checks, a record per sequence and a bit per output
+//     byte that starts one;
+//  5. the group's output, 32 bytes (one a lane) at a time. A byte's sequence
+//     is its rank among the start bits; it is a literal, or the byte `off`
+//     back: an earlier byte of the output, or of the same 32, in which case
+//     the lanes follow each other's references, doubling (five rounds at
+//     most), to the one that holds the value. All that but the reads of the
+//     output itself is done for kSegments pieces together. A stretch inside
+//     one match is copied at once, in 16-byte words when it repeats a short
+//     period.
+// Step 5 costs the same for 32 output bytes whatever the number of
+// sequences in them; copying match by match, each by the whole warp, cost
+// 45 instructions and a chain of shared-memory reads a sequence. The decode
+// of one frame alone: 2162 x 2068 uint16 in plain LZ4 blocks (1200 sequences
+// of 7 bytes a block) 575 -> 95 us, uint32 223 -> 155; uint16 in bslz4
+// blocks (250 sequences, most of the output in a few) 77 -> 57; 4362 x 4148
+// bslz4, whose 4418 blocks keep the SMs issuing either way, 135 -> 135.
+// Bound: the latency of step 5's chain of shared-memory reads where a chunk
+// has few blocks, instruction issue where it has many.
+// Returns false on a malformed block, having written nothing past n.
+__device__ bool warp_lz4_parallel(uint8_t *dst, uint32_t in_at, uint32_t L, uint16_t *next,
+                                  uint16_t *list, uint32_t *ends, uint2 *rec, uint32_t *starts,
+                                  uint32_t n, int lane) {
+  const uint8_t *in = dst + in_at;
+  for (uint32_t base = 0; base < L + 32; base += 32) {
+    const uint32_t m = __ballot_sync(kFull, base + lane >= L || in[base + lane] != 255);
+    if (lane == 0)
+      ends[base >> 5] = m;
   }
   __syncwarp();
-  uint32_t k = 0;
-  int bad = 0;
+  for (uint32_t p = lane; p < L; p += 32) {
+    Seq s;
+    next[p] = static_cast<uint16_t>(parse_seq(in, L, ends, p, &s));
+  }
+  for (uint32_t k = lane; k < n / 32 + 1 + kSegments; k += 32)
+    starts[k] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    for (uint32_t base = 0; base < L; base += 128) {
+      uint32_t a[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const uint32_t p = base + 32 * u + lane;
+        a[u] = p < L ? next[p] : kSeqBad;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (a[u] < L)
+          a[u] = next[a[u]];
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const uint32_t p = base + 32 * u + lane;
+        if (p < L)
+          next[p] = static_cast<uint16_t>(a[u]);
+      }
+    }
+    __syncwarp();
+  }
+  uint32_t quads = 0;
   if (lane == 0) {
     uint32_t p = 0;
-    while (true) {
-      if (p >= L) {
-        bad = 1;
-        break;
-      }
-      list[k++] = static_cast<uint16_t>(p);
-      const uint32_t nx = next[p];
-      if (nx == kSeqEnd)
-        break;
-      if (nx == kSeqBad) {
-        bad = 1;
-        break;
-      }
-      p = nx;
+    while (p < L) { // neither mark is below L, and p rises
+      list[quads++] = static_cast<uint16_t>(p);
+      p = next[p];
     }
+    if (p != kSeqEnd)
+      quads = 0;
   }
-  if (__shfl_sync(kFull, bad, 0))
+  quads = __shfl_sync(kFull, quads, 0);
+  if (quads == 0)
     return false;
-  k = __shfl_sync(kFull, k, 0);
   __syncwarp();
+
+  const uint32_t le = 0xffffffffu >> (31 - lane);
   uint32_t obase = 0;
-  for (uint32_t base = 0; base < k; base += 32) {
-    const uint32_t j = base + lane;
-    const bool active = j < k, last = j + 1 == k;
-    uint32_t lit = 0, ls = 0, off = 0, ml = 0;
-    if (active) {
-      // in bounds: the walk saw this sequence end inside the block
-      uint32_t q = list[j];
-      const uint32_t t = in[q++];
-      lit = t >> 4;
-      if (lit == 15) {
-        uint32_t v;
-        do {
-          v = in[q++];
-          lit += v;
-        } while (v == 255);
+  for (uint32_t qb = 0; qb < quads; qb += 32) {
+    Seq s[kLaneSeqs];
+    uint32_t have = 0, total = 0;
+    bool last = false;
+    uint32_t p = qb + lane < quads ? list[qb + lane] : L;
+#pragma unroll
+    for (uint32_t k = 0; k < kLaneSeqs; k++) {
+      s[k] = Seq{0, 0, 0, 0};
+      if (p < L) { // step 3 saw the sequence end in the block
+        p = parse_seq(in, L, ends, p, &s[k]);
+        total += s[k].lit + s[k].len;
+        have++;
+        last = p >= L;
       }
-      ls = q;
-      q += lit;
-      if (!last) {
-        off = in[q] | (static_cast<uint32_t>(in[q + 1]) << 8);
-        q += 2;
-        ml = (t & 15) + 4;
-        if ((t & 15) == 15) {
-          uint32_t v;
-          do {
-            v = in[q++];
-            ml += v;
-          } while (v == 255);
-        }
-      }
+      __syncwarp();
     }
-    const uint32_t len = lit + ml;
-    uint32_t incl = len;
+    uint32_t incl = total;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t y = __shfl_up_sync(kFull, incl, d);
       if (lane >= d)
         incl += y;
     }
-    const uint32_t op = obase + incl - len;
-    const bool ok = !active || (op + len <= n && (last || (off != 0 && off <= op + lit)));
+    // lengths of up to 255 L a lane: the sums stay below 2^32
+    uint32_t op = obase + incl - total;
+    bool ok = op + total <= n;
+#pragma unroll
+    for (uint32_t k = 0; k < kLaneSeqs; k++)
+      if (k < have) {
+        const uint32_t m = op + s[k].lit;
+        if (!(last && k + 1 == have))
+          ok = ok && s[k].off != 0 && s[k].off <= m;
+        rec[kLaneSeqs * lane + k] = make_uint2((op & 0xffffu) | (m << 16),
+                                               ((s[k].start - op) & 0xffffu) | (s[k].off << 16));
+        if (ok && s[k].lit + s[k].len)
+          atomicOr(&starts[op >> 5], 1u << (op & 31));
+        op = m + s[k].len;
+      }
     if (__any_sync(kFull, !ok))
       return false;
-    if (lit <= 16) {
-      for (uint32_t i = 0; i < lit; i++)
-        dst[op + i] = in[ls + i];
-    }
-    for (uint32_t mask = __ballot_sync(kFull, lit > 16); mask; mask &= mask - 1) {
-      const int sl = __ffs(mask) - 1;
-      const uint32_t o = __shfl_sync(kFull, op, sl), s = __shfl_sync(kFull, ls, sl);
-      const uint32_t c = __shfl_sync(kFull, lit, sl);
-      for (uint32_t i = lane; i < c; i += 32)
-        dst[o + i] = in[s + i];
-    }
+    const uint32_t nseq = __reduce_add_sync(kFull, have);
+    const uint32_t end = obase + __shfl_sync(kFull, incl, 31); // of the group's output
     __syncwarp();
-    const uint32_t mstart = op + lit;
-    for (uint32_t mask = __ballot_sync(kFull, ml != 0); mask; mask &= mask - 1) {
-      const int sl = __ffs(mask) - 1;
-      const uint32_t m = __shfl_sync(kFull, mstart, sl), d = __shfl_sync(kFull, off, sl);
-      const uint32_t c = __shfl_sync(kFull, ml, sl);
-      uint32_t q, step;
-      if (d >= 32) {
-        q = lane;
-        step = d == 32 ? 0 : 32;
-      } else {
-        q = mt.lane_mod[d][lane];
-        step = mt.step[d];
+
+    uint32_t lo = obase; // bytes below are written
+    uint32_t before = 0; // sequences of the group that start before this segment
+    uint32_t S = lo & ~31u;
+    while (S < end) {
+      uint32_t w[kSegments];
+#pragma unroll
+      for (uint32_t u = 0; u < kSegments; u++)
+        w[u] = starts[(S >> 5) + u]; // none at or past `end`
+      if (S < lo)
+        w[0] &= 0xffffffffu << (lo - S);
+      if (w[0] == 0 && S >= lo) {
+        // inside one sequence: a long enough stretch of its match?
+        const uint2 r = rec[before - 1];
+        const uint32_t stop = before < nseq ? rec[before].x & 0xffffu : end;
+        const uint32_t m = r.x >> 16, d = r.y >> 16, len = stop - S;
+        if (S >= m && len >= 64) {
+          bool copied = true;
+          if (d <= 16 && (d & (d - 1)) == 0) {
+            // period 1, 2, 4, 8 or 16: every 16-byte word from S is the same
+            uint32_t q[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+              q[k] = 0;
+#pragma unroll
+              for (uint32_t t = 0; t < 4; t++)
+                q[k] |= static_cast<uint32_t>(dst[S - d + ((4 * k + t) & (d - 1))]) << (8 * t);
+            }
+            const uint32_t nv = len / 16;
+            uint4 *v = reinterpret_cast<uint4 *>(dst + S);
+            for (uint32_t i = lane; i < nv; i += 32)
+              v[i] = make_uint4(q[0], q[1], q[2], q[3]);
+            if (static_cast<uint32_t>(lane) < (len & 15u))
+              dst[S + 16 * nv + lane] = dst[S - d + (lane & (d - 1))];
+            __syncwarp();
+          } else {
+            // a whole number of periods back is as good as one, and the more
+            // is written the further back it can be: as many whole rows of 32
+            // as lie between, up to four at once
+            uint32_t D = d;
+            for (uint32_t c = S; copied && c < stop;) {
+              while (2 * D <= c - (m - d) && D < 128)
+                D *= 2;
+              const uint32_t rows = min(D / 32, 4u);
+              copied = rows > 0; // else: too little written yet
+              uint32_t v[4];
+#pragma unroll
+              for (uint32_t u = 0; u < 4; u++)
+                if (u < rows && c + 32 * u + lane < stop)
+                  v[u] = dst[c + 32 * u + lane - D];
+#pragma unroll
+              for (uint32_t u = 0; u < 4; u++)
+                if (u < rows && c + 32 * u + lane < stop)
+                  dst[c + 32 * u + lane] = static_cast<uint8_t>(v[u]);
+              __syncwarp();
+              c += 32 * rows;
+            }
+          }
+          if (copied) {
+            lo = stop;
+            S = lo & ~31u;
+            continue;
+          }
+        }
       }
-      for (uint32_t i = lane; i < c; i += 32) {
-        dst[m + i] = dst[m - d + q];
-        q += step;
-        if (q >= d)
-          q -= d;
+      // at: where the byte's value is read, for the lanes that read one;
+      // from: the lane of the piece that does
+      uint32_t at[kSegments], from[kSegments];
+      bool within[kSegments], inside = false;
+#pragma unroll
+      for (uint32_t u = 0; u < kSegments; u++) {
+        const uint32_t P = S + 32 * u, i = P + lane;
+        const uint32_t rank = before + __popc(w[u] & le);
+        before += __popc(w[u]);
+        const uint2 r = rec[rank ? rank - 1 : 0u];
+        const bool active = i >= lo && i < end;
+        const bool literal = i < (r.x >> 16);
+        const uint32_t back = i - (r.y >> 16); // off <= i
+        within[u] = active && !literal && back >= P;
+        inside = inside || within[u];
+        from[u] = within[u] ? back - P : static_cast<uint32_t>(lane);
+        // a byte below lo is already there; one at or past the end is unused
+        at[u] = i < lo ? i : 0u;
+        if (active && !within[u])
+          at[u] = literal ? in_at + i + static_cast<uint32_t>(static_cast<int16_t>(r.y & 0xffffu))
+                          : back;
       }
-      __syncwarp();
+      while (__any_sync(kFull, inside)) {
+        inside = false;
+#pragma unroll
+        for (uint32_t u = 0; u < kSegments; u++) {
+          const uint32_t q = __shfl_sync(kFull, from[u], static_cast<int>(from[u]));
+          inside = inside || q != from[u];
+          from[u] = q;
+        }
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kSegments; u++) {
+        const uint32_t i = S + 32 * u + lane;
+        const uint32_t v = __shfl_sync(kFull, static_cast<uint32_t>(dst[at[u]]),
+                                       static_cast<int>(from[u]));
+        if (i >= lo && i < end)
+          dst[i] = static_cast<uint8_t>(v);
+        __syncwarp();
+      }
+      S += 32 * kSegments;
     }
-    obase += __shfl_sync(kFull, incl, 31);
+    obase = end;
   }
   return obase == n;
 }
 
+// The row holding byte `col` counted from the start of `row`; `col` becomes
+// the byte's place in it.
+__device__ __forceinline__ uint8_t *frame_row(const FrameDst &D, uint8_t *row, uint64_t &col) {
+  const uint64_t down = ((col | D.row_bytes) >> 32)
+                            ? col / D.row_bytes
+                            : static_cast<uint32_t>(col) / static_cast<uint32_t>(D.row_bytes);
+  col -= down * D.row_bytes;
+  return row + down * D.pitch;
+}
+
 // Where linear byte `o` of the frame lives.
 __device__ __forceinline__ uint8_t *frame_at(const FrameDst &D, uint64_t o, uint64_t &col) {
-  const uint64_t row = ((o | D.row_bytes) >> 32)
-                           ? o / D.row_bytes
-                           : static_cast<uint32_t>(o) / static_cast<uint32_t>(D.row_bytes);
-  col = o - row * D.row_bytes;
-  return D.base + row * D.pitch;
+  col = o;
+  return frame_row(D, D.base, col);
 }
 
 // Writes `nb` (<= 32) bytes held in w[0..7] to frame bytes [o, o + nb): the
@@ -368,23 +524,26 @@ __device__ __forceinline__ void put(const FrameDst &D, uint64_t o, uint32_t nb,
   }
 }
 
-// Eight elements of E bytes, group g of a bit-transposed block of `plane`
-// bytes per bit plane, back in element order: element i's byte j is byte i
-// of the 8 x 8 transpose of bytes (8j + k) * plane + g, k = 0..7.
+// transpose8x8 on a word's two halves: its first two steps stay within each.
+__device__ __forceinline__ void transpose_halves(uint32_t &lo, uint32_t &hi) {
+  uint32_t t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
+  lo ^= t ^ (t << 7);
+  t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
+  hi ^= t ^ (t << 7);
+  t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
+  lo ^= t ^ (t << 14);
+  t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
+  hi ^= t ^ (t << 14);
+  t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
+  lo ^= t;
+  hi ^= t >> 4;
+}
+
+// Eight elements of E bytes from their bytes: byte i of lo[j], hi[j] (i < 4,
+// i >= 4) is byte j of element i.
 template <int E>
-__device__ __forceinline__ void untranspose(const uint8_t *buf, uint32_t plane, uint32_t g,
-                                            uint32_t (&w)[8]) {
-  uint32_t lo[E], hi[E];
-#pragma unroll
-  for (int j = 0; j < E; j++) {
-    uint64_t x = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      x |= static_cast<uint64_t>(buf[(8 * j + k) * plane + g]) << (8 * k);
-    const uint64_t y = transpose8x8(x);
-    lo[j] = static_cast<uint32_t>(y);
-    hi[j] = static_cast<uint32_t>(y >> 32);
-  }
+__device__ __forceinline__ void weave(const uint32_t (&lo)[E], const uint32_t (&hi)[E],
+                                      uint32_t *w) {
   if constexpr (E == 1) {
     w[0] = lo[0];
     w[1] = hi[0];
@@ -408,31 +567,168 @@ __device__ __forceinline__ void untranspose(const uint8_t *buf, uint32_t plane, 
   }
 }
 
-// Blocks of a chunk, one warp each, grid-strided. Each warp owns out_bytes
-// of shared memory for the decoded block and stage_bytes for its compressed
-// bytes. E > 0: bitshuffle blocks of E-byte elements, un-transposed on the
-// way out; E == 0: plain LZ4, copied out 16 bytes a lane. Warp 0 of block 0
-// also copies the chunk's raw tail (elements after the last block).
+// Eight elements of E bytes, group g of a bit-transposed block of `plane`
+// bytes per bit plane, back in element order: element i's byte j is byte i
+// of the 8 x 8 transpose of bytes (8j + k) * plane + g, k = 0..7.
+template <int E>
+__device__ __forceinline__ void untranspose(const uint8_t *buf, uint32_t plane, uint32_t g,
+                                            uint32_t (&w)[8]) {
+  uint32_t lo[E], hi[E];
+#pragma unroll
+  for (int j = 0; j < E; j++) {
+    uint64_t x = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      x |= static_cast<uint64_t>(buf[(8 * j + k) * plane + g]) << (8 * k);
+    lo[j] = static_cast<uint32_t>(x);
+    hi[j] = static_cast<uint32_t>(x >> 32);
+    transpose_halves(lo[j], hi[j]);
+  }
+  weave<E>(lo, hi, w);
+}
+
+// The 16-byte unit of the bounce buffer that holds unit u: spread so that
+// lanes writing four units each, or reading consecutive words, meet in no
+// bank.
+__device__ __forceinline__ uint32_t spread(uint32_t u) { return u ^ ((u >> 3) & 7u); }
+
+// `bytes` bytes at `src` (shared memory) to frame bytes [o, o + bytes), a
+// word of D.word bytes a lane, so that the warp's stores are consecutive.
+template <bool SPREAD, typename V>
+__device__ __forceinline__ void put_words(const FrameDst &D, uint64_t o, const uint8_t *src,
+                                          uint32_t bytes, int lane) {
+  constexpr uint32_t kRow = 32 * sizeof(V); // bytes the warp writes at a time
+  uint64_t col0;
+  uint8_t *row = frame_at(D, o, col0);
+  auto word = [&](uint32_t b) {
+    return *reinterpret_cast<const V *>(src + (SPREAD ? spread(b >> 4) * 16 + (b & 15u) : b));
+  };
+  if (D.row_bytes < kRow) {
+    for (uint32_t b = lane * sizeof(V); b < bytes; b += kRow) {
+      uint64_t col = col0 + b;
+      uint8_t *to = frame_row(D, row, col);
+      *reinterpret_cast<V *>(to + col) = word(b);
+    }
+    return;
+  }
+  // the lane's word crosses at most one row's end from each of its words to
+  // the next
+  const uint64_t skip = D.pitch - D.row_bytes;
+  uint64_t col = col0 + lane * sizeof(V);
+  uint8_t *to = row + col;
+  constexpr int kU = 4; // words in flight
+  for (uint32_t b0 = lane * sizeof(V); b0 < bytes; b0 += kU * kRow) {
+    V v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; u++)
+      if (b0 + u * kRow < bytes)
+        v[u] = word(b0 + u * kRow);
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      if (col >= D.row_bytes) {
+        col -= D.row_bytes;
+        to += skip;
+      }
+      if (b0 + u * kRow < bytes)
+        *reinterpret_cast<V *>(to) = v[u];
+      col += kRow;
+      to += kRow;
+    }
+  }
+}
+template <bool SPREAD>
+__device__ __forceinline__ void put_all(const FrameDst &D, uint64_t o, const uint8_t *src,
+                                        uint32_t bytes, int lane) {
+  if (D.word == 4)
+    put_words<SPREAD, uint32_t>(D, o, src, bytes, lane);
+  else if (D.word == 2)
+    put_words<SPREAD, uint16_t>(D, o, src, bytes, lane);
+  else
+    put_words<SPREAD, uint8_t>(D, o, src, bytes, lane);
+}
+
+// A decoded bitshuffle block of n bytes at `buf`, back in element order, to
+// the frame: a lane takes a 32-bit word of every bit plane, which holds four
+// groups of eight elements, separates the groups by byte transposes, undoes
+// their bit transposes, and leaves their bytes in `bounce`, from which the
+// warp writes rows of consecutive words. (A lane storing its own 16 bytes
+// in the four-byte words the arena's alignment allows touched every sector
+// four times.)
+template <int E>
+__device__ __forceinline__ void store_planes(const uint8_t *buf, uint32_t n, uint8_t *bounce,
+                                             const FrameDst &D, uint64_t o, int lane) {
+  const uint32_t plane = n / (8 * E);
+  if constexpr (E == 2 || E == 4) {
+    if ((plane & 3u) == 0) {
+      const uint32_t words = plane / 4;
+      for (uint32_t base = 0; base < words; base += 32) {
+        const uint32_t wd = base + lane;
+        if (wd < words) {
+          uint32_t y[4][2 * E];
+#pragma unroll
+          for (int j = 0; j < 2 * E; j++) {
+            uint32_t x[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              x[k] = *reinterpret_cast<const uint32_t *>(buf + (4 * j + k) * plane + 4 * wd);
+            const uint32_t t0 = __byte_perm(x[0], x[1], 0x5140);
+            const uint32_t t1 = __byte_perm(x[2], x[3], 0x5140);
+            const uint32_t t2 = __byte_perm(x[0], x[1], 0x7362);
+            const uint32_t t3 = __byte_perm(x[2], x[3], 0x7362);
+            y[0][j] = __byte_perm(t0, t1, 0x5410);
+            y[1][j] = __byte_perm(t0, t1, 0x7632);
+            y[2][j] = __byte_perm(t2, t3, 0x5410);
+            y[3][j] = __byte_perm(t2, t3, 0x7632);
+          }
+#pragma unroll
+          for (int g = 0; g < 4; g++) {
+            uint32_t lo[E], hi[E], w[2 * E];
+#pragma unroll
+            for (int j = 0; j < E; j++) {
+              lo[j] = y[g][2 * j];
+              hi[j] = y[g][2 * j + 1];
+              transpose_halves(lo[j], hi[j]);
+            }
+            weave<E>(lo, hi, w);
+#pragma unroll
+            for (int h = 0; h < E / 2; h++)
+              reinterpret_cast<uint4 *>(bounce)[spread((4 * lane + g) * (E / 2) + h)] =
+                  make_uint4(w[4 * h], w[4 * h + 1], w[4 * h + 2], w[4 * h + 3]);
+          }
+        }
+        __syncwarp();
+        put_all<true>(D, o + 32ull * E * base, bounce, min(32u, words - base) * 32 * E, lane);
+        __syncwarp();
+      }
+      return;
+    }
+  }
+  for (uint32_t g = lane; g < plane; g += 32) {
+    uint32_t w[8];
+    untranspose<E>(buf, plane, g, w);
+    put(D, o + 8ull * E * g, 8 * E, w);
+  }
+}
+
+// Blocks of a chunk, one warp each, grid-strided. Each warp owns a piece of
+// the shared memory (warp_layout) for the decoded block, its compressed
+// bytes and the decode's tables. E > 0: bitshuffle blocks of E-byte
+// elements, un-transposed on the way out; E == 0: plain LZ4. Warp 0 of block
+// 0 also copies the chunk's raw tail (elements after the last block).
 template <int E>
 __global__ void __launch_bounds__(kDecodeWarps * 32, 1)
     decode_blocks(const uint8_t *__restrict__ chunk, const BlockDesc *__restrict__ blocks,
                   uint32_t nblocks, uint32_t out_bytes, uint32_t stage_bytes, FrameDst D,
                   uint64_t raw_in, uint32_t raw_bytes, uint64_t raw_out, int *err) {
   extern __shared__ __align__(16) uint8_t decode_smem[];
-  __shared__ ModTable mt;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t list_bytes = list_bytes_for(stage_bytes);
-  uint8_t *obuf =
-      decode_smem + static_cast<size_t>(warp) * (out_bytes + stage_bytes + list_bytes);
-  uint8_t *ibuf = obuf + out_bytes;
-  uint16_t *list = reinterpret_cast<uint16_t *>(ibuf + stage_bytes);
-  for (uint32_t i = threadIdx.x; i < 32 * 32; i += blockDim.x) {
-    const uint32_t d = i >> 5, l = i & 31;
-    mt.lane_mod[d][l] = static_cast<uint8_t>(d ? l % d : 0);
-    if (l == 0)
-      mt.step[d] = static_cast<uint8_t>(d ? 32 % d : 0);
-  }
-  __syncthreads();
+  const WarpLayout W = warp_layout(out_bytes, stage_bytes, E);
+  uint8_t *obuf = decode_smem + static_cast<size_t>(warp) * W.total;
+  uint8_t *ibuf = obuf + W.out + W.extra;
+  uint16_t *list = reinterpret_cast<uint16_t *>(ibuf + W.stage);
+  uint32_t *ends = reinterpret_cast<uint32_t *>(ibuf + W.stage + W.list);
+  uint2 *rec = reinterpret_cast<uint2 *>(ibuf + W.stage + W.list + W.ends);
+  uint32_t *starts = reinterpret_cast<uint32_t *>(rec + kGroupSeqs);
   if (blockIdx.x == 0 && warp == 0) {
     for (uint32_t i = lane; i < raw_bytes; i += 32) {
       uint64_t col;
@@ -452,34 +748,23 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, 1)
       for (uint32_t i = lane; i < nvec; i += 32)
         sm[i] = __ldg(g + i);
       __syncwarp();
-      ok = 2 * d.len <= out_bytes
-               ? warp_lz4_parallel(ibuf + skew, d.len, reinterpret_cast<uint16_t *>(obuf), list,
-                                   obuf, d.n, lane, mt)
-               : warp_lz4(ibuf + skew, d.len, obuf, d.n, lane);
+      ok = warp_lz4_parallel(obuf, W.out + W.extra + skew, d.len,
+                             reinterpret_cast<uint16_t *>(obuf), list, ends, rec, starts, d.n,
+                             lane);
     } else {
       ok = warp_lz4(chunk + d.in, d.len, obuf, d.n, lane);
     }
+    __syncwarp();
     if (!ok) {
       if (lane == 0)
         atomicExch(err, 1);
       __syncwarp();
       continue;
     }
-    if constexpr (E > 0) {
-      const uint32_t plane = d.n / (8 * E);
-      for (uint32_t g = lane; g < plane; g += 32) {
-        uint32_t w[8];
-        untranspose<E>(obuf, plane, g, w);
-        put(D, d.out + 8ull * E * g, 8 * E, w);
-      }
-    } else {
-      const uint32_t pieces = (d.n + 15) / 16;
-      for (uint32_t p = lane; p < pieces; p += 32) {
-        const uint4 v = reinterpret_cast<const uint4 *>(obuf)[p];
-        uint32_t w[8] = {v.x, v.y, v.z, v.w, 0, 0, 0, 0};
-        put(D, d.out + 16ull * p, min(16u, d.n - 16 * p), w);
-      }
-    }
+    if constexpr (E > 0)
+      store_planes<E>(obuf, d.n, obuf + W.out, D, d.out, lane);
+    else
+      put_all<false>(D, d.out, obuf, d.n, lane);
     __syncwarp();
   }
 }
@@ -528,7 +813,10 @@ template <typename T> void grow(T **p, size_t &cap, size_t bytes, const char *wh
 
 template <int E> void configure_decoder() {
   check(cudaFuncSetAttribute(decode_blocks<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kDecodeWarps * kWarpSmemMax)),
+                             static_cast<int>(kDecodeWarps *
+                                              warp_layout(static_cast<uint32_t>(kMaxBlockBytes),
+                                                          kStageCap + 16, E)
+                                                  .total)),
         "cudaFuncSetAttribute");
 }
 
@@ -717,15 +1005,17 @@ void DeviceChunkDecoder::enqueue(const uint8_t *chunk, size_t nbytes, const Chun
   }
   const uint32_t out_bytes = static_cast<uint32_t>(round16(std::max<uint64_t>(L.block_bytes, 16)));
   const uint32_t stage_bytes = static_cast<uint32_t>(round16(std::min(max_len, kStageCap) + 15));
-  const size_t smem =
-      static_cast<size_t>(kDecodeWarps) * (out_bytes + stage_bytes + list_bytes_for(stage_bytes));
+  const int e = bs ? static_cast<int>(L.elem) : 0;
+  const size_t smem = static_cast<size_t>(kDecodeWarps) *
+                      warp_layout(out_bytes, stage_bytes, static_cast<uint32_t>(e)).total;
   const unsigned grid = static_cast<unsigned>(std::max<size_t>(
       1, std::min<size_t>((nb + kDecodeWarps - 1) / kDecodeWarps,
                           static_cast<size_t>(device_sm_count()) * 16)));
-  const FrameDst D{static_cast<uint8_t *>(dst), dst_pitch, row_bytes};
+  const uint64_t ways = reinterpret_cast<uintptr_t>(dst) | dst_pitch | row_bytes | L.block_bytes;
+  const FrameDst D{static_cast<uint8_t *>(dst), dst_pitch, row_bytes,
+                   ways % 4 == 0 ? 4u : ways % 2 == 0 ? 2u : 1u};
   const uint64_t raw_out = frame_bytes - L.raw_bytes;
   const uint32_t raw32 = static_cast<uint32_t>(L.raw_bytes);
-  const int e = bs ? static_cast<int>(L.elem) : 0;
   if (e == 0)
     decode_blocks<0><<<grid, kDecodeWarps * 32, smem, s>>>(S.d_in, tbl, n32, out_bytes,
                                                            stage_bytes, D, L.raw_in, raw32,
