@@ -7,36 +7,43 @@
 // and be captured in the same CUDA graph:
 //
 //   setup     frame segments of the live set: the carry's last frame, then
-//             the batch frames; live size n
+//             the batch frames; live size n; the block tables cleared
 //   gather    the batch's signal lists appended after the carried pixels,
-//             so the live set is in (frame, index) order; per-root fields
-//             cleared
+//             so the live set is in (frame, index) order; the per-root
+//             words of every position that can become a root cleared
 //   link      left, up and previous-frame neighbours joined by a lock-free
 //             union-find that links toward the lower position, so a root is
 //             its component's first pixel in (frame, index) order
-//   flatten   root of every pixel; component size and last frame
-//   mark      finished roots (no pixel on the batch's last frame) as a
-//             bitmap, with a count per 32-position word
-//   scan      of the counts
-//   compact   the finished roots, in position order
+//   flatten   root of every pixel, as a bitmap too; component size and last
+//             frame; the last frame's block table kept for the next batch
+//   close     the finished roots (no pixel on the batch's last frame), in
+//             position order
 //   count     per 32 roots of that list, how many close on each frame
 //             (last-frame bucket)
 //   scan      of those counts, bucket-major: the reference's emission order
 //             is (last frame, first pixel), which is exactly bucket then
 //             position
-//   rank      each finished component's emission rank; size filters
-//   scan      member offsets of the components that pass the size filters
+//   rank      each finished component's emission rank; size filters; room
+//             for the members of the components that pass them
 //   scatter   members, in any order; the open pixels (their component is
 //             not finished) as a bitmap with a count per 32 positions
+//   scan      of the open counts
 //   accept    per component: members sorted by position (so (frame, index)
 //             order), then the FP64 pass in that order, peak-centroid
 //             filter
 //   scan      output rows and pixel offsets of the accepted spots
 //   write     spots and their pixels
-//   scan      of the open counts
 //   carry     the open components' pixels compacted, in order, into
-//             the other live buffer and re-rooted at their first pixel
-//   finalize  running counts and the carry for the next batch
+//             the other live buffer and re-rooted at their first pixel;
+//             running counts and the carry for the next batch
+//
+// close and each scan are one launch (sf_lookback.cuh), where a scan was
+// three: a batch took 32 launches and takes 16, and a one-frame batch is bound
+// by them. (scatter and write finding their places the same way, without the
+// scans before them, were slower: 109 against 57 + 8 us and 82 against
+// 60 + 8 for 16 frames of 4362 x 4148, 15 and 17 against 9 for one of
+// 2162 x 2068: every tile waits for its first loads, then for its prefix,
+// before its copies.)
 //
 // Every loop here walks a bounded range; union-find paths strictly decrease
 // in position, so no loop depends on another thread making progress.
@@ -45,19 +52,26 @@
 #include <cstddef>
 
 #include "sf_label.hh"
+#include "sf_lookback.cuh"
 
 namespace sf {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr uint32_t kNone = 0xffffffffu;
-constexpr int kThreads = 256;
+constexpr uint32_t kDropped = 0xfffffffeu; // RootInfo::slot of a component the size filter removed
+constexpr int kThreads = kTileThreads;
 // Components up to kSmallCap members take lab_accept's launch with small
 // per-warp buffers (many warps per SM); the larger ones are listed by
 // lab_rank in two lists, up to kMidCap members and beyond, and taken by
 // launches with larger buffers.
 constexpr uint32_t kSmallCap = 256;
 constexpr uint32_t kMidCap = 512;
+// 32-position words a warp of lab_scatter takes at a time.
+constexpr int kScatterWords = 4;
+// The spots' scan packs pixels above rows, neither of which reaches 2^31.
+constexpr int kPackShift = 31;
+constexpr uint64_t kPackLow = (1ull << kPackShift) - 1;
 // The least a growing labeller makes room for: 16 Ki pixels, 3 MB.
 constexpr uint64_t kRoomPixels = 16384;
 
@@ -104,19 +118,19 @@ struct LabArgs {
   uint32_t *ix, *val, *par;
   int32_t *nfr;
   uint32_t *nix, *nval, *npar;
-  uint32_t *root, *size;
-  int32_t *lastz;
-  uint32_t *rank_of_root, *cursor;
-  uint32_t *bits, *bcnt; // finished-root bitmap; word counts, then bucket counts
+  uint32_t *root;
+  RootInfo *info;
+  uint32_t *bits, *bcnt; // root bitmap; bucket counts
   uint32_t *flist;       // the finished roots in position order
   uint32_t *comp_root, *msize, *members;
-  uint64_t *mpk;
+  uint64_t *mpk, *pack;
   uint4 *runs; // per batch: lab_link's entries, see lab_gather
   uint32_t *run_starts; // bit p & 31 of word p >> 5: position p starts a run
   Spot *spot_tmp;
   Pixel *pix_tmp;
-  uint64_t *pack;
-  uint32_t *obits, *ocnt; // open pixels: bitmap and (scanned) count per 32 positions
+  uint32_t *obits, *ocnt; // open pixels: bitmap, and how many before each 32 positions
+  // the lookbacks' words, per tile
+  uint64_t *close_st, *count_st, *open_st, *pack_st;
   uint32_t *big; // ranks of the kept components with more than kMidCap members
   uint32_t *mid; // ... with more than kSmallCap and at most kMidCap
   Spot *spots;
@@ -200,62 +214,108 @@ __device__ __forceinline__ int segment_of(const uint64_t *seg_start, int nseg, u
   return lo;
 }
 
-__device__ __forceinline__ int bucket_of(const int64_t *seg_z, int nseg, int64_t z) {
-  int lo = 0, hi = nseg - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (seg_z[mid] <= z)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
-}
-
 __device__ __forceinline__ int64_t last_batch_frame(const LabArgs &a) {
   return a.sc->batch_z0 + a.nframes - 1;
 }
 
-// A root whose component is finished by this batch.
-__device__ __forceinline__ bool finished_root(const LabArgs &a, uint64_t g, uint64_t n) {
-  if (g >= n || a.root[g] != g)
-    return false;
+// The bucket (frame segment) a component with last frame z closes in: the
+// carry's, if any, comes first, then the batch's consecutive frames.
+__device__ __forceinline__ int bucket_of(const LabelScalars *sc, int32_t z) {
+  const int64_t f = static_cast<int64_t>(z) - sc->batch_z0;
+  const int64_t last = static_cast<int64_t>(sc->nseg) - 1;
+  if (f < 0)
+    return 0;
+  return static_cast<int>(min(f + (sc->carry_n > 0 ? 1 : 0), last));
+}
+
+// Whether a root's component is finished by this batch.
+__device__ __forceinline__ bool finished(const LabArgs &a, int32_t lastz) {
   if (a.close_all || a.two_d || a.nframes == 0)
     return true;
-  return static_cast<int64_t>(a.lastz[g]) < last_batch_frame(a);
+  return static_cast<int64_t>(lastz) < last_batch_frame(a);
+}
+
+// Exclusive prefix of a value per thread over the block's kThreads threads;
+// *total gets the sum.
+__device__ __forceinline__ uint64_t block_prefix(uint64_t v, uint64_t *total) {
+  __shared__ uint64_t sums[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t t = __shfl_up_sync(kFull, incl, d);
+    if (lane >= d)
+      incl += t;
+  }
+  if (lane == 31)
+    sums[warp] = incl;
+  __syncthreads();
+  uint64_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; w++) {
+    if (w < warp)
+      before += sums[w];
+    all += sums[w];
+  }
+  __syncthreads();
+  *total = all;
+  return before + incl - v;
 }
 
 // --------------------------------------------------------------------------
 
-__global__ void lab_setup(LabArgs a) {
-  if (threadIdx.x != 0 || blockIdx.x != 0)
+// Block 0's first warp lays out the frame segments; every block clears its
+// share of the batch frames' block tables.
+__global__ void __launch_bounds__(kThreads) lab_setup(LabArgs a) {
+  const uint64_t words = static_cast<uint64_t>(a.nframes) * a.nblk;
+  for (uint64_t i = gtid(); i < words / 4; i += gstride())
+    reinterpret_cast<uint4 *>(a.tab)[i] = make_uint4(kNone, kNone, kNone, kNone);
+  if (gtid() < words % 4)
+    a.tab[words - 1 - gtid()] = kNone;
+  if (blockIdx.x != 0 || threadIdx.x >= 32)
     return;
+  const int lane = threadIdx.x;
   LabelScalars *sc = a.sc;
   const uint64_t carry = sc->carry_n;
-  int nseg = 0;
-  if (carry > 0) {
+  const int64_t z0 = sc->batch_z0;
+  const int first = carry > 0 ? 1 : 0;
+  if (lane == 0 && first) {
     a.seg_z[0] = sc->carry_last_z;
     a.seg_start[0] = sc->carry_last_start;
     a.seg_count[0] = carry - sc->carry_last_start;
-    nseg = 1;
   }
   uint64_t pos = carry;
-  for (int f = 0; f < a.nframes; f++) {
-    uint32_t c = a.counts[a.count_map ? a.count_map[f] : f];
-    if (c > a.caps[f]) // an over-dense frame: its list holds only this many
-      c = a.caps[f];
-    if (pos + c > a.live_cap) {
-      sc->status = kLabelLiveOverflow;
-      c = static_cast<uint32_t>(a.live_cap - pos);
+  bool over = false;
+  for (int f0 = 0; f0 < a.nframes; f0 += 32) {
+    const int f = f0 + lane;
+    uint64_t c = 0;
+    if (f < a.nframes) // an over-dense frame: its list holds only caps[f]
+      c = min(a.counts[a.count_map ? a.count_map[f] : f], a.caps[f]);
+    uint64_t incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t t = __shfl_up_sync(kFull, incl, d);
+      if (lane >= d)
+        incl += t;
     }
-    a.seg_z[nseg] = sc->batch_z0 + f;
-    a.seg_start[nseg] = pos;
-    a.seg_count[nseg] = c;
-    pos += c;
-    nseg++;
+    over = over || pos + incl > a.live_cap;
+    const uint64_t start = min(pos + incl - c, a.live_cap);
+    const uint64_t end = min(pos + incl, a.live_cap);
+    if (f < a.nframes) {
+      a.seg_z[first + f] = z0 + f;
+      a.seg_start[first + f] = start;
+      a.seg_count[first + f] = end - start;
+    }
+    pos = __shfl_sync(kFull, end, 31);
   }
+  over = __any_sync(kFull, over);
+  if (lane != 0)
+    return;
+  if (over)
+    sc->status = kLabelLiveOverflow;
+  int nseg = first + a.nframes;
   if (nseg == 0) { // nothing held and nothing added: one empty segment
-    a.seg_z[0] = sc->batch_z0;
+    a.seg_z[0] = z0;
     a.seg_start[0] = 0;
     a.seg_count[0] = 0;
     nseg = 1;
@@ -264,11 +324,13 @@ __global__ void lab_setup(LabArgs a) {
   sc->nw = (pos + 31) / 32;
   sc->nseg = nseg;
   sc->signal_pixels += pos - carry;
-  sc->closed32 = sc->open32 = 0;
+  sc->closed = sc->seg_len = 0;
+  sc->open32 = 0;
   sc->runs_n = 0;
   sc->big_n = 0;
   sc->mid_n = 0;
   sc->link_next = sc->accept_next = sc->big_next = sc->mid_next = 0;
+  sc->close_next = sc->count_next = sc->open_next = sc->pack_next = 0;
   sc->members_pack = 0;
   sc->accepted_pack = 0;
 }
@@ -287,8 +349,10 @@ __device__ __forceinline__ const uint32_t *table_of(const LabArgs &a, int s, int
   return s < first_batch_seg ? a.carry_tab : a.tab + static_cast<uint64_t>(s - first_batch_seg) * a.nblk;
 }
 
-// The new pixels' lists are copied after the carried pixels; per-root
-// fields are cleared. Each new pixel's parent is set to the first pixel of
+// The new pixels' lists are copied after the carried pixels; the per-root
+// words are cleared where a root can come to be: at the carried pixels and
+// at the first pixel of each piece of a run (no other pixel is ever its own
+// parent), about a third of the pixels. Each new pixel's parent is set to the first pixel of
 // its horizontal run (left neighbours, src/dials_spots.cc:106-110) within its
 // 32-aligned chunk of positions, found with one ballot, so that the trees
 // start one level deep; a run that enters a chunk from the previous one is
@@ -310,6 +374,10 @@ __global__ void __launch_bounds__(kThreads) lab_gather(LabArgs a) {
       sh_start[k] = a.seg_start[k];
       sh_z[k] = a.seg_z[k];
     }
+  // the lookback words of lab_close and of the open counts' scan
+  for (uint64_t t = gtid(); t * kThreads < sc->nw; t += gstride())
+    a.close_st[t] = 0;
+  clear_scan_words(a.open_st, sc->nw, gtid(), gstride());
   __syncthreads();
   const uint64_t *seg_start = in_shared ? sh_start : a.seg_start;
   const int64_t *seg_z = in_shared ? sh_z : a.seg_z;
@@ -322,10 +390,6 @@ __global__ void __launch_bounds__(kThreads) lab_gather(LabArgs a) {
     int seg = 0;       // a new pixel's frame segment
     uint32_t pidx = 0; // and its index, for the work list
     if (g < n) {
-      a.size[g] = 0;
-      a.lastz[g] = INT_MIN;
-      a.rank_of_root[g] = kNone;
-      a.cursor[g] = 0;
       if (g >= carry) {
         const int s = segment_of(seg_start, nseg, g);
         seg = s;
@@ -370,6 +434,8 @@ __global__ void __launch_bounds__(kThreads) lab_gather(LabArgs a) {
     // 16-byte load
     const bool boundary = left && lane == 0;
     const bool entry = mine && (!left || boundary);
+    if (entry || g < min(carry, n))
+      a.info[g] = RootInfo{0u, INT_MIN, kNone, 0u};
     const uint32_t want = __ballot_sync(kFull, entry);
     // pieces end at the next piece, at a lane that is not ours, or at the
     // chunk's end
@@ -550,16 +616,6 @@ __global__ void __launch_bounds__(kThreads) lab_link(LabArgs a) {
   }
 }
 
-// After the batch: the last frame's table becomes the carry's, since every
-// pixel of the last frame is carried, in the same order.
-__global__ void __launch_bounds__(kThreads) lab_keep_table(LabArgs a) {
-  if (a.nframes == 0 || a.close_all || a.two_d)
-    return;
-  const uint32_t *last = a.tab + static_cast<uint64_t>(a.nframes - 1) * a.nblk;
-  for (uint64_t b = gtid(); b < a.nblk; b += gstride())
-    a.carry_tab[b] = last[b];
-}
-
 // Roots, component sizes and last frames. A warp's lanes hold 32
 // consecutive positions; each stretch of adjacent lanes with one root (a
 // run, mostly) makes one update. Positions are in (frame, index) order, so
@@ -577,6 +633,9 @@ __global__ void __launch_bounds__(kThreads) lab_flatten(LabArgs a) {
       r = uf_root(a.par, static_cast<uint32_t>(g)); // lab_link is done: no more links
       a.root[g] = r;
     }
+    const uint32_t roots = __ballot_sync(kFull, r == static_cast<uint32_t>(g));
+    if (lane == 0)
+      a.bits[base >> 5] = roots;
     const uint32_t before = __shfl_up_sync(kFull, r, 1);
     const bool head = lane == 0 || before != r;
     const uint32_t heads = __ballot_sync(kFull, head);
@@ -585,43 +644,44 @@ __global__ void __launch_bounds__(kThreads) lab_flatten(LabArgs a) {
     const int end = later ? __ffs(later) - 2 : 31;
     const int32_t zlast = __shfl_sync(kFull, z, end);
     if (head && r != kNone) {
-      atomicAdd(&a.size[r], static_cast<uint32_t>(end - lane + 1));
-      atomicMax(&a.lastz[r], zlast);
+      atomicAdd(&a.info[r].size, static_cast<uint32_t>(end - lane + 1));
+      atomicMax(&a.info[r].lastz, zlast);
     }
+  }
+  // the last frame's block table becomes the carry's, since every pixel of
+  // the last frame is carried, in the same order (lab_link was its last use)
+  if (a.nframes > 0 && !a.close_all && !a.two_d) {
+    const uint32_t *table = a.tab + static_cast<uint64_t>(a.nframes - 1) * a.nblk;
+    for (uint64_t b = gtid(); b < a.nblk; b += gstride())
+      a.carry_tab[b] = table[b];
   }
 }
 
-__global__ void __launch_bounds__(kThreads) lab_mark(LabArgs a) {
-  const LabelScalars *sc = a.sc;
-  const uint64_t n = sc->n, nw = sc->nw;
-  const int lane = threadIdx.x & 31;
-  const uint64_t warp = gtid() >> 5, nwarps = gstride() >> 5;
-  for (uint64_t w = warp; w < nw; w += nwarps) {
-    const uint32_t m = __ballot_sync(kFull, finished_root(a, w * 32 + lane, n));
-    if (lane == 0) {
-      a.bits[w] = m;
-      a.bcnt[w] = __popc(m);
-    }
-  }
-}
-
-// The finished roots in position order, from the bitmap and the scanned
-// word counts (a thread per word: most words hold none, few more than one).
-// Also the length of the bucket-count table that the next scan covers.
-__global__ void __launch_bounds__(kThreads) lab_compact(LabArgs a) {
+// The finished roots in position order, a thread per bitmap word (most words
+// hold none, few more than one), kThreads words a tile; a tile's place in
+// the list comes from the tiles before it. The last tile knows how many
+// there are.
+__global__ void __launch_bounds__(kThreads) lab_close(LabArgs a) {
   LabelScalars *sc = a.sc;
   const uint64_t nw = sc->nw;
-  if (gtid() == 0) {
-    const uint64_t closed = sc->closed32;
-    sc->closed = closed;
-    sc->seg_len = sc->nseg * ((closed + 31) / 32);
-  }
-  for (uint64_t w = gtid(); w < nw; w += gstride()) {
-    uint32_t m = a.bits[w];
-    uint32_t at = a.bcnt[w];
-    while (m) {
+  const uint64_t tiles = (nw + kThreads - 1) / kThreads;
+  __shared__ TileTurn turn;
+  while (next_tile(&turn, &sc->close_next, tiles)) {
+    const uint64_t w = turn.tile * kThreads + threadIdx.x;
+    uint32_t roots = w < nw ? a.bits[w] : 0u, m = 0;
+    for (; roots; roots &= roots - 1) {
+      const int k = __ffs(roots) - 1;
+      if (finished(a, a.info[w * 32 + k].lastz))
+        m |= 1u << k;
+    }
+    uint64_t total;
+    const uint64_t mine = block_prefix(__popc(m), &total);
+    const uint64_t before = tile_prefix(&turn, a.close_st, total, &sc->status);
+    for (uint64_t at = before + mine; m; m &= m - 1)
       a.flist[at++] = static_cast<uint32_t>(w * 32 + __ffs(m) - 1);
-      m &= m - 1;
+    if (turn.tile == tiles - 1 && threadIdx.x == 0) {
+      sc->closed = before + total;
+      sc->seg_len = sc->nseg * ((before + total + 31) / 32);
     }
   }
 }
@@ -634,9 +694,12 @@ __global__ void __launch_bounds__(kThreads) lab_count(LabArgs a) {
   const int nseg = static_cast<int>(sc->nseg);
   const int lane = threadIdx.x & 31;
   const uint64_t warp = gtid() >> 5, nwarps = gstride() >> 5;
+  // the lookback words of the scans of these counts and of the spots
+  clear_scan_words(a.count_st, sc->seg_len, gtid(), gstride());
+  clear_scan_words(a.pack_st, closed, gtid(), gstride());
   for (uint64_t j = warp; j < groups; j += nwarps) {
     const uint64_t k = j * 32 + lane;
-    const int b = k < closed ? bucket_of(a.seg_z, nseg, a.lastz[a.flist[k]]) : -1;
+    const int b = k < closed ? bucket_of(sc, a.info[a.flist[k]].lastz) : -1;
     for (int s = 0; s < nseg; s++) {
       const uint32_t m = __ballot_sync(kFull, b == s);
       if (lane == 0)
@@ -645,10 +708,12 @@ __global__ void __launch_bounds__(kThreads) lab_count(LabArgs a) {
   }
 }
 
+// Emission ranks; and for each component that passes the size filters a
+// place for its members and its spot, claimed a warp at a time: they are
+// scratch, so their order does not matter.
 __global__ void __launch_bounds__(kThreads) lab_rank(LabArgs a) {
   LabelScalars *sc = a.sc;
   const uint64_t closed = sc->closed, groups = (closed + 31) / 32;
-  const int nseg = static_cast<int>(sc->nseg);
   const int lane = threadIdx.x & 31;
   const uint64_t warp = gtid() >> 5, nwarps = gstride() >> 5;
   uint32_t small = 0, large = 0;
@@ -656,19 +721,36 @@ __global__ void __launch_bounds__(kThreads) lab_rank(LabArgs a) {
     const uint64_t k = j * 32 + lane;
     const bool valid = k < closed;
     const uint32_t g = valid ? a.flist[k] : 0u;
-    const int b = valid ? bucket_of(a.seg_z, nseg, a.lastz[g]) : -1;
+    const RootInfo info = valid ? a.info[g] : RootInfo{0u, 0, kNone, 0u};
+    const int b = valid ? bucket_of(sc, info.lastz) : -1;
     // earlier roots of this group in the same bucket come first
     const uint32_t peers = __match_any_sync(kFull, b);
+    const uint32_t size = info.size;
+    const bool keep = valid && size >= a.min_size && size <= a.max_size;
+    const uint32_t kept = __ballot_sync(kFull, keep);
+    uint32_t incl = keep ? size : 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, incl, d);
+      if (lane >= d)
+        incl += t;
+    }
+    uint64_t base = 0; // members (low 32) | components (high 32)
+    if (lane == 31 && kept)
+      base = atomicAdd(reinterpret_cast<unsigned long long *>(&sc->members_pack),
+                       static_cast<unsigned long long>(incl) |
+                           (static_cast<unsigned long long>(__popc(kept)) << 32));
+    base = __shfl_sync(kFull, base, 31);
     if (!valid)
       continue;
     const uint32_t rank =
         a.bcnt[b * groups + j] + __popc(peers & ((1u << lane) - 1u));
-    a.rank_of_root[g] = rank;
     a.comp_root[rank] = g;
-    const uint32_t size = a.size[g];
-    const bool keep = size >= a.min_size && size <= a.max_size;
     a.msize[rank] = keep ? size : 0u;
-    a.mpk[rank] = keep ? (static_cast<uint64_t>(size) | (1ull << 32)) : 0ull;
+    const uint32_t moff = static_cast<uint32_t>(base) + incl - (keep ? size : 0u);
+    const uint32_t sidx = static_cast<uint32_t>(base >> 32) + __popc(kept & ((1u << lane) - 1u));
+    a.mpk[rank] = moff | (static_cast<uint64_t>(sidx) << 32);
+    a.info[g].slot = keep ? moff : kDropped;
     if (keep && size > kMidCap)
       a.big[atomicAdd(&sc->big_n, 1u)] = rank;
     else if (keep && size > kSmallCap)
@@ -676,54 +758,56 @@ __global__ void __launch_bounds__(kThreads) lab_rank(LabArgs a) {
     small += size < a.min_size;
     large += size > a.max_size;
   }
-  if (small)
+  small = __reduce_add_sync(kFull, small);
+  large = __reduce_add_sync(kFull, large);
+  if (lane == 0 && small)
     atomicAdd(reinterpret_cast<unsigned long long *>(&sc->too_small), small);
-  if (large)
+  if (lane == 0 && large)
     atomicAdd(reinterpret_cast<unsigned long long *>(&sc->too_large), large);
 }
 
 // Member lists, and the open pixels (their component is not finished by
-// this batch, so they are carried) as a bitmap and count per 32 positions. A warp takes 32 consecutive
-// positions; the lanes of one component claim their slots with one atomic
-// and fill them in lane order.
+// this batch, so they are carried) as a bitmap and count per 32 positions.
+// A warp takes kScatterWords times 32 consecutive positions at a time, their
+// roots' words read together; the lanes of one component claim their slots
+// with one atomic and fill them in lane order.
 // So each component's list is a set of runs, one per 32-position chunk it
 // has pixels in, each run ascending and within its chunk; lab_accept orders
 // the runs rather than the members.
 __global__ void __launch_bounds__(kThreads) lab_scatter(LabArgs a) {
-  const uint64_t n = a.sc->n;
+  const uint64_t n = a.sc->n, nw = a.sc->nw;
   const int lane = threadIdx.x & 31;
   const uint64_t warps = gstride() >> 5;
-  for (uint64_t base = (gtid() >> 5) * 32; base < n; base += warps * 32) {
-    const uint64_t g = base + lane;
-    uint32_t r = kNone, rank = kNone, moff = 0;
-    bool open = false;
-    if (g < n) {
-      r = a.root[g];
-      rank = a.rank_of_root[r];
-      open = rank == kNone; // not finished by this batch: carried
-      if (rank != kNone) {
-        // the component's size and member offset read together
-        const uint32_t size = a.msize[rank];
-        moff = static_cast<uint32_t>(a.mpk[rank]);
-        if (size == 0)
-          rank = kNone;
+  for (uint64_t w0 = (gtid() >> 5) * kScatterWords; w0 < nw; w0 += warps * kScatterWords) {
+    uint32_t r[kScatterWords], slot[kScatterWords];
+#pragma unroll
+    for (int i = 0; i < kScatterWords; i++) {
+      const uint64_t g = (w0 + i) * 32 + lane;
+      r[i] = g < n ? a.root[g] : kNone;
+    }
+#pragma unroll
+    for (int i = 0; i < kScatterWords; i++)
+      slot[i] = r[i] != kNone ? a.info[r[i]].slot : kDropped;
+#pragma unroll
+    for (int i = 0; i < kScatterWords; i++) {
+      const uint64_t g = (w0 + i) * 32 + lane;
+      const uint32_t open = __ballot_sync(kFull, slot[i] == kNone);
+      if (lane == 0 && w0 + i < nw) {
+        a.obits[w0 + i] = open;
+        a.ocnt[w0 + i] = __popc(open);
       }
+      const bool member = slot[i] < kDropped;
+      const uint32_t peers = __match_any_sync(kFull, member ? r[i] : kNone);
+      if (member) {
+        const int leader = __ffs(peers) - 1;
+        uint32_t at = 0;
+        if (lane == leader)
+          at = atomicAdd(&a.info[r[i]].cursor, static_cast<uint32_t>(__popc(peers)));
+        at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
+        a.members[slot[i] + at] = static_cast<uint32_t>(g);
+      }
+      __syncwarp();
     }
-    const uint32_t ob = __ballot_sync(kFull, open);
-    if (lane == 0) {
-      a.obits[base >> 5] = ob;
-      a.ocnt[base >> 5] = __popc(ob);
-    }
-    const uint32_t key = rank == kNone ? kNone : r;
-    const uint32_t peers = __match_any_sync(kFull, key);
-    if (key == kNone)
-      continue;
-    const int leader = __ffs(peers) - 1;
-    uint32_t at = 0;
-    if (lane == leader)
-      at = atomicAdd(&a.cursor[r], static_cast<uint32_t>(__popc(peers)));
-    at = __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
-    a.members[moff + at] = static_cast<uint32_t>(g);
   }
 }
 
@@ -1413,10 +1497,8 @@ __global__ void __launch_bounds__(kCompWarps * 32, kAcceptBlocks<CAP>)
       if (!ok) {
         separated++;
         a.msize[r] = 0;
-        a.pack[r] = 0;
-      } else {
-        a.pack[r] = (static_cast<uint64_t>(n) << 32) | 1u;
       }
+      a.pack[r] = ok ? (static_cast<uint64_t>(n) << kPackShift) | 1u : 0u;
     }
     __syncwarp();
   }
@@ -1424,22 +1506,25 @@ __global__ void __launch_bounds__(kCompWarps * 32, kAcceptBlocks<CAP>)
     atomicAdd(reinterpret_cast<unsigned long long *>(&sc->separated), separated);
 }
 
-// The accepted spots to their rows and their pixels to the kept list.
+// The accepted spots to their rows and their pixels to the kept list, a warp
+// a spot: the row and the first kWriteWords * 32 words of the pixels read
+// together, before any is stored.
 __global__ void __launch_bounds__(kThreads) lab_write(LabArgs a) {
   LabelScalars *sc = a.sc;
   const uint64_t closed = sc->closed;
   const uint64_t kept_base = sc->kept_total;
   const int lane = threadIdx.x & 31;
   const uint64_t gw = gtid() >> 5, nw = gstride() >> 5;
+  constexpr uint32_t kWriteWords = 6;
   static_assert(offsetof(Spot, first) == 96, "Spot::first is the row's last word");
+  static_assert(sizeof(Pixel) == 12, "a pixel is three words");
   for (uint64_t r = gw; r < closed; r += nw) {
     // the component's three words read together, not one after another
     const uint32_t n = a.msize[r];
     const uint64_t pk = a.pack[r], mp = a.mpk[r];
     if (n == 0)
       continue;
-    const uint64_t row = pk & 0xffffffffu;
-    const uint64_t pix = pk >> 32;
+    const uint64_t row = pk & kPackLow, pix = pk >> kPackShift;
     const uint32_t moff = static_cast<uint32_t>(mp);
     const uint32_t sidx = static_cast<uint32_t>(mp >> 32);
     if (row >= a.spot_cap || sidx >= a.spot_cap || pix + n > a.live_cap) {
@@ -1448,26 +1533,39 @@ __global__ void __launch_bounds__(kThreads) lab_write(LabArgs a) {
       continue;
     }
     // the 104-byte row as 13 words, one a lane; the last is Spot::first
-    if (lane < 13) {
-      const uint64_t *src = reinterpret_cast<const uint64_t *>(a.spot_tmp + sidx);
-      uint64_t *dst = reinterpret_cast<uint64_t *>(a.spots + row);
-      dst[lane] = lane == 12 ? kept_base + pix : src[lane];
+    uint64_t word = kept_base + pix;
+    if (lane < 12)
+      word = reinterpret_cast<const uint64_t *>(a.spot_tmp + sidx)[lane];
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(a.pix_tmp + moff);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(a.kept + pix);
+    const uint32_t words = 3 * n;
+    for (uint32_t w0 = lane; w0 < words; w0 += 32 * kWriteWords) {
+      uint32_t v[kWriteWords];
+#pragma unroll
+      for (uint32_t u = 0; u < kWriteWords; u++)
+        if (w0 + 32 * u < words)
+          v[u] = src[w0 + 32 * u];
+#pragma unroll
+      for (uint32_t u = 0; u < kWriteWords; u++)
+        if (w0 + 32 * u < words)
+          dst[w0 + 32 * u] = v[u];
     }
-    for (uint32_t k = lane; k < n; k += 32)
-      a.kept[pix + k] = a.pix_tmp[moff + k];
+    if (lane < 13)
+      reinterpret_cast<uint64_t *>(a.spots + row)[lane] = word;
   }
 }
 
-
-// Where an open pixel lands in the carry: the scanned count of open pixels
-// in the 32-position words before its own, plus the open ones before it in
-// its word.
+// Where an open pixel lands in the carry: the open pixels in the
+// 32-position words before its own, plus the open ones before it in its
+// word.
 __device__ __forceinline__ uint32_t open_position(const LabArgs &a, uint64_t g) {
   return a.ocnt[g >> 5] + __popc(a.obits[g >> 5] & ((1u << (g & 31)) - 1u));
 }
 
 // The open pixels to the other live buffer, in order, a warp per
-// 32-position word (most words hold none).
+// 32-position word (most words hold none). One thread closes the batch's
+// books, none of which the other blocks read: the running counts and what
+// the next batch starts from.
 __global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
   LabelScalars *sc = a.sc;
   const uint64_t nw = sc->nw;
@@ -1485,16 +1583,12 @@ __global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
     a.nval[at] = a.val[g];
     a.npar[at] = open_position(a, r); // the root is open too, and comes first
   }
-}
-
-__global__ void lab_finalize(LabArgs a) {
-  if (threadIdx.x != 0 || blockIdx.x != 0)
+  if (gtid() != 0)
     return;
-  LabelScalars *sc = a.sc;
   const bool all = a.close_all || a.two_d || a.nframes == 0;
   sc->groups += sc->closed;
-  const uint64_t rows = sc->accepted_pack & 0xffffffffu;
-  const uint64_t pixels = sc->accepted_pack >> 32;
+  const uint64_t rows = sc->accepted_pack & kPackLow;
+  const uint64_t pixels = sc->accepted_pack >> kPackShift;
   sc->accepted += rows;
   sc->kept_total += pixels;
   sc->batch_spots = rows;
@@ -1567,8 +1661,9 @@ void DeviceLabeller::release() {
   for (Live &l : live_)
     l = Live();
   tab_ = nullptr;
-  root_ = size_ = rank_of_root_ = cursor_ = nullptr;
-  lastz_ = nullptr;
+  root_ = nullptr;
+  info_ = nullptr;
+  close_st_ = count_st_ = open_st_ = pack_st_ = nullptr;
   bits_ = bcnt_ = flist_ = comp_root_ = msize_ = members_ = obits_ = ocnt_ = big_ = mid_ = nullptr;
   mpk_ = pack_ = nullptr;
   runs_ = nullptr;
@@ -1648,20 +1743,17 @@ bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
     part(&l.parent, live);
   }
   part(&root_, live);
-  part(&size_, live);
-  part(&rank_of_root_, live);
-  part(&cursor_, live);
-  part(&lastz_, live);
-  part(&bits_, nwmax);                                // finished-root bitmap
+  part(&info_, live);
+  part(&bits_, nwmax);                                // root bitmap
   part(&bcnt_, static_cast<uint64_t>(fc + 1) * nwmax); // bucket counts
   part(&flist_, live);                                // finished roots
   part(&comp_root_, live);
   part(&msize_, live);
   part(&mpk_, live);
+  part(&pack_, live);
   part(&runs_, live);
   part(&run_starts_, live / 32 + 1);
   part(&members_, live);
-  part(&pack_, live);
   part(&obits_, nwmax);
   part(&ocnt_, nwmax);
   part(&big_, live / (kMidCap + 1) + 1);
@@ -1674,6 +1766,10 @@ bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
   part(&seg_count_, static_cast<uint64_t>(fc) + 1);
   part(&seg_z_, static_cast<uint64_t>(fc) + 1);
   part(&tab_, static_cast<uint64_t>(fc) * nblk_); // block tables
+  part(&close_st_, nwmax / kThreads + 1);
+  part(&count_st_, scan_words(static_cast<uint64_t>(fc + 1) * nwmax));
+  part(&open_st_, scan_words(nwmax));
+  part(&pack_st_, scan_words(live));
   uint64_t total = 0;
   for (const Part &q : parts)
     total += (q.bytes + 255) / 256 * 256;
@@ -1686,14 +1782,6 @@ bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
   for (const Part &q : parts) {
     *q.p = arena_ + at;
     at += (q.bytes + 255) / 256 * 256;
-  }
-  try {
-    scan32_.reserve((fc + 1) * nwmax);
-    scan32_.reserve(live);
-    scan64_.reserve(live);
-  } catch (const DeviceError &) {
-    release();
-    return false;
   }
   batch_cap_ = bc;
   frame_cap_ = fc;
@@ -1745,22 +1833,23 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   a.nval = nxt.value;
   a.npar = nxt.parent;
   a.root = root_;
-  a.size = size_;
-  a.lastz = lastz_;
-  a.rank_of_root = rank_of_root_;
-  a.cursor = cursor_;
+  a.info = info_;
+  a.close_st = close_st_;
+  a.count_st = count_st_;
+  a.open_st = open_st_;
+  a.pack_st = pack_st_;
   a.bits = bits_;
   a.bcnt = bcnt_;
   a.flist = flist_;
   a.comp_root = comp_root_;
   a.msize = msize_;
   a.mpk = mpk_;
+  a.pack = pack_;
   a.runs = runs_;
   a.run_starts = run_starts_;
   a.spot_tmp = spot_tmp_;
   a.pix_tmp = pix_tmp_;
   a.members = members_;
-  a.pack = pack_;
   a.obits = obits_;
   a.ocnt = ocnt_;
   a.big = big_;
@@ -1777,24 +1866,19 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
 
   const unsigned grid = grid_;
   LabelScalars *sc = sc_;
-  if (nframes > 0)
-    check(cudaMemsetAsync(tab_, 0xff, static_cast<uint64_t>(nframes) * nblk_ * sizeof(uint32_t), s),
-          "clearing block tables");
-  lab_setup<<<1, 32, 0, s>>>(a);
+  lab_setup<<<grid, kThreads, 0, s>>>(a);
   lab_gather<<<grid, kThreads, 0, s>>>(a);
   lab_link<<<grid, kThreads, 0, s>>>(a);
-  lab_keep_table<<<grid, kThreads, 0, s>>>(a);
   lab_flatten<<<grid, kThreads, 0, s>>>(a);
-  lab_mark<<<grid, kThreads, 0, s>>>(a);
-  const uint64_t nwmax = live_cap_ / 32 + 1;
-  scan32_.run(bcnt_, bcnt_, &sc->nw, 1, nwmax, &sc->closed32, s);
-  lab_compact<<<grid, kThreads, 0, s>>>(a);
+  lab_close<<<grid, kThreads, 0, s>>>(a);
   lab_count<<<grid, kThreads, 0, s>>>(a);
-  scan32_.run(bcnt_, bcnt_, &sc->seg_len, 1, static_cast<uint64_t>(frame_cap_ + 1) * nwmax,
-              nullptr, s);
+  const unsigned sms = grid_ / 8;
+  launch_scan<uint32_t>(bcnt_, &sc->seg_len, nullptr, &sc->count_next, count_st_, &sc->status,
+                        sms, s);
   lab_rank<<<grid, kThreads, 0, s>>>(a);
-  scan64_.run(mpk_, mpk_, &sc->closed, 1, live_cap_, &sc->members_pack, s);
   lab_scatter<<<grid, kThreads, 0, s>>>(a);
+  launch_scan<uint32_t>(ocnt_, &sc->nw, &sc->open32, &sc->open_next, open_st_, &sc->status, sms,
+                        s);
   // The few large and middle-sized components on streams of their own,
   // launched first so that their blocks are placed before the many small
   // components' launch fills the SMs: each of them is one warp's long walk,
@@ -1812,11 +1896,10 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   check(cudaEventRecord(join2_, aux2_), "cudaEventRecord");
   check(cudaStreamWaitEvent(s, join_, 0), "cudaStreamWaitEvent");
   check(cudaStreamWaitEvent(s, join2_, 0), "cudaStreamWaitEvent");
-  scan64_.run(pack_, pack_, &sc->closed, 1, live_cap_, &sc->accepted_pack, s);
+  launch_scan<uint64_t>(pack_, &sc->closed, &sc->accepted_pack, &sc->pack_next, pack_st_,
+                        &sc->status, sms, s);
   lab_write<<<grid, kThreads, 0, s>>>(a);
-  scan32_.run(ocnt_, ocnt_, &sc->nw, 1, nwmax, &sc->open32, s);
   lab_carry<<<grid, kThreads, 0, s>>>(a);
-  lab_finalize<<<1, 32, 0, s>>>(a);
   check(cudaGetLastError(), "launching the labeller");
   cur_ ^= 1;
 }

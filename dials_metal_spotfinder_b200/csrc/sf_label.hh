@@ -11,7 +11,6 @@
 #include <vector>
 
 #include "sf_host.hh"
-#include "sf_scan.cuh"
 
 namespace sf {
 
@@ -49,7 +48,7 @@ struct LabelScalars {
   uint64_t nseg;          // frame segments (carried last frame + batch frames)
   uint64_t seg_len;       // bucket-count table length: nseg * ceil(closed / 32)
   uint64_t closed;        // finished components
-  uint32_t closed32, open32;
+  uint32_t open32;        // pixels carried on
   uint32_t runs_n;        // lab_link's work list
   uint32_t big_n;         // components past the middle spot-pass buffers
   // work counters: warps take the next entries as they finish their last,
@@ -57,9 +56,9 @@ struct LabelScalars {
   // whole grid-stride share
   uint32_t link_next, accept_next, big_next, mid_next;
   uint32_t mid_n;         // components past the small buffers, within the middle ones
-  uint32_t pad0;
+  uint32_t close_next, count_next, open_next, pack_next; // tiles taken
   uint64_t members_pack;  // members (low 32) | components passing the size filters (high 32)
-  uint64_t accepted_pack; // accepted spots (low 32) | their pixels (high 32)
+  uint64_t accepted_pack; // accepted spots | their pixels << 31
   uint64_t batch_spots, batch_pixels;
   // the carry between batches
   uint64_t carry_n;
@@ -72,7 +71,20 @@ struct LabelScalars {
   int32_t pad1;
 };
 
-enum : int32_t { kLabelOk = 0, kLabelLiveOverflow = 1, kLabelSpotOverflow = 2 };
+enum : int32_t {
+  kLabelOk = 0,
+  kLabelLiveOverflow = 1,
+  kLabelSpotOverflow = 2,
+  kLabelWaitTimeout = 3, // a tile's wait for the tiles before it gave up
+};
+
+// What a component's root holds, in one 16-byte word at its position.
+struct RootInfo {
+  uint32_t size;
+  int32_t lastz;   // its last frame
+  uint32_t slot;   // its members' place; all ones while it is open
+  uint32_t cursor; // members placed
+};
 
 class DeviceLabeller {
 public:
@@ -140,9 +152,9 @@ private:
     uint32_t *value = nullptr;
     uint32_t *parent = nullptr;
   } live_[2];
-  uint32_t *root_ = nullptr, *size_ = nullptr, *rank_of_root_ = nullptr, *cursor_ = nullptr;
-  int32_t *lastz_ = nullptr;
-  uint32_t *bits_ = nullptr, *bcnt_ = nullptr; // finished-root bitmap; counts (see lab_mark)
+  uint32_t *root_ = nullptr;
+  RootInfo *info_ = nullptr;
+  uint32_t *bits_ = nullptr, *bcnt_ = nullptr; // root bitmap; bucket counts (lab_count)
   uint32_t *flist_ = nullptr;                   // the finished roots in position order
   uint32_t *comp_root_ = nullptr, *msize_ = nullptr, *members_ = nullptr;
   uint64_t *mpk_ = nullptr; // member offset (low 32) | size-filtered index (high 32)
@@ -151,6 +163,8 @@ private:
   Spot *spot_tmp_ = nullptr;  // spots by size-filtered index, before acceptance
   Pixel *pix_tmp_ = nullptr;  // their pixels, by member offset
   uint64_t *pack_ = nullptr;
+  uint64_t *close_st_ = nullptr, *count_st_ = nullptr, *open_st_ = nullptr,
+           *pack_st_ = nullptr; // lookback words
   uint32_t *obits_ = nullptr, *ocnt_ = nullptr; // open pixels per 32 positions
   uint32_t *big_ = nullptr; // ranks of the components lab_accept's large launch takes
   uint32_t *mid_ = nullptr; // ... and its middle launch
@@ -168,9 +182,6 @@ private:
   cudaStream_t aux2_ = nullptr; // the middle-sized components' spot pass
   cudaEvent_t fork_ = nullptr, join_ = nullptr, join2_ = nullptr;
   int64_t *z_stage_ = nullptr; // pinned
-
-  DeviceScan<uint32_t> scan32_;
-  DeviceScan<uint64_t> scan64_;
 };
 
 } // namespace sf
