@@ -202,7 +202,7 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   check(cudaMemsetAsync(tile_count, 0, L.ntiles * 4, s), "clearing tile counts");
   check(cudaMemsetAsync(pool_next, 0, 16, s), "clearing the pool cursor");
   check(cudaMemsetAsync(block_sums, 0, place_groups(L.ntiles) * 4, s), "clearing the tile sums");
-  check(cudaMemsetAsync(run_status, 0, 4, s), "clearing the status");
+  check(cudaMemsetAsync(run_status, 0, 8, s), "clearing the status");
   // Off-frame pixels read as masked: every byte of the arena that the frame
   // does not cover is 0xFF. The layout is a function of the shape and only
   // the frame's own pixels are written below, so after a completed call with
@@ -226,6 +226,8 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   T.frames = frames;
   T.nframes = 1;
   T.ntasks = L.ntasks;
+  T.next_task = reinterpret_cast<uint32_t *>(run_status) + 1;
+  T.ranges = nullptr;
   T.tile_count = tile_count;
   T.tile_start = tile_start;
   T.block_sums = block_sums;

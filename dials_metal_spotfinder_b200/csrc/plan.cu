@@ -179,6 +179,13 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     throw std::invalid_argument("batch too large for one plan");
 
   grid_blocks_ = static_cast<int>(std::min<uint64_t>((ntasks_ + wpc - 1) / wpc, max_blocks_));
+  int32_t tallest = 0, longest = 0;
+  for (const FrameDesc &d : host_frames_) {
+    tallest = std::max(tallest, d.height);
+    longest = std::max(longest, d.seg_rows);
+  }
+  share_rows_ = longest >= kMinSharedSeg && static_cast<uint32_t>(tallest) <= kMaxSharedRows &&
+                ntasks_ <= kMaxSharedTasks;
   const uint64_t warps = static_cast<uint64_t>(grid_blocks_) * wpc;
   const uint64_t chunks =
       (total_capacity_ + (kChunkRecords - kMaxStaged) - 1) / (kChunkRecords - kMaxStaged) +
@@ -201,11 +208,15 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     check(cudaMemcpy(frames_, host_frames_.data(), nf * sizeof(FrameDesc),
                      cudaMemcpyHostToDevice),
           "uploading frame descriptors");
-    cleared_bytes_ = (ntiles_ + nblocks + 2) * 4;
-    alloc(reinterpret_cast<void **>(&tile_count_), cleared_bytes_, "cudaMalloc tile counts");
+    cleared_bytes_ = warps * 8 + (ntiles_ + nblocks + 3) * 4;
+    unsigned char *cleared = nullptr;
+    alloc(reinterpret_cast<void **>(&cleared), cleared_bytes_, "cudaMalloc tile counts");
+    ranges_ = reinterpret_cast<unsigned long long *>(cleared);
+    tile_count_ = reinterpret_cast<uint32_t *>(ranges_ + warps);
     block_sums_ = tile_count_ + ntiles_;
     pool_next_ = block_sums_ + nblocks;
-    run_status_ = reinterpret_cast<int *>(pool_next_ + 1);
+    next_task_ = pool_next_ + 1;
+    run_status_ = reinterpret_cast<int *>(next_task_ + 1);
     alloc(reinterpret_cast<void **>(&tile_start_), ntiles_ * 4, "cudaMalloc tile starts");
     alloc(reinterpret_cast<void **>(&pool_), pool_records * sizeof(SignalPixel),
           "cudaMalloc staging pool");
@@ -239,7 +250,7 @@ void ThresholdPlan::release() {
     sl = Slot();
   }
   cudaFree(frames_);
-  cudaFree(tile_count_);
+  cudaFree(ranges_); // and what follows it
   cudaFree(tile_start_);
   cudaFree(pool_);
   cudaFree(linear_);
@@ -296,11 +307,13 @@ void ThresholdPlan::upload_device(int slot, int f, const void *device, size_t pi
 
 void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid) {
   Slot &sl = slots_.at(slot);
-  check(cudaMemsetAsync(tile_count_, 0, cleared_bytes_, stream), "clearing tile counts");
+  check(cudaMemsetAsync(ranges_, 0, cleared_bytes_, stream), "clearing tile counts");
   ThresholdLaunch L;
   L.frames = frames_;
   L.nframes = static_cast<int32_t>(host_frames_.size());
   L.ntasks = ntasks_;
+  L.next_task = next_task_;
+  L.ranges = share_rows_ ? ranges_ : nullptr;
   L.tile_count = tile_count_;
   L.tile_start = tile_start_;
   L.block_sums = block_sums_;

@@ -41,6 +41,14 @@ constexpr uint32_t kChunkRecords = 1024;   // staging pool allocation unit
 // wastes fewer than this.
 constexpr uint32_t kMaxStaged = 2 * kStripOut;
 
+// Limits of the word in which the threshold's warps share a task's rows (row
+// numbers of kSharedRowBits bits, task numbers of the 22 bits above two): plans
+// beyond them, and tasks too short to be worth sharing, are not shared.
+constexpr int kSharedRowBits = 21;
+constexpr uint32_t kMaxSharedRows = (1u << kSharedRowBits) - 64;
+constexpr uint32_t kMaxSharedTasks = 1u << (64 - 2 * kSharedRowBits);
+constexpr int kMinSharedSeg = 96;
+
 // Pixel-type traits. The window sums of the reference are accumulated in
 // accumulator_t<T> (uint32 for 16-bit pixels, uint64 for 32-bit) and tested
 // in real_t<T> (float / double), src/dext.hh:18-38. Here the count and the

@@ -34,6 +34,8 @@ struct ThresholdLaunch {
   const FrameDesc *frames;
   int32_t nframes;
   uint32_t ntasks;
+  uint32_t *next_task;        // zeroed
+  unsigned long long *ranges; // one per warp of the launch, zeroed; null: tasks are not shared
   uint32_t *tile_count;
   uint32_t *tile_start;
   uint32_t *block_sums; // the counts' sums over each kPlaceTiles tiles
@@ -175,12 +177,14 @@ private:
 
   std::vector<Slot> slots_;
   FrameDesc *frames_ = nullptr;
-  // One allocation, cleared by one memset before each run: the tiles'
-  // counts, their sums per kPlaceTiles, the pool's cursor and the run's
-  // status.
+  // One allocation, cleared by one memset before each run: the warps' shared
+  // ranges, the tiles' counts, their sums per kPlaceTiles, the pool's and the
+  // tasks' cursors and the run's status.
   uint32_t *tile_count_ = nullptr;
   uint64_t cleared_bytes_ = 0;
-  uint32_t *block_sums_ = nullptr, *pool_next_ = nullptr;
+  uint32_t *block_sums_ = nullptr, *pool_next_ = nullptr, *next_task_ = nullptr;
+  unsigned long long *ranges_ = nullptr; // one per warp
+  bool share_rows_ = false;
   int *run_status_ = nullptr;
   uint32_t *tile_start_ = nullptr;
   SignalPixel *pool_ = nullptr;

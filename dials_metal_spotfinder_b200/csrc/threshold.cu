@@ -4,8 +4,9 @@
 //
 // Decomposition. A task is one strip of 256 buffer columns (232 output
 // columns plus halo) by one segment of output rows of one frame. A warp owns
-// a task at a time and walks down it row by row; warps never talk to each
-// other. Each warp has a ring of 20 rows of its strip in shared memory, fed
+// a task at a time and walks down it row by row; one that has nothing left
+// takes rows from another's task (see pack_range), but none waits for
+// another. Each warp has a ring of 20 rows of its strip in shared memory, fed
 // 2 rows at a time by TMA (one elected lane issues, an mbarrier per stage).
 //
 // Per input row r entering at the bottom of the ring, each lane (8 columns)
@@ -308,6 +309,8 @@ struct ThresholdArgs {
   const FrameDesc *frames;
   int32_t nframes;
   uint32_t ntasks;
+  uint32_t *next_task;          // zeroed before the launch
+  unsigned long long *ranges;   // one per warp, zeroed too; null: tasks are not shared
   uint32_t *tile_count; // zeroed before the launch
   uint32_t *tile_start;
   uint32_t *block_sums; // per kPlaceTiles tiles; zeroed too
@@ -331,6 +334,90 @@ __device__ __forceinline__ int find_frame(const FrameDesc *frames, int n,
   return lo;
 }
 
+// What a warp still has to do, in one word that its owner and others change
+// by atomics: the task, the end of its output rows, and the first row not
+// yet claimed. The owner claims kQuantum rows at a time, a box ahead of
+// needing them; a warp with nothing left to do takes the lower half of what
+// another has not claimed. 0: nothing.
+//
+// Warps of equal tasks do not finish together (an SM's schedulers favour
+// some, strips differ in masked columns and candidates): without this, 12.9
+// of the 16 warps an SM holds were active on average, and 16 frames of
+// 4362 x 4148 uint16 took 1104 us (958 with it), 16 of 2162 x 2068 327 (304),
+// 8 of 4362 x 4148 uint32 1103 (995). Halves down to kLeastShare rows are
+// worth the 20 rows of halo they cost again: at least 64 gave 976 and 329
+// us, 24 the same as 32; claims of 8 rows the same as of 16.
+constexpr uint32_t kQuantum = 16;
+constexpr uint32_t kLeastShare = 32;
+constexpr int kRowBits = kSharedRowBits;
+constexpr uint32_t kRowMask = (1u << kRowBits) - 1;
+static_assert(kMaxSharedRows + 2 * kQuantum <= kRowMask, "a claim past the end stays in its field");
+
+__device__ __forceinline__ unsigned long long pack_range(uint32_t task, uint32_t end,
+                                                         uint32_t next) {
+  return (static_cast<unsigned long long>(task) << (2 * kRowBits)) |
+         (static_cast<unsigned long long>(end) << kRowBits) | next;
+}
+__device__ __forceinline__ uint32_t range_task(unsigned long long r) {
+  return static_cast<uint32_t>(r >> (2 * kRowBits));
+}
+__device__ __forceinline__ uint32_t range_end(unsigned long long r) {
+  return static_cast<uint32_t>(r >> kRowBits) & kRowMask;
+}
+__device__ __forceinline__ uint32_t range_next(unsigned long long r) {
+  return static_cast<uint32_t>(r) & kRowMask;
+}
+
+// Takes half of what some warp has not claimed: looks at 256 warps' words at
+// a time, from a place of its own on, and goes for the one with most left;
+// false when none had enough (or kTakeTries looks found others quicker).
+constexpr uint32_t kTakeTries = 64;
+__device__ bool take_rows(unsigned long long *ranges, uint32_t nwarps, uint32_t from, int lane,
+                          uint32_t *task, uint32_t *r0, uint32_t *r1) {
+  constexpr uint32_t kLook = 8;
+  for (uint32_t seen = 0, tries = 0; seen < nwarps && tries < kTakeTries; tries++) {
+    unsigned long long best = 0;
+    uint32_t most = 0, where = 0;
+    unsigned long long v[kLook];
+#pragma unroll
+    for (uint32_t k = 0; k < kLook; k++) {
+      const uint32_t i = (from + seen + 32 * k + lane) % nwarps;
+      v[k] = *reinterpret_cast<volatile unsigned long long *>(ranges + i);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kLook; k++) {
+      const uint32_t end = range_end(v[k]), next = range_next(v[k]);
+      const uint32_t left = end > next ? end - next : 0u;
+      if (left > most) {
+        most = left;
+        best = v[k];
+        where = (from + seen + 32 * k + lane) % nwarps;
+      }
+    }
+    const uint32_t top = __reduce_max_sync(kFull, most);
+    if (top < kLeastShare) {
+      seen += 32 * kLook;
+      continue;
+    }
+    const int who = __ffs(__ballot_sync(kFull, most == top)) - 1;
+    uint32_t split = 0;
+    if (lane == who) {
+      const uint32_t end = range_end(best), next = range_next(best);
+      split = next + ((end - next) / 2 + 1) / 2 * 2;
+      if (atomicCAS(ranges + where, best, pack_range(range_task(best), split, next)) != best)
+        split = 0; // it moved on
+    }
+    split = __shfl_sync(kFull, split, who);
+    if (split == 0)
+      continue;
+    *r0 = split;
+    *r1 = __shfl_sync(kFull, range_end(best), who);
+    *task = __shfl_sync(kFull, range_task(best), who);
+    return true;
+  }
+  return false;
+}
+
 // Ring slot of the row `back` rows above the row in slot `slot`.
 __device__ __forceinline__ int back_slot(int slot, int back) {
   const int s = slot - back;
@@ -349,7 +436,8 @@ constexpr int kPreRows = 16;
 // flight; the first two boxes do not land on the zero rows.
 static_assert(kRingRows >= kPreRows + 2 + kBoxRows, "ring too short");
 static_assert(kRingRows - kPreRows >= 2 * kBoxRows, "prologue boxes overlap the zero rows");
-static_assert(kBoxRows % 2 == 0 && kRingRows % kBoxRows == 0, "rows go in pairs");
+static_assert(kBoxRows == 2 && kRingRows % kBoxRows == 0, "a box is a pair of rows");
+static_assert(kQuantum % 2 == 0 && kQuantum / kBoxRows >= 2, "claims go in pairs of rows");
 
 // Per-warp shared memory (the square-root table is static).
 template <typename T> struct WarpSmem {
@@ -413,18 +501,40 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
   const uint32_t gwarp = blockIdx.x * WPC + warp;
   const uint32_t nwarps = gridDim.x * WPC;
 
-  for (uint32_t task = gwarp; task < args.ntasks && !failed; task += nwarps) {
+  const bool shared_rows = args.ranges != nullptr;
+  bool taking = false; // no whole task is left: rows of others' tasks
+  for (uint32_t turn = gwarp; !failed;) {
+    uint32_t task = turn, from = 0, to = 0;
+    if (!taking && turn >= args.ntasks) {
+      if (!shared_rows)
+        break;
+      taking = true;
+    }
+    if (taking && !take_rows(args.ranges, nwarps, gwarp * 37u, lane, &task, &from, &to))
+      break;
     const int f = find_frame(args.frames, args.nframes, task);
     const FrameDesc fd = args.frames[f];
     const uint32_t local = task - fd.task_begin;
     const int strip = static_cast<int>(local % fd.strips);
     const int seg = static_cast<int>(local / fd.strips);
-    const int r0 = seg * fd.seg_rows;
-    const int r1 = min(r0 + fd.seg_rows, fd.height);
+    if (!taking) {
+      from = seg * fd.seg_rows;
+      to = min(from + fd.seg_rows, static_cast<uint32_t>(fd.height));
+      uint32_t t = 0;
+      if (lane == 0)
+        t = nwarps + atomicAdd(args.next_task, 1u);
+      turn = __shfl_sync(kFull, t, 0);
+    }
+    const int r0 = static_cast<int>(from);
+    // output rows below `limit` are this warp's
+    uint32_t limit = shared_rows ? min(from + kQuantum, to) : to;
+    bool more = limit < to, asked = false;
+    unsigned long long claim = 0;
+    if (shared_rows && lane == 0)
+      atomicExch(args.ranges + gwarp, more ? pack_range(task, to, limit) : 0ull);
     const int rs = r0 - kHalo;       // first input row (frame coordinates)
-    const int nrows = (r1 - r0) + 2 * kHalo;
-    const int nboxes = (nrows + kBoxRows - 1) / kBoxRows;
-    const int nrows2 = (nrows + 1) & ~1; // rows are taken in pairs
+    int nrows = static_cast<int>(limit - from) + 2 * kHalo;
+    int nboxes = (nrows + kBoxRows - 1) / kBoxRows;
     const int32_t tma_x = strip * kStripOut;
     const int64_t tma_y0 = fd.row0 + rs;
 
@@ -517,9 +627,9 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       lA.unpack(q);
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        const A d = static_cast<A>(p[k]) - static_cast<A>(q[k]);
-        vsA[k] = vs[k] + d;
-        vqA[k] = vq[k] + d * (static_cast<A>(p[k]) + static_cast<A>(q[k]));
+        vsA[k] = vs[k] + static_cast<A>(p[k]) - static_cast<A>(q[k]);
+        vqA[k] = static_cast<A>(p[k]) * static_cast<A>(p[k]) -
+                 (static_cast<A>(q[k]) * static_cast<A>(q[k]) - vq[k]);
       }
       if ((flags & 1u) | (dirty & 0x40u)) {
         const uint32_t mk7 = static_cast<uint32_t>(hist_mk >> 48) & 0xffu; // row r-7
@@ -541,9 +651,9 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       lB.unpack(q);
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        const A d = static_cast<A>(p[k]) - static_cast<A>(q[k]);
-        vs[k] = vsA[k] + d;
-        vq[k] = vqA[k] + d * (static_cast<A>(p[k]) + static_cast<A>(q[k]));
+        vs[k] = vsA[k] + static_cast<A>(p[k]) - static_cast<A>(q[k]);
+        vq[k] = static_cast<A>(p[k]) * static_cast<A>(p[k]) -
+                (static_cast<A>(q[k]) * static_cast<A>(q[k]) - vqA[k]);
       }
       if ((flags & 2u) | (dirty & 0x20u)) {
         const uint32_t mk6 = static_cast<uint32_t>(hist_mk >> 40) & 0xffu; // row r-6
@@ -788,6 +898,23 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
 
     for (int b = 0; b < nboxes && !failed; b++) {
       const int st = b % kRingStages;
+      // the next rows are claimed a box ahead of the one that needs them
+      if (asked && b == nboxes - 1) {
+        const unsigned long long r = __shfl_sync(kFull, claim, 0);
+        const uint32_t next = range_next(r), end = range_end(r);
+        asked = false;
+        more = next + kQuantum < end;
+        if (next < end) {
+          limit = min(next + kQuantum, end);
+          nrows = static_cast<int>(limit - from) + 2 * kHalo;
+          nboxes = (nrows + kBoxRows - 1) / kBoxRows;
+        }
+      }
+      if (more && !asked && b == nboxes - 2) {
+        if (lane == 0)
+          claim = atomicAdd(args.ranges + gwarp, static_cast<unsigned long long>(kQuantum));
+        asked = true;
+      }
       if (lane == 0 && b >= 1 && b + 1 < nboxes) {
         // Box b+1 reuses the stage of box b+1-kRingStages, whose rows are
         // all older than r-16 for every row of box b: free.
@@ -810,10 +937,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       // (its box holds it), whose results go nowhere.
       const int rr0 = b * kBoxRows;
       const int slot0 = st * kBoxRows;
-      const int rend = min(kBoxRows, nrows2 - rr0);
-#pragma unroll 1
-      for (int i = 0; i < rend; i += 2)
-        process_pair(rr0 + i, slot0 + i);
+      process_pair(rr0, slot0);
       __syncwarp();
     }
     if (failed) {
@@ -853,6 +977,8 @@ static cudaError_t launch_wpc(const CUtensorMap &map, const ThresholdLaunch &L,
   a.frames = L.frames;
   a.nframes = L.nframes;
   a.ntasks = L.ntasks;
+  a.next_task = L.next_task;
+  a.ranges = L.ranges;
   a.tile_count = L.tile_count;
   a.tile_start = L.tile_start;
   a.block_sums = L.block_sums;
