@@ -43,24 +43,41 @@ constexpr uint64_t kLinearUpload = 512 * 1024;
 
 uint64_t round_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 
-// Output rows per task. A warp's cost is its rows plus the 20 rows of halo
-// it re-reads, and the launch lasts as many waves as the tasks need; pick the
-// segment height that minimises waves x (rows + halo).
-int choose_seg_rows(const std::vector<ThresholdPlan::Shape> &shapes, uint64_t resident) {
+// Output rows per task. A task costs its rows plus the 20 rows of halo it
+// re-reads; how long a row takes depends on the warps that share the SM: as
+// 5 + w for w of them, and no less than for 7, when a warp waits on itself
+// (16-bit pixels, one frame of each of several sizes over many heights; 0.08
+// us a unit). So the height with the least (rows + 20) x (5 + w), an SM's w
+// taken as the most that any has when the blocks are dealt out, in as many
+// rounds as they need; no shorter than kMinSeg rows, below which the halo is
+// most of the work and the gain is in the noise. The threshold of one frame:
+// 2162 x 2068 uint16 59 -> 52 us (17 rows; 16, the least there was, put a
+// tenth warp on some SMs), 1062 x 1028 44 -> 36 us (6 rows), 256 x 384
+// 35 -> 27 us (4 rows).
+constexpr uint64_t kRowBase = 5, kRowLeast = 12;
+constexpr int kMinSeg = 4;
+int choose_seg_rows(const std::vector<ThresholdPlan::Shape> &shapes, uint64_t sms, int wpc,
+                    int blocks_per_sm) {
   int max_h = 1;
   for (const auto &s : shapes)
     max_h = std::max(max_h, s.height);
   int best = max_h;
-  double best_cost = 1e300;
-  for (int seg = 16; seg <= max_h; seg++) {
+  uint64_t best_cost = ~0ull;
+  for (int seg = std::min(kMinSeg, max_h); seg <= max_h; seg++) {
     uint64_t tasks = 0;
     for (const auto &s : shapes) {
       const uint64_t strips = (s.width + kStripOut - 1) / kStripOut;
       tasks += strips * ((s.height + seg - 1) / seg);
     }
-    const uint64_t waves = (tasks + resident - 1) / resident;
-    const double cost = static_cast<double>(waves) * (std::min(seg, max_h) + 2 * kHalo);
-    if (cost < best_cost - 1e-9) {
+    const uint64_t per_block = static_cast<uint64_t>(wpc);
+    const uint64_t blocks = (tasks + per_block - 1) / per_block;
+    const uint64_t per_sm = (blocks + sms - 1) / sms * per_block;
+    const uint64_t fit = static_cast<uint64_t>(blocks_per_sm) * per_block;
+    const uint64_t rest = per_sm % fit;
+    const uint64_t row = per_sm / fit * std::max(kRowLeast, kRowBase + fit) +
+                         (rest ? std::max(kRowLeast, kRowBase + rest) : 0);
+    const uint64_t cost = row * static_cast<uint64_t>(std::min(seg, max_h) + 2 * kHalo);
+    if (cost < best_cost) {
       best_cost = cost;
       best = seg;
     }
@@ -78,7 +95,7 @@ int model_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shap
     throw DeviceError("the threshold kernel does not fit on this device");
   if (blocks_per_sm > 0)
     occ = std::min(occ, blocks_per_sm);
-  return choose_seg_rows(shapes, static_cast<uint64_t>(device_sm_count()) * occ * wpc);
+  return choose_seg_rows(shapes, static_cast<uint64_t>(device_sm_count()), wpc, occ);
 }
 
 void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes, uint64_t pitch_elems,
@@ -144,7 +161,7 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
   sms_ = device_sm_count();
   max_blocks_ = sms_ * per_sm;
   if (tuning_.seg_rows <= 0)
-    tuning_.seg_rows = choose_seg_rows(shapes, static_cast<uint64_t>(max_blocks_) * wpc);
+    tuning_.seg_rows = choose_seg_rows(shapes, static_cast<uint64_t>(sms_), wpc, per_sm);
 
   uint64_t row = 0, tile = 0, out = 0;
   uint32_t task = 0;
