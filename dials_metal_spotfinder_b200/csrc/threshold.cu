@@ -29,6 +29,16 @@
 // frame and a masked pixel are treated identically by every step of the
 // reference's arithmetic (excluded from every sum, 1 in the erode input).
 //
+// Bound: instruction issue (2.7 of 4 a cycle) and the integer pipe (74 % busy)
+// at the 16 warps an SM holds for 16-bit pixels; 4362 x 4148 uint16 takes
+// 56 us a frame in a batch, 810 GB/s of its own bytes. Integer work is
+// therefore moved or saved where that costs no more instructions: low halves
+// by a multiply-add, float bits formed by the sums themselves, what the
+// 11-row sums leave out selected before the addition instead of corrected
+// after it, one masked test a pair of rows (956 -> 897 us for 16 frames). Not
+// kept: high halves by a high multiply (927), and additions as multiply-adds
+// in the vertical (926) or the horizontal sums (910), which cost two each.
+//
 // Cost. The running sums are updated as if every pixel entering and leaving
 // were valid -- then the packed counts cancel and an update is one add of
 // (entering - leaving) -- and corrected afterwards for the few pixels that
@@ -132,7 +142,8 @@ __device__ __forceinline__ uint32_t dispersion_bits(const uint32_t (&hs)[8],
 }
 
 // The same when every window holds 49 pixels: m, m - 1 and the square root
-// are constants (sq49 = sqrt_term(49)). s * 48 is formed as 8 * (s * 6):
+// are constants (sq49 = sqrt_term(49)), and hs is the sum under the exponent
+// of 2^23. s * 48 is formed as 8 * (s * 6):
 // scaling by a power of two is exact and commutes with rounding, so
 // fl(s * 48) = 8 fl(s * 6), and t3 - fl(s * 48) is one fused operation on
 // the already rounded fl(s * 6), which the right side needs anyway.
@@ -147,8 +158,7 @@ __device__ __forceinline__ uint32_t dispersion_bits49(const uint32_t (&hs)[8],
   uint32_t bits = 0;
 #pragma unroll
   for (int k = 6; k >= 0; k -= 2) {
-    const float2 S = __fadd2_rn(make_float2(magic_bits(hs[k] & 0x3fffffu),
-                                            magic_bits(hs[k + 1] & 0x3fffffu)),
+    const float2 S = __fadd2_rn(make_float2(__uint_as_float(hs[k]), __uint_as_float(hs[k + 1])),
                                 magic);
     const float2 Q = make_float2(__uint2float_rn(hq[k]), __uint2float_rn(hq[k + 1]));
     const float2 t1 = __fmul2_rn(c49, Q);
@@ -212,17 +222,23 @@ template <> struct LaneRow<uint16_t> {
   __device__ __forceinline__ void load(const uint16_t *row, int lane) {
     v = reinterpret_cast<const uint4 *>(row)[lane];
   }
-  __device__ __forceinline__ void unpack(uint32_t (&p)[8]) const {
-    p[0] = v.x & 0xffffu; p[1] = v.x >> 16;
-    p[2] = v.y & 0xffffu; p[3] = v.y >> 16;
-    p[4] = v.z & 0xffffu; p[5] = v.z >> 16;
-    p[6] = v.w & 0xffffu; p[7] = v.w >> 16;
+  // `down` is 0xffff0000: the low half is the word less the high half times
+  // 2^16, a multiply-add on the FMA pipe instead of another mask on the
+  // integer one.
+  __device__ __forceinline__ void unpack(uint32_t (&p)[8], uint32_t down) const {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      p[2 * k + 1] = w[k] >> 16;
+      p[2 * k] = p[2 * k + 1] * down + w[k];
+    }
   }
-  // Nonzero iff a pixel is 0xfffe or 0xffff (masked): the halfword maxima
-  // of the four words, compared with 0xfffe per half.
-  __device__ __forceinline__ uint32_t any_masked() const {
-    const uint32_t m = __vmaxu2(__vmaxu2(v.x, v.y), __vmaxu2(v.z, v.w));
-    return __vcmpgeu2(m, 0xfffefffeu);
+  // Whether a pixel of either row is 0xfffe or 0xffff (masked): the halfword
+  // maxima of the eight words, compared with 0xfffe per half.
+  static __device__ __forceinline__ bool any_masked(const LaneRow &r, const LaneRow &s) {
+    const uint32_t m = __vmaxu2(__vmaxu2(__vmaxu2(r.v.x, r.v.y), __vmaxu2(r.v.z, r.v.w)),
+                                __vmaxu2(__vmaxu2(s.v.x, s.v.y), __vmaxu2(s.v.z, s.v.w)));
+    return (m & 0xffffu) >= 0xfffeu || m >= 0xfffe0000u;
   }
   // Bit k set where pixel k is masked.
   __device__ __forceinline__ uint32_t masked_bits() const {
@@ -241,7 +257,7 @@ template <> struct LaneRow<uint32_t> {
     a = v[0];
     b = v[1];
   }
-  __device__ __forceinline__ void unpack(uint32_t (&p)[8]) const {
+  __device__ __forceinline__ void unpack(uint32_t (&p)[8], uint32_t) const {
     p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w;
     p[4] = b.x; p[5] = b.y; p[6] = b.z; p[7] = b.w;
   }
@@ -251,14 +267,17 @@ template <> struct LaneRow<uint32_t> {
            (a.w >= m ? 8u : 0u) | (b.x >= m ? 16u : 0u) | (b.y >= m ? 32u : 0u) |
            (b.z >= m ? 64u : 0u) | (b.w >= m ? 128u : 0u);
   }
-  __device__ __forceinline__ uint32_t any_masked() const { return masked_bits(); }
+  static __device__ __forceinline__ bool any_masked(const LaneRow &r, const LaneRow &s) {
+    return (r.masked_bits() | s.masked_bits()) != 0;
+  }
 };
 
 template <typename T>
-__device__ __forceinline__ void load_pixels(const T *row, int lane, uint32_t (&p)[8]) {
+__device__ __forceinline__ void load_pixels(const T *row, int lane, uint32_t (&p)[8],
+                                            uint32_t down) {
   LaneRow<T> r;
   r.load(row, lane);
-  r.unpack(p);
+  r.unpack(p, down);
 }
 
 __device__ __forceinline__ uint32_t shfl_up(uint32_t v) { return __shfl_up_sync(kFull, v, 1); }
@@ -278,7 +297,7 @@ __device__ __forceinline__ uint64_t shfl_down(uint64_t v) {
 // own vertical sums v[0..8) and the neighbouring lanes' by shuffle. The edge
 // lanes see no neighbour; their edge columns are halo and never used.
 template <int R, typename A>
-__device__ __forceinline__ void hsum(const A (&v)[8], A (&h)[8]) {
+__device__ __forceinline__ void hsum(const A (&v)[8], A (&h)[8], A from = 0) {
   A e[8 + 2 * R];
 #pragma unroll
   for (int i = 0; i < R; i++)
@@ -289,7 +308,7 @@ __device__ __forceinline__ void hsum(const A (&v)[8], A (&h)[8]) {
 #pragma unroll
   for (int i = 0; i < R; i++)
     e[R + 8 + i] = shfl_down(v[i]);
-  A run = 0;
+  A run = from;
 #pragma unroll
   for (int i = 0; i < 2 * R + 1; i++)
     run += e[i];
@@ -299,6 +318,38 @@ __device__ __forceinline__ void hsum(const A (&v)[8], A (&h)[8]) {
     run += e[k + 2 * R] - e[k - 1];
     h[k] = run;
   }
+}
+
+// The lane's pixels of a row as they enter or leave the 11-row sums: each
+// counts as a valid one that is not kept (the count cancels between the row
+// that enters and the one that leaves), and one that is masked or kept, whose
+// bit is in `ng`, is changed to take its count back and add nothing.
+template <typename T> using GroundWord = typename Traits<T>::Acc;
+template <typename T>
+__device__ __forceinline__ void load_ground(const T *row, int lane, GroundWord<T> (&g)[8],
+                                            uint32_t down) {
+  uint32_t p[8];
+  load_pixels<T>(row, lane, p, down);
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    g[k] = p[k];
+}
+template <typename T>
+__device__ __forceinline__ void only_ground(GroundWord<T> (&in)[8], GroundWord<T> (&out)[8],
+                                            uint32_t ng_in, uint32_t ng_out) {
+  constexpr GroundWord<T> kNot = GroundWord<T>(0) - (GroundWord<T>(1) << Traits<T>::kShift11);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    in[k] = (ng_in >> k) & 1u ? kNot : in[k];
+    out[k] = (ng_out >> k) & 1u ? kNot : out[k];
+  }
+}
+template <typename T>
+__device__ __forceinline__ void add_rows(GroundWord<T> (&sum)[8], const GroundWord<T> (&in)[8],
+                                         const GroundWord<T> (&out)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    sum[k] += in[k] - out[k];
 }
 
 // --------------------------------------------------------------------------
@@ -319,6 +370,7 @@ struct ThresholdArgs {
   uint32_t pool_cap; // records
   int *status;
   uint32_t wait_limit;
+  uint32_t down; // 0xffff0000 (LaneRow::unpack), from here so that it stays a multiplier
 };
 
 __device__ __forceinline__ int find_frame(const FrameDesc *frames, int n,
@@ -493,6 +545,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
   }
   __syncthreads();
   const float sq49 = static_cast<float>(sqrt_tab[49]);
+  const uint32_t down = args.down;
 
   uint32_t phase = 0; // bit s = parity of the next wait on stage s
   uint32_t chunk = kNoChunk, fill = 0;
@@ -590,7 +643,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
     uint64_t gv_lo = ~0ull; // valid-and-not-kept bits of rows r-6 .. r-13
     uint32_t gv_hi = ~0u;   //   rows r-14 .. r-17
     uint64_t hist_cs = 0;   // candidate bits of rows r-6 .. r-13
-    uint32_t dirty = 0;     // warp-uniform: bit i = row r-1-i holds a masked pixel
+    uint32_t dirty = 0;     // warp-uniform: bit i = the pair of row r-1-i holds a masked pixel
     uint32_t gdirty = 0;    // warp-uniform: bit i = row r-6-i holds a non-g pixel
 
     auto row_at = [&](int slot) { return ring + slot * kStripCols; };
@@ -611,9 +664,11 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       const bool emitB = rr + 1 >= 2 * kHalo && rr + 1 < nrows;
       const uint32_t csA = static_cast<uint32_t>(hist_cs >> 32) & (emitA ? outmask : 0u);
       const uint32_t csB = static_cast<uint32_t>(hist_cs >> 24) & (emitB ? outmask : 0u);
-      const uint32_t flags = __reduce_or_sync(
-          kFull, (nA.any_masked() ? 1u : 0u) | (nB.any_masked() ? 2u : 0u) |
-                     ((csA | csB) ? 4u : 0u));
+      // bits 0 and 1: a masked pixel in row r, r+1 (in either: the pair is
+      // tested as one); bit 2: a candidate
+      const uint32_t flags =
+          __reduce_or_sync(kFull, (LaneRow<T>::any_masked(nA, nB) ? 3u : 0u) |
+                                      ((csA | csB) ? 4u : 0u));
       uint32_t mkA = 0, mkB = 0;
       if (flags & 3u) {
         mkA = nA.masked_bits();
@@ -623,8 +678,8 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       // ---- 7-row sums: + rows r, r+1, - rows r-7, r-6 ------------------
       uint32_t p[8], q[8];
       A vsA[8], vqA[8];
-      nA.unpack(p);
-      lA.unpack(q);
+      nA.unpack(p, down);
+      lA.unpack(q, down);
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         vsA[k] = vs[k] + static_cast<A>(p[k]) - static_cast<A>(q[k]);
@@ -647,8 +702,8 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
           }
         }
       }
-      nB.unpack(p);
-      lB.unpack(q);
+      nB.unpack(p, down);
+      lB.unpack(q, down);
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         vs[k] = vsA[k] + static_cast<A>(p[k]) - static_cast<A>(q[k]);
@@ -673,13 +728,17 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       }
 
       // ---- dispersion test at rows a = r-3 and a+1 ---------------------
+      // with 49 pixels in every window the sums start with that count taken
+      // off and the exponent of 2^23 put on, and so come out as floats' bits
+      constexpr A kClean =
+          sizeof(T) == 2 ? A(0x4b000000u - 49u * static_cast<uint32_t>(C7)) : A(0);
       // row a's window is rows r-6 .. r, row a+1's r-5 .. r+1
       const bool wdA = ((dirty & 0x3fu) | (flags & 1u)) != 0;
       const bool wdB = ((dirty & 0x1fu) | (flags & 3u)) != 0;
       uint32_t s0A, s0B;
       {
         A hs[8], hq[8];
-        hsum<3>(vsA, hs);
+        hsum<3>(vsA, hs, wdA ? A(0) : kClean);
         hsum<3>(vqA, hq);
         if constexpr (sizeof(T) == 2)
           s0A = wdA ? dispersion_bits(hs, hq, sqrt_tab) : dispersion_bits49(hs, hq, sq49);
@@ -688,7 +747,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       }
       {
         A hs[8], hq[8];
-        hsum<3>(vs, hs);
+        hsum<3>(vs, hs, wdB ? A(0) : kClean);
         hsum<3>(vq, hq);
         if constexpr (sizeof(T) == 2)
           s0B = wdB ? dispersion_bits(hs, hq, sqrt_tab) : dispersion_bits49(hs, hq, sq49);
@@ -720,44 +779,21 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       // ---- 11-row sums at rows b, b+1: + rows r-5, r-4, - rows r-16, r-15
       const uint32_t ng16 = ~(gv_hi >> 16) & 0xffu; // row r-16
       const uint32_t ng15 = ~(gv_hi >> 8) & 0xffu;  // row r-15
-      load_pixels<T>(row_at(back_slot(slot, 5)), lane, p);
-      load_pixels<T>(row_at(back_slot(slot, 16)), lane, q);
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        vg[k] += static_cast<A>(p[k]) - static_cast<A>(q[k]);
-      if ((gflags & 1u) | ((gdirty >> 10) & 1u)) {
-        const uint32_t ng5 = ~gvA & 0xffu;
-        if (ng5 | ng16) {
-#pragma unroll
-          for (int k = 0; k < 8; k++) {
-            if ((ng5 >> k) & 1u)
-              vg[k] -= static_cast<A>(p[k]) + C11;
-            if ((ng16 >> k) & 1u)
-              vg[k] += static_cast<A>(q[k]) + C11;
-          }
-        }
-      }
+      GroundWord<T> gp[8], gq[8];
+      load_ground<T>(row_at(back_slot(slot, 5)), lane, gp, down);
+      load_ground<T>(row_at(back_slot(slot, 16)), lane, gq, down);
+      if ((gflags & 1u) | ((gdirty >> 10) & 1u))
+        only_ground<T>(gp, gq, ~gvA, ng16);
+      add_rows<T>(vg, gp, gq);
       A vgA[8];
 #pragma unroll
       for (int k = 0; k < 8; k++)
         vgA[k] = vg[k];
-      load_pixels<T>(row_at(back_slot(slot, 4)), lane, p);
-      load_pixels<T>(row_at(back_slot(slot, 15)), lane, q);
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        vg[k] += static_cast<A>(p[k]) - static_cast<A>(q[k]);
-      if ((gflags & 2u) | ((gdirty >> 9) & 1u)) {
-        const uint32_t ng4 = ~gvB & 0xffu;
-        if (ng4 | ng15) {
-#pragma unroll
-          for (int k = 0; k < 8; k++) {
-            if ((ng4 >> k) & 1u)
-              vg[k] -= static_cast<A>(p[k]) + C11;
-            if ((ng15 >> k) & 1u)
-              vg[k] += static_cast<A>(q[k]) + C11;
-          }
-        }
-      }
+      load_ground<T>(row_at(back_slot(slot, 4)), lane, gp, down);
+      load_ground<T>(row_at(back_slot(slot, 15)), lane, gq, down);
+      if ((gflags & 2u) | ((gdirty >> 9) & 1u))
+        only_ground<T>(gp, gq, ~gvB, ng15);
+      add_rows<T>(vg, gp, gq);
 
       // ---- histories -----------------------------------------------------
       gv_hi = (gv_hi << 16) | static_cast<uint32_t>(gv_lo >> 48);
@@ -987,6 +1023,7 @@ static cudaError_t launch_wpc(const CUtensorMap &map, const ThresholdLaunch &L,
   a.pool_cap = L.pool_cap;
   a.status = L.status;
   a.wait_limit = L.wait_limit;
+  a.down = 0xffff0000u;
   uint32_t blocks = (L.ntasks + WPC - 1) / WPC;
   if (L.max_blocks > 0 && blocks > static_cast<uint32_t>(L.max_blocks))
     blocks = static_cast<uint32_t>(L.max_blocks);
