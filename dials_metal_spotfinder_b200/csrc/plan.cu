@@ -240,10 +240,10 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     for (Slot &sl : slots_) {
       alloc(&sl.arena, arena_bytes, "cudaMalloc arena");
       check(cudaMemset(sl.arena, 0xff, arena_bytes), "filling the arena");
-      alloc(reinterpret_cast<void **>(&sl.out), total_capacity_ * sizeof(SignalPixel),
-            "cudaMalloc output lists");
-      alloc(reinterpret_cast<void **>(&sl.frame_count), (nf + 1) * 4,
-            "cudaMalloc frame counts");
+      const uint64_t head = round_up((nf + 1) * 4, kListsAt);
+      alloc(reinterpret_cast<void **>(&sl.frame_count),
+            head + total_capacity_ * sizeof(SignalPixel), "cudaMalloc output lists");
+      sl.out = reinterpret_cast<SignalPixel *>(reinterpret_cast<char *>(sl.frame_count) + head);
       sl.status = reinterpret_cast<int *>(sl.frame_count + nf);
       check(cudaMemset(sl.frame_count, 0, (nf + 1) * 4), "clearing frame counts");
       encode_arena_map(&sl.map, sl.arena, elem_bytes_, pitch_, arena_rows_);
@@ -262,8 +262,7 @@ ThresholdPlan::~ThresholdPlan() { release(); }
 void ThresholdPlan::release() {
   for (Slot &sl : slots_) {
     cudaFree(sl.arena);
-    cudaFree(sl.out);
-    cudaFree(sl.frame_count);
+    cudaFree(sl.frame_count); // and the lists after it
     sl = Slot();
   }
   cudaFree(frames_);

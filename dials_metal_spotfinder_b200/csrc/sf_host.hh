@@ -142,6 +142,9 @@ public:
   SignalPixel *out(int slot) const { return slots_[slot].out; }
   uint64_t out_base(int f) const { return host_frames_[f].out_base; }
   uint32_t capacity(int f) const { return host_frames_[f].capacity; }
+  // The counts, with the status word after the last; the lists follow them
+  // in the same allocation, from a multiple of kListsAt bytes on.
+  static constexpr uint64_t kListsAt = 256;
   uint32_t *frame_count(int slot) const { return slots_[slot].frame_count; }
   int *status(int slot) const { return slots_[slot].status; }
   uint32_t ntasks() const { return ntasks_; }
