@@ -67,6 +67,7 @@ constexpr int kThreads = kTileThreads;
 // launches with larger buffers.
 constexpr uint32_t kSmallCap = 256;
 constexpr uint32_t kMidCap = 512;
+constexpr int kGatherFrames = 4; // see lab_gather
 // 32-position words a warp of lab_scatter takes at a time.
 constexpr int kScatterWords = 4;
 // The spots' scan packs pixels above rows, neither of which reaches 2^31.
@@ -357,9 +358,15 @@ __device__ __forceinline__ const uint32_t *table_of(const LabArgs &a, int s, int
 // 32-aligned chunk of positions, found with one ballot, so that the trees
 // start one level deep; a run that enters a chunk from the previous one is
 // joined by lab_link at the chunk's first position.
+// A warp takes kGatherWords chunks at a time, all their records read before
+// any is used. Four: a quarter of the run list's claims, block-wide waits and
+// segment lookups (16 frames of 4362 x 4148 142 -> 133 us for 460 MB moved); one
+// for batches of fewer than kGatherFrames frames, which four leave with too
+// few warps (one frame of 2162 x 2068 11 us; 13 with four).
+template <int kGatherWords>
 __global__ void __launch_bounds__(kThreads) lab_gather(LabArgs a) {
   LabelScalars *sc = a.sc;
-  const uint64_t n = sc->n, carry = sc->carry_n;
+  const uint64_t n = sc->n, carry = sc->carry_n, carry_last = sc->carry_last_start;
   const int nseg = static_cast<int>(sc->nseg);
   const int first_batch_seg = carry > 0 ? 1 : 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -381,84 +388,107 @@ __global__ void __launch_bounds__(kThreads) lab_gather(LabArgs a) {
   __syncthreads();
   const uint64_t *seg_start = in_shared ? sh_start : a.seg_start;
   const int64_t *seg_z = in_shared ? sh_z : a.seg_z;
-  // block-uniform trip count: the run list is appended to once per block
-  for (uint64_t block_base = static_cast<uint64_t>(blockIdx.x) * kThreads; block_base < n;
-       block_base += static_cast<uint64_t>(gridDim.x) * kThreads) {
-    const uint64_t base = block_base + static_cast<uint64_t>(warp) * 32;
-    const uint64_t g = base + lane;
-    bool left = false;
-    int seg = 0;       // a new pixel's frame segment
-    uint32_t pidx = 0; // and its index, for the work list
-    if (g < n) {
-      if (g >= carry) {
-        const int s = segment_of(seg_start, nseg, g);
-        seg = s;
-        const int f = s - first_batch_seg;
-        const uint64_t i = g - seg_start[s];
-        const SignalPixel *list = a.lists + a.offs[f];
-        const SignalPixel px = list[i];
-        a.fr[g] = static_cast<int32_t>(seg_z[s]);
-        a.ix[g] = px.index;
-        a.val[g] = px.value;
-        pidx = px.index;
-        const uint32_t prev = i == 0 ? 0u : list[i - 1].index;
-        left = i > 0 && prev + 1 == px.index && a.wdiv.rem(px.index) != 0;
+  constexpr uint64_t kTile = static_cast<uint64_t>(kThreads) * kGatherWords;
+  // block-uniform trip count: the run list is appended to once per tile
+  for (uint64_t tile = blockIdx.x * kTile; tile < n; tile += gridDim.x * kTile) {
+    const uint64_t wbase = tile + static_cast<uint64_t>(warp) * (32 * kGatherWords);
+    // nearly always one frame's: its segment is looked up once
+    const int s_lo = segment_of(seg_start, nseg, wbase);
+    const int s_hi = segment_of(seg_start, nseg, wbase + 32 * kGatherWords - 1);
+    uint4 px[kGatherWords];
+    uint32_t before[kGatherWords]; // lane 0: the index before its pixel's
+    int seg[kGatherWords];
+#pragma unroll
+    for (int c = 0; c < kGatherWords; c++) {
+      const uint64_t g = wbase + 32 * c + lane;
+      seg[c] = s_lo;
+      before[c] = 0;
+      if (g < n && g >= carry) {
+        if (s_lo != s_hi)
+          seg[c] = segment_of(seg_start, nseg, g);
+        const uint64_t i = g - seg_start[seg[c]];
+        const SignalPixel *list = a.lists + a.offs[seg[c] - first_batch_seg];
+        px[c] = reinterpret_cast<const uint4 *>(list)[i];
+        if (lane == 0 && i > 0)
+          before[c] = list[i - 1].index;
+      }
+    }
+    uint32_t want[kGatherWords], run[kGatherWords], total = 0;
+#pragma unroll
+    for (int c = 0; c < kGatherWords; c++) {
+      const uint64_t base = wbase + 32 * c, g = base + lane;
+      const bool mine = g < n && g >= carry;
+      bool left = false;
+      const uint32_t shifted = __shfl_up_sync(kFull, px[c].x, 1);
+      if (mine) {
+        const uint64_t i = g - seg_start[seg[c]];
+        const uint32_t index = px[c].x;
+        const uint32_t prev = lane == 0 || i == 0 ? before[c] : shifted;
+        a.fr[g] = static_cast<int32_t>(seg_z[seg[c]]);
+        a.ix[g] = index;
+        a.val[g] = px[c].y;
+        left = i > 0 && prev + 1 == index && a.wdiv.rem(index) != 0;
         // This pixel is the first of every block from the one after the
         // previous pixel's up to its own.
-        uint32_t *tab = a.tab + static_cast<uint64_t>(f) * a.nblk;
-        const uint64_t b1 = px.index >> kBlockShift;
+        uint32_t *tab = a.tab + static_cast<uint64_t>(seg[c] - first_batch_seg) * a.nblk;
+        const uint64_t b1 = index >> kBlockShift;
         const uint64_t b0 = i == 0 ? 0 : (prev >> kBlockShift) + 1;
         for (uint64_t b = b0; b <= b1; b++)
           tab[b] = static_cast<uint32_t>(i);
-      } else if (g > sc->carry_last_start) {
+      } else if (g < n && g > carry_last) {
         // the carried last frame, which the first batch frame links to
         const uint32_t v = a.ix[g];
         left = a.ix[g - 1] + 1 == v && a.wdiv.rem(v) != 0;
       }
+      const uint32_t linked = __ballot_sync(kFull, left);
+      if (lane == 0 && base < n)
+        a.run_starts[base >> 5] = ~linked;
+      if (mine) {
+        // the run's first lane in this chunk: the highest lane at or below
+        // this one that is not joined to its left neighbour
+        const uint32_t starts = ~linked & (0xffffffffu >> (31 - lane));
+        const int first = starts ? 31 - __clz(starts) : 0;
+        a.par[g] = static_cast<uint32_t>(base + first);
+      }
+      // lab_link's work list: one entry per piece of a run within a chunk --
+      // its first position, its first pixel's index, its length, whether it
+      // continues a run from the chunk before (lane 0 joined to its left
+      // neighbour) and its frame segment, so that lab_link starts from one
+      // 16-byte load
+      const bool boundary = left && lane == 0;
+      const bool entry = mine && (!left || boundary);
+      if (entry || g < min(carry, n))
+        a.info[g] = RootInfo{0u, INT_MIN, kNone, 0u};
+      want[c] = __ballot_sync(kFull, entry);
+      // pieces end at the next piece, at a lane that is not ours, or at the
+      // chunk's end
+      const uint32_t stops = want[c] | ~__ballot_sync(kFull, mine);
+      const uint32_t after = lane == 31 ? 0u : stops & (0xfffffffeu << lane);
+      const uint32_t len = (after ? __ffs(after) - 1 : 32) - lane;
+      run[c] = len | (boundary ? 0x40u : 0u) | (static_cast<uint32_t>(seg[c]) << 8);
+      total += __popc(want[c]);
     }
-    const uint32_t linked = __ballot_sync(kFull, left);
-    if (lane == 0 && base < n)
-      a.run_starts[base >> 5] = ~linked;
-    const bool mine = g < n && g >= carry;
-    if (mine) {
-      // the run's first lane in this chunk: the highest lane at or below
-      // this one that is not joined to its left neighbour
-      const uint32_t starts = ~linked & (0xffffffffu >> (31 - lane));
-      const int first = starts ? 31 - __clz(starts) : 0;
-      a.par[g] = static_cast<uint32_t>(base + first);
-    }
-    // lab_link's work list: one entry per piece of a run within a chunk --
-    // its first position, its first pixel's index, its length, whether it
-    // continues a run from the chunk before (lane 0 joined to its left
-    // neighbour) and its frame segment, so that lab_link starts from one
-    // 16-byte load
-    const bool boundary = left && lane == 0;
-    const bool entry = mine && (!left || boundary);
-    if (entry || g < min(carry, n))
-      a.info[g] = RootInfo{0u, INT_MIN, kNone, 0u};
-    const uint32_t want = __ballot_sync(kFull, entry);
-    // pieces end at the next piece, at a lane that is not ours, or at the
-    // chunk's end
-    const uint32_t stops = want | ~__ballot_sync(kFull, mine);
-    const uint32_t after = lane == 31 ? 0u : stops & (0xfffffffeu << lane);
-    const uint32_t len = (after ? __ffs(after) - 1 : 32) - lane;
     if (lane == 0)
-      warp_count[warp] = __popc(want);
+      warp_count[warp] = total;
     __syncthreads();
     if (threadIdx.x == 0) {
-      uint32_t total = 0;
+      uint32_t all = 0;
       for (int w = 0; w < kThreads / 32; w++) {
         const uint32_t c = warp_count[w];
-        warp_count[w] = total;
-        total += c;
+        warp_count[w] = all;
+        all += c;
       }
-      block_at = total ? atomicAdd(&sc->runs_n, total) : 0u;
+      block_at = all ? atomicAdd(&sc->runs_n, all) : 0u;
     }
     __syncthreads();
-    if (entry)
-      a.runs[block_at + warp_count[warp] + __popc(want & ((1u << lane) - 1u))] =
-          make_uint4(static_cast<uint32_t>(g), pidx,
-                     len | (boundary ? 0x40u : 0u) | (static_cast<uint32_t>(seg) << 8), 0u);
+    uint32_t at = block_at + warp_count[warp];
+#pragma unroll
+    for (int c = 0; c < kGatherWords; c++) {
+      if ((want[c] >> lane) & 1u)
+        a.runs[at + __popc(want[c] & ((1u << lane) - 1u))] =
+            make_uint4(static_cast<uint32_t>(wbase + 32 * c + lane), px[c].x, run[c], 0u);
+      at += __popc(want[c]);
+    }
     __syncthreads();
   }
 }
@@ -1867,7 +1897,10 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   const unsigned grid = grid_;
   LabelScalars *sc = sc_;
   lab_setup<<<grid, kThreads, 0, s>>>(a);
-  lab_gather<<<grid, kThreads, 0, s>>>(a);
+  if (nframes >= kGatherFrames)
+    lab_gather<4><<<grid, kThreads, 0, s>>>(a);
+  else
+    lab_gather<1><<<grid, kThreads, 0, s>>>(a);
   lab_link<<<grid, kThreads, 0, s>>>(a);
   lab_flatten<<<grid, kThreads, 0, s>>>(a);
   lab_close<<<grid, kThreads, 0, s>>>(a);
