@@ -64,9 +64,6 @@ struct HostLabeller {
   }
 
   void collect() {
-    check(cudaMemcpyAsync(host_sc, dev->scalars(), sizeof(LabelScalars),
-                          cudaMemcpyDeviceToHost, stream),
-          "reading the labeller state");
     check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     if (host_sc->status != kLabelOk)
       throw DeviceError("labeller capacity exceeded (status " +
@@ -150,6 +147,8 @@ int sf_labeller_create(size_t height, size_t width, const sf_group_options *opti
     sf::check(cudaMalloc(&h->offs, sizeof(uint64_t)), "cudaMalloc");
     sf::check(cudaMemset(h->offs, 0, sizeof(uint64_t)), "cudaMemset");
     sf::check(cudaMallocHost(&h->host_sc, sizeof(sf::LabelScalars)), "cudaMallocHost");
+    std::memset(static_cast<void *>(h->host_sc), 0, sizeof(sf::LabelScalars));
+    h->dev->report_to(h->host_sc);
     sf::check(cudaStreamSynchronize(cudaStreamLegacy), "cudaMemset");
     *out = reinterpret_cast<sf_labeller *>(h.release());
     return 0;

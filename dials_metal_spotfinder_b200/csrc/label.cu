@@ -142,6 +142,7 @@ struct LabArgs {
   uint32_t *carry_tab; // block table of the carry's last frame
   uint64_t nblk;
   LabelScalars *sc;
+  LabelScalars *report; // page-locked host copy of *sc after the batch; or null
 };
 
 __device__ __forceinline__ uint64_t gtid() {
@@ -1592,29 +1593,8 @@ __device__ __forceinline__ uint32_t open_position(const LabArgs &a, uint64_t g) 
   return a.ocnt[g >> 5] + __popc(a.obits[g >> 5] & ((1u << (g & 31)) - 1u));
 }
 
-// The open pixels to the other live buffer, in order, a warp per
-// 32-position word (most words hold none). One thread closes the batch's
-// books, none of which the other blocks read: the running counts and what
-// the next batch starts from.
-__global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
+__device__ void close_books(const LabArgs &a) {
   LabelScalars *sc = a.sc;
-  const uint64_t nw = sc->nw;
-  const int lane = threadIdx.x & 31;
-  const uint64_t warps = gstride() >> 5;
-  for (uint64_t w = gtid() >> 5; w < nw; w += warps) {
-    const uint32_t bits = a.obits[w], cnt = a.ocnt[w]; // read together
-    if (!((bits >> lane) & 1u))
-      continue;
-    const uint64_t g = w * 32 + static_cast<uint64_t>(lane);
-    const uint32_t at = cnt + __popc(bits & ((1u << lane) - 1u));
-    const uint32_t r = a.root[g];
-    a.nfr[at] = a.fr[g];
-    a.nix[at] = a.ix[g];
-    a.nval[at] = a.val[g];
-    a.npar[at] = open_position(a, r); // the root is open too, and comes first
-  }
-  if (gtid() != 0)
-    return;
   const bool all = a.close_all || a.two_d || a.nframes == 0;
   sc->groups += sc->closed;
   const uint64_t rows = sc->accepted_pack & kPackLow;
@@ -1630,6 +1610,36 @@ __global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
   // lands (with anything carried, the last frame has pixels).
   sc->carry_last_start = sc->carry_n > 0 ? open_position(a, a.seg_start[sc->nseg - 1]) : 0;
   sc->batch_z0 += a.nframes;
+  if (a.report)
+    *a.report = *sc;
+}
+
+// The open pixels to the other live buffer, in order, a warp per
+// 32-position word (most words hold none). One thread of the last block, which
+// has the fewest words, closes the batch's books before its share of them:
+// the running counts and what the next batch starts from, none of which the
+// other blocks read, and their copy in host memory, which the host then has
+// as soon as the stream has passed (a copy of its own, and a second wait, cost
+// every reader 14 us).
+__global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
+  LabelScalars *sc = a.sc;
+  const uint64_t nw = sc->nw;
+  const int lane = threadIdx.x & 31;
+  const uint64_t warps = gstride() >> 5;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+    close_books(a);
+  for (uint64_t w = gtid() >> 5; w < nw; w += warps) {
+    const uint32_t bits = a.obits[w], cnt = a.ocnt[w]; // read together
+    if (!((bits >> lane) & 1u))
+      continue;
+    const uint64_t g = w * 32 + static_cast<uint64_t>(lane);
+    const uint32_t at = cnt + __popc(bits & ((1u << lane) - 1u));
+    const uint32_t r = a.root[g];
+    a.nfr[at] = a.fr[g];
+    a.nix[at] = a.ix[g];
+    a.nval[at] = a.val[g];
+    a.npar[at] = open_position(a, r); // the root is open too, and comes first
+  }
 }
 
 } // namespace
@@ -1893,6 +1903,7 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   a.carry_tab = carry_tab_;
   a.nblk = nblk_;
   a.sc = sc_;
+  a.report = report_;
 
   const unsigned grid = grid_;
   LabelScalars *sc = sc_;

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cstring>
 #include <memory>
 #include <string>
 #include <vector>
@@ -58,7 +59,7 @@ struct Engine {
   };
   std::vector<Series> series;
   int parity = 0;
-  LabelScalars *host_sc = nullptr;
+  LabelScalars *host_sc = nullptr; // per series, written by its labeller's batches
   // Compressed uploads, decoded on the device in the copy stream.
   DeviceChunkDecoder decoder;
   // Host threads for the framing walks of a batch of chunks, made on first
@@ -294,7 +295,8 @@ struct Engine {
       }
       members[k].push_back(f);
     }
-    check(cudaMallocHost(&host_sc, sizeof(LabelScalars)), "cudaMallocHost");
+    check(cudaMallocHost(&host_sc, series.size() * sizeof(LabelScalars)), "cudaMallocHost");
+    std::memset(static_cast<void *>(host_sc), 0, series.size() * sizeof(LabelScalars));
     for (size_t k = 0; k < series.size(); k++) {
       Series &se = series[k];
       const std::vector<int32_t> &fs = members[k];
@@ -318,6 +320,7 @@ struct Engine {
             "copy");
       check(cudaMemcpy(se.d_map, fs.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice), "copy");
       se.lab = std::make_unique<DeviceLabeller>(se.height, se.width, opt);
+      se.lab->report_to(host_sc + k);
       se.lab->reserve(total, se.nframes, carry_cap ? carry_cap : 2 * biggest + (1u << 20));
       se.lab->set_next_frame(first_frame, group);
     }
@@ -334,15 +337,12 @@ struct Engine {
   }
 
   const LabelScalars &group_state(int k) {
-    Series &se = series_at(k);
-    check(cudaMemcpyAsync(host_sc, se.lab->scalars(), sizeof(LabelScalars),
-                          cudaMemcpyDeviceToHost, group),
-          "reading the grouping state");
+    series_at(k);
     check(cudaStreamSynchronize(group), "cudaStreamSynchronize");
-    if (host_sc->status != kLabelOk)
-      throw DeviceError("grouping capacity exceeded (status " + std::to_string(host_sc->status) +
-                        ")");
-    return *host_sc;
+    const LabelScalars &sc = host_sc[k];
+    if (sc.status != kLabelOk)
+      throw DeviceError("grouping capacity exceeded (status " + std::to_string(sc.status) + ")");
+    return sc;
   }
 
   void upload(int slot, int frame, const void *host) {

@@ -124,6 +124,9 @@ public:
   int parity() const { return cur_; }
 
   LabelScalars *scalars() const { return sc_; }
+  // Page-locked host memory that each batch leaves a copy of the scalars in
+  // (there once its stream has passed); set before the first one.
+  void report_to(LabelScalars *host) { report_ = host; }
   Spot *batch_spots() const { return spots_out_; }
   Pixel *batch_pixels() const { return kept_out_; }
   uint64_t spot_capacity() const { return spot_cap_; }
@@ -178,6 +181,7 @@ private:
   uint64_t nblk_ = 0;
   unsigned grid_ = 0;
   LabelScalars *sc_ = nullptr;
+  LabelScalars *report_ = nullptr;
   cudaStream_t aux_ = nullptr;  // the large components' spot pass
   cudaStream_t aux2_ = nullptr; // the middle-sized components' spot pass
   cudaEvent_t fork_ = nullptr, join_ = nullptr, join2_ = nullptr;
