@@ -479,9 +479,7 @@ int sf_engine_finish(sf_engine *engine) {
     Engine *e = reinterpret_cast<Engine *>(engine);
     if (e->series.empty())
       throw std::invalid_argument("grouping is not enabled");
-    for (Engine::Series &se : e->series)
-      se.lab->enqueue(0, e->plan->out(0), se.d_offs, e->plan->frame_count(0), se.d_map,
-                      se.d_caps, true, e->group);
+    e->enqueue_series(0, true);
     e->parity ^= 1;
     return 0;
   });

@@ -404,9 +404,7 @@ struct Server {
       if (se.error.empty()) {
         Engine &e = *se.eng;
         // finish() closes what is open; its spots are read back directly
-        for (Engine::Series &s : e.series)
-          s.lab->enqueue(0, e.plan->out(0), s.d_offs, e.plan->frame_count(0), s.d_map,
-                         s.d_caps, true, e.group);
+        e.enqueue_series(0, true);
         e.parity ^= 1;
         e.synchronize();
         collect_direct(se);
