@@ -3,7 +3,7 @@
 // gpu::find<T> (src/dext_cuda.cu:585-728).
 //
 // Per host thread: one stream, one ThresholdPlan for the last frame shape
-// seen, a pinned word for the count and five events for stage profiling --
+// seen, a page-locked head of the list and five events for stage profiling --
 // created on first use and reused, so a steady stream of same-shaped frames
 // allocates nothing after the first.
 
@@ -46,11 +46,7 @@ private:
 struct FindWorkspace {
   cudaStream_t stream = nullptr;
   cudaEvent_t marks[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  // the count, the status word and, kListsAt bytes in, the list's first
-  // kHeadRecords records, which come back in one copy: a short list needs no
-  // second one and no second wait (256 x 384: 73 -> 61 us a call)
-  static constexpr size_t kHeadRecords = 1024;
-  unsigned char *pinned = nullptr;
+  HostHead *head = nullptr; // written by the placement
   std::unique_ptr<ThresholdPlan> plan;
   int eb = 0;
   size_t h = 0, w = 0;
@@ -63,17 +59,16 @@ struct FindWorkspace {
     for (cudaEvent_t &e : marks)
       if (e)
         cudaEventDestroy(e);
-    if (pinned)
-      cudaFreeHost(pinned);
+    if (head)
+      cudaFreeHost(head);
     plan.reset();
   }
 
   void prepare(int elem_bytes, size_t height, size_t width) {
     if (!stream)
       check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
-    if (!pinned)
-      check(cudaMallocHost(&pinned, ThresholdPlan::kListsAt + kHeadRecords * sizeof(SignalPixel)),
-            "cudaMallocHost");
+    if (!head)
+      check(cudaMallocHost(&head, sizeof(HostHead)), "cudaMallocHost");
     if (plan && eb == elem_bytes && h == height && w == width)
       return;
     cudaStreamSynchronize(stream);
@@ -122,19 +117,13 @@ int find_impl(int elem_bytes, const void *image, size_t height, size_t width,
   plan.upload(0, 0, image, s);
   if (timing)
     check(cudaEventRecord(ev[1], s), "cudaEventRecord");
-  plan.enqueue(0, s, timing ? ev[2] : nullptr);
+  plan.enqueue(0, s, timing ? ev[2] : nullptr, ws.head);
   if (timing)
     check(cudaEventRecord(ev[3], s), "cudaEventRecord");
-  const size_t head = std::min<size_t>(
-      {FindWorkspace::kHeadRecords, plan.capacity(0), capacity});
-  check(cudaMemcpyAsync(ws.pinned, plan.frame_count(0),
-                        ThresholdPlan::kListsAt + head * sizeof(SignalPixel),
-                        cudaMemcpyDeviceToHost, s),
-        "reading the signal count back");
   check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
 
-  const uint32_t count = reinterpret_cast<const uint32_t *>(ws.pinned)[0];
-  const int status = reinterpret_cast<const int *>(ws.pinned)[1];
+  const uint32_t count = ws.head->count;
+  const int status = ws.head->status;
   if (status == kStatusTmaTimeout)
     throw DeviceError("a TMA load did not complete in time");
   *found = count;
@@ -153,14 +142,14 @@ int find_impl(int elem_bytes, const void *image, size_t height, size_t width,
   const bool fits = count <= plan.capacity(0) && count <= capacity;
   const auto t0 = std::chrono::steady_clock::now();
   if (fits) {
+    const uint32_t head = std::min(count, HostHead::kRecords);
     const bool rest = count > head;
     if (rest)
       check(cudaMemcpyAsync(out + head, plan.out(0) + head, (count - head) * sizeof(SignalPixel),
                             cudaMemcpyDeviceToHost, s),
             "copying the signal pixels back");
     if (count > 0)
-      std::memcpy(out, ws.pinned + ThresholdPlan::kListsAt,
-                  std::min<size_t>(count, head) * sizeof(SignalPixel));
+      std::memcpy(out, ws.head->list, head * sizeof(SignalPixel));
     if (rest)
       check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
   }

@@ -253,6 +253,7 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   P.frame_count = count;
   P.run_status = run_status;
   P.status = status;
+  P.head = nullptr;
   check(launch_place(P, s), "launching the placement");
 
   uint32_t host_words[2] = {0, 0};

@@ -92,8 +92,14 @@ __global__ void __launch_bounds__(kPlaceThreads) place_copy(PlaceLaunch L) {
   }
   if (counts && threadIdx.x == 0) {
     L.frame_count[f] = all;
-    if (group == 0)
-      *L.status = *L.run_status;
+    if (group == 0) {
+      const int status = *L.run_status;
+      *L.status = status;
+      if (L.head) {
+        L.head->count = all;
+        L.head->status = status;
+      }
+    }
   }
   const uint32_t mine = piece_s[lane];
   const uint32_t piece_at = warp_incl_scan(mine, lane) - mine; // of piece `lane`
@@ -131,8 +137,11 @@ __global__ void __launch_bounds__(kPlaceThreads) place_copy(PlaceLaunch L) {
 #pragma unroll
       for (int u = 0; u < kU; u++) {
         const uint32_t k = base + 32 * u + lane;
-        if (k < total && at + k < fd.capacity)
+        if (k < total && at + k < fd.capacity) {
           out[at + k] = v[u];
+          if (L.head && at + k < HostHead::kRecords)
+            reinterpret_cast<uint4 *>(L.head->list)[at + k] = v[u];
+        }
       }
     }
   }

@@ -240,10 +240,10 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     for (Slot &sl : slots_) {
       alloc(&sl.arena, arena_bytes, "cudaMalloc arena");
       check(cudaMemset(sl.arena, 0xff, arena_bytes), "filling the arena");
-      const uint64_t head = round_up((nf + 1) * 4, kListsAt);
-      alloc(reinterpret_cast<void **>(&sl.frame_count),
-            head + total_capacity_ * sizeof(SignalPixel), "cudaMalloc output lists");
-      sl.out = reinterpret_cast<SignalPixel *>(reinterpret_cast<char *>(sl.frame_count) + head);
+      alloc(reinterpret_cast<void **>(&sl.out), total_capacity_ * sizeof(SignalPixel),
+            "cudaMalloc output lists");
+      alloc(reinterpret_cast<void **>(&sl.frame_count), (nf + 1) * 4,
+            "cudaMalloc frame counts");
       sl.status = reinterpret_cast<int *>(sl.frame_count + nf);
       check(cudaMemset(sl.frame_count, 0, (nf + 1) * 4), "clearing frame counts");
       encode_arena_map(&sl.map, sl.arena, elem_bytes_, pitch_, arena_rows_);
@@ -262,7 +262,8 @@ ThresholdPlan::~ThresholdPlan() { release(); }
 void ThresholdPlan::release() {
   for (Slot &sl : slots_) {
     cudaFree(sl.arena);
-    cudaFree(sl.frame_count); // and the lists after it
+    cudaFree(sl.out);
+    cudaFree(sl.frame_count);
     sl = Slot();
   }
   cudaFree(frames_);
@@ -321,7 +322,7 @@ void ThresholdPlan::upload_device(int slot, int f, const void *device, size_t pi
         "copying a frame into the arena");
 }
 
-void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid) {
+void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid, HostHead *head) {
   Slot &sl = slots_.at(slot);
   check(cudaMemsetAsync(ranges_, 0, cleared_bytes_, stream), "clearing tile counts");
   ThresholdLaunch L;
@@ -360,6 +361,7 @@ void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid) {
   P.frame_count = sl.frame_count;
   P.run_status = run_status_;
   P.status = sl.status;
+  P.head = head;
   check(launch_place(P, stream), "launching the placement");
 }
 

@@ -54,6 +54,17 @@ cudaError_t launch_threshold(const CUtensorMap &map, const ThresholdLaunch &L,
 template <typename T> size_t threshold_smem_bytes(int wpc);
 template <typename T> int threshold_occupancy(int wpc);
 
+// What a one-frame batch leaves in page-locked host memory besides its list on
+// the device: the count, the status and the list's first records, so that a
+// short list needs no copy and no second wait.
+struct HostHead {
+  static constexpr uint32_t kRecords = 1024;
+  uint32_t count;
+  int status;
+  uint32_t pad[2];
+  SignalPixel list[kRecords];
+};
+
 // Ordered compaction of the staged records (place.cu). Every frame's
 // tile_base is a multiple of kPlaceTiles.
 struct PlaceLaunch {
@@ -69,6 +80,7 @@ struct PlaceLaunch {
   uint32_t *frame_count; // nframes
   const int *run_status; // the threshold's status, copied to *status
   int *status;
+  HostHead *head; // a one-frame batch's, in page-locked host memory; or null
 };
 constexpr int kPlaceThreads = 256;
 constexpr int kPlaceTiles = 1024;
@@ -121,7 +133,9 @@ public:
   // Enqueue the threshold of slot `slot` on `stream`: clears, threshold,
   // placement. When `mid` is given it is recorded between the threshold and
   // the placement, so the two can be timed apart.
-  void enqueue(int slot, cudaStream_t stream, cudaEvent_t mid = nullptr);
+  // `head`, of a plan of one frame: see HostHead.
+  void enqueue(int slot, cudaStream_t stream, cudaEvent_t mid = nullptr,
+               HostHead *head = nullptr);
 
   // Copy a frame (row-major, height x width; host, device or managed memory)
   // into frame f of a slot. Frames of kLinearUpload bytes and more go through
@@ -142,9 +156,6 @@ public:
   SignalPixel *out(int slot) const { return slots_[slot].out; }
   uint64_t out_base(int f) const { return host_frames_[f].out_base; }
   uint32_t capacity(int f) const { return host_frames_[f].capacity; }
-  // The counts, with the status word after the last; the lists follow them
-  // in the same allocation, from a multiple of kListsAt bytes on.
-  static constexpr uint64_t kListsAt = 256;
   uint32_t *frame_count(int slot) const { return slots_[slot].frame_count; }
   int *status(int slot) const { return slots_[slot].status; }
   uint32_t ntasks() const { return ntasks_; }
