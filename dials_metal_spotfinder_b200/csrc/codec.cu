@@ -306,6 +306,14 @@ ChunkLayout parse_chunk(int algorithm, const uint8_t *data, size_t nbytes, size_
   return L;
 }
 
+bool may_copy_first(int algorithm, size_t nbytes, size_t n_elems, size_t elem) {
+  // a chunk of blocks that did not compress is a few bytes a block longer
+  // than its frame; one of many tiny blocks may be longer yet, and waits
+  const size_t bytes = n_elems * elem;
+  return (algorithm == SF_CHUNK_LZ4 || algorithm == SF_CHUNK_BSLZ4) && nbytes >= kHeader &&
+         nbytes <= bytes + bytes / 8;
+}
+
 void decode_chunk_host(const uint8_t *data, const ChunkLayout &L, uint8_t *out) {
   if (L.algorithm == SF_CHUNK_RAW) {
     std::memcpy(out, data, L.n_elems * L.elem);

@@ -956,9 +956,20 @@ void DeviceChunkDecoder::enqueue_raw(const void *src, size_t height, size_t row_
   check(cudaEventRecord(S.freed, s), "cudaEventRecord");
 }
 
+int DeviceChunkDecoder::start_copy(const uint8_t *chunk, size_t nbytes) {
+  Set &S = next_set(round16(nbytes) + 16);
+  check(cudaMemcpyAsync(S.d_in, chunk, nbytes, cudaMemcpyDefault, h2d_), "copying a chunk");
+  return static_cast<int>(&S - sets_);
+}
+
+void DeviceChunkDecoder::abandon() noexcept {
+  if (h2d_)
+    cudaStreamSynchronize(h2d_);
+}
+
 void DeviceChunkDecoder::enqueue(const uint8_t *chunk, size_t nbytes, const ChunkLayout &L,
                                  size_t height, size_t width, void *dst, size_t dst_pitch,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, int started) {
   const size_t row_bytes = width * L.elem;
   if (L.algorithm == SF_CHUNK_RAW) {
     enqueue_raw(chunk, height, row_bytes, dst, dst_pitch, s);
@@ -970,7 +981,7 @@ void DeviceChunkDecoder::enqueue(const uint8_t *chunk, size_t nbytes, const Chun
   const size_t nb = L.block_in.size();
   if (nb == 0 && L.raw_bytes == 0)
     return;
-  Set &S = next_set(round16(nbytes) + 16);
+  Set &S = sets_[started == kNotStarted ? start_copy(chunk, nbytes) : started];
   Table &T = next_table(std::max<size_t>(nb, 1));
   BlockDesc *t = static_cast<BlockDesc *>(T.h);
   uint32_t max_len = 0;
@@ -978,13 +989,12 @@ void DeviceChunkDecoder::enqueue(const uint8_t *chunk, size_t nbytes, const Chun
     t[b] = BlockDesc{L.block_in[b], L.block_out[b], L.block_len[b], L.block_n[b]};
     max_len = std::max(max_len, L.block_len[b]);
   }
-  check(cudaMemcpyAsync(S.d_in, chunk, nbytes, cudaMemcpyDefault, h2d_), "copying a chunk");
   if (nb)
     check(cudaMemcpyAsync(T.d, T.h, nb * sizeof(BlockDesc), cudaMemcpyHostToDevice, h2d_),
           "copying a block table");
-  check(cudaEventRecord(S.copied, h2d_), "cudaEventRecord");
+  // the chunk's copy was enqueued before the table's
   check(cudaEventRecord(T.copied, h2d_), "cudaEventRecord");
-  check(cudaStreamWaitEvent(s, S.copied, 0), "ordering after the copy");
+  check(cudaStreamWaitEvent(s, T.copied, 0), "ordering after the copies");
 
   const uint64_t frame_bytes = static_cast<uint64_t>(height) * row_bytes;
   const auto *tbl = static_cast<const BlockDesc *>(T.d);
@@ -1065,9 +1075,6 @@ extern "C" int sf_chunk_decode_device(int algorithm, const void *chunk, size_t n
     if (!chunk || !device_image || height == 0 || width == 0 ||
         (elem_bytes != 2 && elem_bytes != 4) || pitch_bytes < width * elem_bytes)
       return -1;
-    const sf::ChunkLayout L =
-        sf::parse_chunk(algorithm, static_cast<const uint8_t *>(chunk), nbytes, height * width,
-                        static_cast<size_t>(elem_bytes));
     // per host thread: a stream and a decoder, reused by later calls
     struct Local {
       cudaStream_t s = nullptr;
@@ -1082,8 +1089,18 @@ extern "C" int sf_chunk_decode_device(int algorithm, const void *chunk, size_t n
     static thread_local Local loc;
     if (!loc.s)
       sf::check(cudaStreamCreateWithFlags(&loc.s, cudaStreamNonBlocking), "cudaStreamCreate");
-    loc.dec.enqueue(static_cast<const uint8_t *>(chunk), nbytes, L, height, width, device_image,
-                    pitch_bytes, loc.s);
+    const auto *bytes = static_cast<const uint8_t *>(chunk);
+    const size_t eb = static_cast<size_t>(elem_bytes);
+    const int started = sf::may_copy_first(algorithm, nbytes, height * width, eb)
+                            ? loc.dec.start_copy(bytes, nbytes)
+                            : sf::DeviceChunkDecoder::kNotStarted;
+    try {
+      const sf::ChunkLayout L = sf::parse_chunk(algorithm, bytes, nbytes, height * width, eb);
+      loc.dec.enqueue(bytes, nbytes, L, height, width, device_image, pitch_bytes, loc.s, started);
+    } catch (...) {
+      loc.dec.abandon();
+      throw;
+    }
     sf::check(cudaStreamSynchronize(loc.s), "cudaStreamSynchronize");
     if (loc.dec.take_error())
       throw sf::DeviceError("a malformed LZ4 block");

@@ -34,6 +34,10 @@ void encode_chunk(int algorithm, const uint8_t *in, size_t n_elems, size_t elem,
 // against the frame; throws std::invalid_argument on a mismatch.
 ChunkLayout parse_chunk(int algorithm, const uint8_t *data, size_t nbytes, size_t n_elems,
                         size_t elem);
+// Whether a chunk's bytes may go to the device before its framing has been
+// checked: a compressed one of about the frame's size at most, so that a
+// chunk that will be refused takes no more staging memory than a good one.
+bool may_copy_first(int algorithm, size_t nbytes, size_t n_elems, size_t elem);
 void decode_chunk_host(const uint8_t *data, const ChunkLayout &L, uint8_t *out);
 
 // Brings frames from host memory into device frames (decode.cu): compressed
@@ -56,8 +60,18 @@ public:
   DeviceChunkDecoder(const DeviceChunkDecoder &) = delete;
   DeviceChunkDecoder &operator=(const DeviceChunkDecoder &) = delete;
 
+  // `started`: the chunk's start_copy(), whose bytes are on their way.
   void enqueue(const uint8_t *chunk, size_t nbytes, const ChunkLayout &L, size_t height,
-               size_t width, void *dst, size_t dst_pitch, cudaStream_t s);
+               size_t width, void *dst, size_t dst_pitch, cudaStream_t s,
+               int started = kNotStarted);
+  // Starts the copy of a chunk whose framing is still to be checked, so that
+  // its bytes cross the link while the host walks them. Up to kSets chunks,
+  // each then given to enqueue() in the same order and before any other.
+  // Where that fails, abandon() waits for the copies, after which the
+  // caller's memory is free again; no decode reads what they brought.
+  int start_copy(const uint8_t *chunk, size_t nbytes);
+  void abandon() noexcept;
+  static constexpr int kNotStarted = -1;
   // A raw frame of height rows of row_bytes each, contiguous at `src` (host
   // or device memory).
   void enqueue_raw(const void *src, size_t height, size_t row_bytes, void *dst, size_t dst_pitch,
@@ -80,7 +94,7 @@ private:
   struct Set {
     uint8_t *d_in = nullptr;
     size_t in_cap = 0;
-    cudaEvent_t copied = nullptr; // its host-to-device copies are done
+    cudaEvent_t copied = nullptr; // a raw frame's host-to-device copy is done
     cudaEvent_t freed = nullptr;  // the decode that read it is done
     bool used = false;
   };
