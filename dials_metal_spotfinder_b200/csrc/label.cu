@@ -1665,8 +1665,8 @@ DeviceLabeller::DeviceLabeller(int height, int width, const GroupOptions &option
         "cudaFuncSetAttribute");
   grid_ = static_cast<unsigned>(device_sm_count() * 8);
   check(cudaMallocHost(&z_stage_, sizeof(int64_t)), "cudaMallocHost");
-  check(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking), "cudaStreamCreate");
-  check(cudaStreamCreateWithFlags(&aux2_, cudaStreamNonBlocking), "cudaStreamCreate");
+  aux_ = create_stream(2);
+  aux2_ = create_stream(2);
   check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&join2_, cudaEventDisableTiming), "cudaEventCreate");

@@ -115,6 +115,15 @@ void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes, uint64_t pit
     throw DeviceError("cuTensorMapEncodeTiled failed with code " + std::to_string(r));
 }
 
+cudaStream_t create_stream(int rank) {
+  int least = 0, greatest = 0;
+  check(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange");
+  cudaStream_t s = nullptr;
+  check(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, std::max(greatest, least - rank)),
+        "cudaStreamCreate");
+  return s;
+}
+
 int device_sm_count() {
   int dev = 0, n = 0;
   check(cudaGetDevice(&dev), "cudaGetDevice");

@@ -334,7 +334,7 @@ struct Engine {
       members[k].push_back(f);
     }
     for (size_t k = 0; k < std::min(series.size() - 1, kSide); k++) {
-      check(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking), "cudaStreamCreate");
+      side[k] = create_stream(2);
       check(cudaEventCreateWithFlags(&joins[k], cudaEventDisableTiming), "cudaEventCreate");
     }
     if (series.size() > 1)

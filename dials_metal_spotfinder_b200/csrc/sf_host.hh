@@ -105,6 +105,10 @@ void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes,
 
 int device_sm_count();
 
+// A non-blocking stream whose waiting blocks are placed `rank` steps before a
+// plain one's (rank 0), as far as the device has steps.
+cudaStream_t create_stream(int rank);
+
 // Launch geometry of the threshold for one batch shape.
 struct PlanTuning {
   int seg_rows = 0;        // output rows per task; 0 picks by frame count
