@@ -31,9 +31,8 @@ struct HostLabeller {
   uint64_t height = 0, width = 0;
   SignalPixel *list = nullptr;
   uint64_t list_cap = 0;
-  uint32_t *meta = nullptr; // count, capacity
-  uint64_t *offs = nullptr; // {0}
   LabelScalars *host_sc = nullptr;
+  LabelHead *head = nullptr; // page-locked: a small batch's results
   uint64_t carry = 0;
 
   ~HostLabeller() {
@@ -41,10 +40,10 @@ struct HostLabeller {
       cudaStreamSynchronize(stream);
     dev.reset();
     cudaFree(list);
-    cudaFree(meta);
-    cudaFree(offs);
     if (host_sc)
       cudaFreeHost(host_sc);
+    if (head)
+      cudaFreeHost(head);
     if (stream)
       cudaStreamDestroy(stream);
   }
@@ -63,12 +62,30 @@ struct HostLabeller {
     }
   }
 
-  void collect() {
+  // Before a batch of `pixels`: whether its results will be in the head, if
+  // they fit there.
+  bool want_head(uint64_t pixels) {
+    if (!DeviceLabeller::takes_head(pixels))
+      return false;
+    if (!head) {
+      check(cudaMallocHost(&head, sizeof(LabelHead)), "cudaMallocHost");
+      dev->head_to(head);
+    }
+    return true;
+  }
+
+  void collect(bool in_head) {
     check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    if (host_sc->status != kLabelOk)
-      throw DeviceError("labeller capacity exceeded (status " +
-                        std::to_string(host_sc->status) + ")");
-    const uint64_t ns = host_sc->batch_spots, np = host_sc->batch_pixels;
+    const LabelScalars &sc = *host_sc;
+    if (sc.status != kLabelOk)
+      throw DeviceError("labeller capacity exceeded (status " + std::to_string(sc.status) + ")");
+    const uint64_t ns = sc.batch_spots, np = sc.batch_pixels;
+    if (in_head && ns <= LabelHead::kSpots && np <= LabelHead::kPixels) {
+      spots.insert(spots.end(), head->spots, head->spots + ns);
+      pixels.insert(pixels.end(), head->pixels, head->pixels + np);
+      carry = sc.carry_n;
+      return;
+    }
     const size_t s0 = spots.size(), p0 = pixels.size();
     spots.resize(s0 + ns);
     pixels.resize(p0 + np);
@@ -81,7 +98,7 @@ struct HostLabeller {
                             cudaMemcpyDeviceToHost, stream),
             "reading spot pixels");
     check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    carry = host_sc->carry_n;
+    carry = sc.carry_n;
   }
 
   void add(int64_t frame, const sf_signal_pixel *sig, size_t n) {
@@ -97,11 +114,9 @@ struct HostLabeller {
     if (n)
       check(cudaMemcpyAsync(list, sig, n * sizeof(SignalPixel), cudaMemcpyHostToDevice, stream),
             "copying the signal list");
-    const uint32_t m[2] = {static_cast<uint32_t>(n), static_cast<uint32_t>(n)};
-    check(cudaMemcpyAsync(meta, m, sizeof(m), cudaMemcpyHostToDevice, stream), "copying counts");
-    dev->set_next_frame(frame, stream);
-    dev->enqueue(1, list, offs, meta, nullptr, meta + 1, false, stream);
-    collect();
+    const bool in_head = want_head(carry + n);
+    dev->enqueue_frame(frame, list, static_cast<uint32_t>(n), carry, stream);
+    collect(in_head);
     started = true;
     last = frame;
   }
@@ -110,8 +125,9 @@ struct HostLabeller {
     if (!started)
       return;
     dev->reserve(1, 1, carry + 1, true);
-    dev->enqueue(0, list, offs, meta, nullptr, meta + 1, true, stream);
-    collect();
+    const bool in_head = want_head(carry);
+    dev->enqueue_rest(carry, stream);
+    collect(in_head);
   }
 };
 
@@ -143,13 +159,9 @@ int sf_labeller_create(size_t height, size_t width, const sf_group_options *opti
     h->dev = std::make_unique<sf::DeviceLabeller>(static_cast<int>(height),
                                                   static_cast<int>(width), opt);
     sf::check(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
-    sf::check(cudaMalloc(&h->meta, 2 * sizeof(uint32_t)), "cudaMalloc");
-    sf::check(cudaMalloc(&h->offs, sizeof(uint64_t)), "cudaMalloc");
-    sf::check(cudaMemset(h->offs, 0, sizeof(uint64_t)), "cudaMemset");
     sf::check(cudaMallocHost(&h->host_sc, sizeof(sf::LabelScalars)), "cudaMallocHost");
     std::memset(static_cast<void *>(h->host_sc), 0, sizeof(sf::LabelScalars));
     h->dev->report_to(h->host_sc);
-    sf::check(cudaStreamSynchronize(cudaStreamLegacy), "cudaMemset");
     *out = reinterpret_cast<sf_labeller *>(h.release());
     return 0;
   });

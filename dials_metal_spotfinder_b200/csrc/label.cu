@@ -37,6 +37,8 @@
 //             the other live buffer and re-rooted at their first pixel;
 //             running counts and the carry for the next batch
 //
+// Small batches run the same steps in three launches (lab_small_open).
+//
 // close and each scan are one launch (sf_lookback.cuh), where a scan was
 // three: a batch took 32 launches and takes 16, and a one-frame batch is bound
 // by them. (scatter and write finding their places the same way, without the
@@ -67,6 +69,12 @@ constexpr int kThreads = kTileThreads;
 // launches with larger buffers.
 constexpr uint32_t kSmallCap = 256;
 constexpr uint32_t kMidCap = 512;
+// Batches of up to this many pixels, carried ones too, take the launches of
+// one block (lab_small_open, lab_small_close), where the host knows how many
+// there are: a frame added to a series and its results read took 186 us with
+// the launches of many and takes 124 at 1.1 k pixels, 143 at 2.6 k and 157 at
+// 3.2 k on average (their most 1.9 k, 4.4 k and 5.3 k); the two meet at 7 k.
+constexpr uint64_t kSmallPixels = 4096;
 constexpr int kGatherFrames = 4; // see lab_gather
 // 32-position words a warp of lab_scatter takes at a time.
 constexpr int kScatterWords = 4;
@@ -115,6 +123,9 @@ struct LabArgs {
   const uint32_t *counts;
   const int32_t *count_map; // frame f's count is counts[count_map[f]]; null: counts[f]
   const uint32_t *caps;
+  // a batch of one frame known to the host: counts and caps are null
+  uint32_t one_count;
+  int64_t one_z;
   int32_t *fr;
   uint32_t *ix, *val, *par;
   int32_t *nfr;
@@ -143,6 +154,7 @@ struct LabArgs {
   uint64_t nblk;
   LabelScalars *sc;
   LabelScalars *report; // page-locked host copy of *sc after the batch; or null
+  LabelHead *head;      // lab_small_close: and of its spots and pixels; or null
 };
 
 __device__ __forceinline__ uint64_t gtid() {
@@ -268,7 +280,7 @@ __device__ __forceinline__ uint64_t block_prefix(uint64_t v, uint64_t *total) {
 
 // Block 0's first warp lays out the frame segments; every block clears its
 // share of the batch frames' block tables.
-__global__ void __launch_bounds__(kThreads) lab_setup(LabArgs a) {
+__device__ __forceinline__ void setup_step(const LabArgs &a) {
   const uint64_t words = static_cast<uint64_t>(a.nframes) * a.nblk;
   for (uint64_t i = gtid(); i < words / 4; i += gstride())
     reinterpret_cast<uint4 *>(a.tab)[i] = make_uint4(kNone, kNone, kNone, kNone);
@@ -279,8 +291,10 @@ __global__ void __launch_bounds__(kThreads) lab_setup(LabArgs a) {
   const int lane = threadIdx.x;
   LabelScalars *sc = a.sc;
   const uint64_t carry = sc->carry_n;
-  const int64_t z0 = sc->batch_z0;
+  const int64_t z0 = a.counts || a.nframes == 0 ? sc->batch_z0 : a.one_z;
   const int first = carry > 0 ? 1 : 0;
+  if (lane == 0 && !a.counts && a.nframes > 0)
+    sc->batch_z0 = z0;
   if (lane == 0 && first) {
     a.seg_z[0] = sc->carry_last_z;
     a.seg_start[0] = sc->carry_last_start;
@@ -292,7 +306,7 @@ __global__ void __launch_bounds__(kThreads) lab_setup(LabArgs a) {
     const int f = f0 + lane;
     uint64_t c = 0;
     if (f < a.nframes) // an over-dense frame: its list holds only caps[f]
-      c = min(a.counts[a.count_map ? a.count_map[f] : f], a.caps[f]);
+      c = a.counts ? min(a.counts[a.count_map ? a.count_map[f] : f], a.caps[f]) : a.one_count;
     uint64_t incl = c;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -365,7 +379,7 @@ __device__ __forceinline__ const uint32_t *table_of(const LabArgs &a, int s, int
 // for batches of fewer than kGatherFrames frames, which four leave with too
 // few warps (one frame of 2162 x 2068 11 us; 13 with four).
 template <int kGatherWords>
-__global__ void __launch_bounds__(kThreads) lab_gather(LabArgs a) {
+__device__ __forceinline__ void gather_step(const LabArgs &a) {
   LabelScalars *sc = a.sc;
   const uint64_t n = sc->n, carry = sc->carry_n, carry_last = sc->carry_last_start;
   const int nseg = static_cast<int>(sc->nseg);
@@ -578,7 +592,7 @@ __device__ __forceinline__ uint32_t unite_overlaps(const LabArgs &a, uint32_t ra
 // here. The first pixel of each run then unites it with every run of the row
 // above, and of the previous frame's same row, that overlaps its span: each
 // up or previous-frame edge of the run's pixels ends in one of those runs.
-__global__ void __launch_bounds__(kThreads) lab_link(LabArgs a) {
+__device__ __forceinline__ void link_step(const LabArgs &a) {
   // the batch's frame segments, read once per block
   __shared__ uint64_t sh_start[kMaxSegments], sh_count[kMaxSegments];
   __shared__ int64_t sh_z[kMaxSegments];
@@ -651,7 +665,7 @@ __global__ void __launch_bounds__(kThreads) lab_link(LabArgs a) {
 // consecutive positions; each stretch of adjacent lanes with one root (a
 // run, mostly) makes one update. Positions are in (frame, index) order, so
 // a stretch's last frame is its last lane's.
-__global__ void __launch_bounds__(kThreads) lab_flatten(LabArgs a) {
+__device__ __forceinline__ void flatten_step(const LabArgs &a) {
   const uint64_t n = a.sc->n;
   const int lane = threadIdx.x & 31;
   const uint64_t warps = gstride() >> 5;
@@ -692,7 +706,7 @@ __global__ void __launch_bounds__(kThreads) lab_flatten(LabArgs a) {
 // hold none, few more than one), kThreads words a tile; a tile's place in
 // the list comes from the tiles before it. The last tile knows how many
 // there are.
-__global__ void __launch_bounds__(kThreads) lab_close(LabArgs a) {
+__device__ __forceinline__ void close_step(const LabArgs &a) {
   LabelScalars *sc = a.sc;
   const uint64_t nw = sc->nw;
   const uint64_t tiles = (nw + kThreads - 1) / kThreads;
@@ -719,7 +733,7 @@ __global__ void __launch_bounds__(kThreads) lab_close(LabArgs a) {
 
 // Per 32 consecutive roots of the list, how many close in each bucket, laid
 // out bucket-major (bucket s, group j at s * groups + j).
-__global__ void __launch_bounds__(kThreads) lab_count(LabArgs a) {
+__device__ __forceinline__ void count_step(const LabArgs &a) {
   const LabelScalars *sc = a.sc;
   const uint64_t closed = sc->closed, groups = (closed + 31) / 32;
   const int nseg = static_cast<int>(sc->nseg);
@@ -742,7 +756,7 @@ __global__ void __launch_bounds__(kThreads) lab_count(LabArgs a) {
 // Emission ranks; and for each component that passes the size filters a
 // place for its members and its spot, claimed a warp at a time: they are
 // scratch, so their order does not matter.
-__global__ void __launch_bounds__(kThreads) lab_rank(LabArgs a) {
+__device__ __forceinline__ void rank_step(const LabArgs &a) {
   LabelScalars *sc = a.sc;
   const uint64_t closed = sc->closed, groups = (closed + 31) / 32;
   const int lane = threadIdx.x & 31;
@@ -805,7 +819,7 @@ __global__ void __launch_bounds__(kThreads) lab_rank(LabArgs a) {
 // So each component's list is a set of runs, one per 32-position chunk it
 // has pixels in, each run ascending and within its chunk; lab_accept orders
 // the runs rather than the members.
-__global__ void __launch_bounds__(kThreads) lab_scatter(LabArgs a) {
+__device__ __forceinline__ void scatter_step(const LabArgs &a) {
   const uint64_t n = a.sc->n, nw = a.sc->nw;
   const int lane = threadIdx.x & 31;
   const uint64_t warps = gstride() >> 5;
@@ -1460,9 +1474,8 @@ __device__ bool spot_pass_warp(const DivU32 &W, double max_sep, const WarpBuffer
 template <uint32_t CAP> constexpr int kAcceptBlocks = CAP <= 256 ? 8 : CAP <= 512 ? 6 : 1;
 
 template <uint32_t CAP>
-__global__ void __launch_bounds__(kCompWarps * 32, kAcceptBlocks<CAP>)
-    lab_accept(LabArgs a, uint32_t lo, uint32_t hi, int list) {
-  extern __shared__ __align__(16) unsigned char comp_smem[];
+__device__ __forceinline__ void accept_step(const LabArgs &a, uint32_t lo, uint32_t hi, int list,
+                                            unsigned char *comp_smem) {
   LabelScalars *sc = a.sc;
   const uint64_t closed = list == 0 ? sc->closed : list == 1 ? sc->big_n : sc->mid_n;
   uint32_t *next = list == 0 ? &sc->accept_next : list == 1 ? &sc->big_next : &sc->mid_next;
@@ -1540,7 +1553,8 @@ __global__ void __launch_bounds__(kCompWarps * 32, kAcceptBlocks<CAP>)
 // The accepted spots to their rows and their pixels to the kept list, a warp
 // a spot: the row and the first kWriteWords * 32 words of the pixels read
 // together, before any is stored.
-__global__ void __launch_bounds__(kThreads) lab_write(LabArgs a) {
+template <bool kHead>
+__device__ __forceinline__ void write_step(const LabArgs &a) {
   LabelScalars *sc = a.sc;
   const uint64_t closed = sc->closed;
   const uint64_t kept_base = sc->kept_total;
@@ -1570,6 +1584,9 @@ __global__ void __launch_bounds__(kThreads) lab_write(LabArgs a) {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(a.pix_tmp + moff);
     uint32_t *dst = reinterpret_cast<uint32_t *>(a.kept + pix);
     const uint32_t words = 3 * n;
+    uint32_t *head = nullptr;
+    if (kHead && a.head && pix + n <= LabelHead::kPixels)
+      head = reinterpret_cast<uint32_t *>(a.head->pixels + pix);
     for (uint32_t w0 = lane; w0 < words; w0 += 32 * kWriteWords) {
       uint32_t v[kWriteWords];
 #pragma unroll
@@ -1578,11 +1595,17 @@ __global__ void __launch_bounds__(kThreads) lab_write(LabArgs a) {
           v[u] = src[w0 + 32 * u];
 #pragma unroll
       for (uint32_t u = 0; u < kWriteWords; u++)
-        if (w0 + 32 * u < words)
+        if (w0 + 32 * u < words) {
           dst[w0 + 32 * u] = v[u];
+          if (kHead && head)
+            head[w0 + 32 * u] = v[u];
+        }
     }
-    if (lane < 13)
+    if (lane < 13) {
       reinterpret_cast<uint64_t *>(a.spots + row)[lane] = word;
+      if (kHead && a.head && row < LabelHead::kSpots)
+        reinterpret_cast<uint64_t *>(a.head->spots + row)[lane] = word;
+    }
   }
 }
 
@@ -1621,7 +1644,7 @@ __device__ void close_books(const LabArgs &a) {
 // other blocks read, and their copy in host memory, which the host then has
 // as soon as the stream has passed (a copy of its own, and a second wait, cost
 // every reader 14 us).
-__global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
+__device__ __forceinline__ void carry_step(const LabArgs &a) {
   LabelScalars *sc = a.sc;
   const uint64_t nw = sc->nw;
   const int lane = threadIdx.x & 31;
@@ -1640,6 +1663,87 @@ __global__ void __launch_bounds__(kThreads) lab_carry(LabArgs a) {
     a.nval[at] = a.val[g];
     a.npar[at] = open_position(a, r); // the root is open too, and comes first
   }
+}
+
+// ---- the steps as launches of their own ------------------------------------
+
+__global__ void __launch_bounds__(kThreads) lab_setup(const __grid_constant__ LabArgs a) {
+  setup_step(a);
+}
+template <int kGatherWords>
+__global__ void __launch_bounds__(kThreads) lab_gather(const __grid_constant__ LabArgs a) {
+  gather_step<kGatherWords>(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_link(const __grid_constant__ LabArgs a) {
+  link_step(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_flatten(const __grid_constant__ LabArgs a) {
+  flatten_step(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_close(const __grid_constant__ LabArgs a) {
+  close_step(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_count(const __grid_constant__ LabArgs a) {
+  count_step(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_rank(const __grid_constant__ LabArgs a) {
+  rank_step(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_scatter(const __grid_constant__ LabArgs a) {
+  scatter_step(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_write(const __grid_constant__ LabArgs a) {
+  write_step<false>(a);
+}
+__global__ void __launch_bounds__(kThreads) lab_carry(const __grid_constant__ LabArgs a) {
+  carry_step(a);
+}
+template <uint32_t CAP>
+__global__ void __launch_bounds__(kCompWarps * 32, kAcceptBlocks<CAP>)
+    lab_accept(const __grid_constant__ LabArgs a, uint32_t lo, uint32_t hi, int list) {
+  extern __shared__ __align__(16) unsigned char comp_smem[];
+  accept_step<CAP>(a, lo, hi, list, comp_smem);
+}
+
+// ---- the same by one block, for small batches ------------------------------
+// All the steps before the spot pass, and all after it: three launches a
+// batch for sixteen, which the host's enqueueing bounds (4 us a launch) where
+// a step has less than a pixel a thread to do. Nothing here is shared between
+// blocks, so a __syncthreads() does what a launch's end does. 27 to 34 us and
+// 9 us for 1.3 k pixels of a 256 x 384 frame, bound by the chains of dependent
+// loads of ten steps; a series of 12 such frames, from their images, 3.5 -> 2.5 ms.
+
+__global__ void __launch_bounds__(kThreads, 1) lab_small_open(const __grid_constant__ LabArgs a) {
+  LabelScalars *sc = a.sc;
+  setup_step(a);
+  __syncthreads();
+  gather_step<1>(a);
+  __syncthreads();
+  link_step(a);
+  __syncthreads();
+  flatten_step(a);
+  __syncthreads();
+  close_step(a);
+  __syncthreads();
+  count_step(a);
+  __syncthreads();
+  scan_tiles<uint32_t>(a.bcnt, sc->seg_len, nullptr, &sc->count_next, a.count_st, &sc->status);
+  __syncthreads();
+  rank_step(a);
+  __syncthreads();
+  scatter_step(a);
+  __syncthreads();
+  scan_tiles<uint32_t>(a.ocnt, sc->nw, &sc->open32, &sc->open_next, a.open_st, &sc->status);
+}
+
+__global__ void __launch_bounds__(kThreads, 1) lab_small_close(const __grid_constant__ LabArgs a) {
+  LabelScalars *sc = a.sc;
+  scan_tiles<uint64_t>(a.pack, sc->closed, &sc->accepted_pack, &sc->pack_next, a.pack_st,
+                       &sc->status);
+  __syncthreads();
+  write_step<true>(a);
+  __syncthreads();
+  carry_step(a);
 }
 
 } // namespace
@@ -1664,13 +1768,21 @@ DeviceLabeller::DeviceLabeller(int height, int width, const GroupOptions &option
                              static_cast<int>(kCompWarps * warp_comp_bytes<kCompCap>())),
         "cudaFuncSetAttribute");
   grid_ = static_cast<unsigned>(device_sm_count() * 8);
-  check(cudaMallocHost(&z_stage_, sizeof(int64_t)), "cudaMallocHost");
-  aux_ = create_stream(2);
-  aux2_ = create_stream(2);
-  check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
-  check(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming), "cudaEventCreate");
-  check(cudaEventCreateWithFlags(&join2_, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaStreamSynchronize(cudaStreamLegacy), "clearing labeller scalars");
+}
+
+// The streams beside the caller's, which only batches of more than kSmallPixels
+// need.
+void DeviceLabeller::create_streams() {
+  if (join2_)
+    return;
+  if (!aux_)
+    aux_ = create_stream(2);
+  if (!aux2_)
+    aux2_ = create_stream(2);
+  for (cudaEvent_t *e : {&fork_, &join_, &join2_})
+    if (!*e)
+      check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
 }
 
 DeviceLabeller::~DeviceLabeller() {
@@ -1738,6 +1850,8 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
     check(cudaMemcpy(val.data(), c.value, host.carry_n * 4, cudaMemcpyDeviceToHost), "carry");
     check(cudaMemcpy(par.data(), c.parent, host.carry_n * 4, cudaMemcpyDeviceToHost), "carry");
   }
+  if (!room)
+    create_streams();
   release();
   batch_cap_ = carry_cap_ = live_cap_ = spot_cap_ = 0;
   frame_cap_ = 0;
@@ -1832,6 +1946,8 @@ bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
 }
 
 void DeviceLabeller::set_next_frame(int64_t z, cudaStream_t s) {
+  if (!z_stage_)
+    check(cudaMallocHost(&z_stage_, sizeof(int64_t)), "cudaMallocHost");
   check(cudaStreamSynchronize(s), "cudaStreamSynchronize"); // the staging word is reused
   *z_stage_ = z;
   check(cudaMemcpyAsync(&sc_->batch_z0, z_stage_, sizeof(int64_t), cudaMemcpyHostToDevice, s),
@@ -1840,8 +1956,43 @@ void DeviceLabeller::set_next_frame(int64_t z, cudaStream_t s) {
 
 void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64_t *offs,
                              const uint32_t *counts, const int32_t *count_map,
-                             const uint32_t *caps, bool close_all,
-                             cudaStream_t s) {
+                             const uint32_t *caps, bool close_all, cudaStream_t s) {
+  Batch b;
+  b.nframes = nframes;
+  b.lists = lists;
+  b.offs = offs;
+  b.counts = counts;
+  b.count_map = count_map;
+  b.caps = caps;
+  b.close_all = close_all;
+  b.most = live_cap_;
+  enqueue_batch(b, s);
+}
+
+bool DeviceLabeller::takes_head(uint64_t pixels) { return pixels <= kSmallPixels; }
+
+void DeviceLabeller::enqueue_frame(int64_t z, const SignalPixel *list, uint32_t count,
+                                   uint64_t carried, cudaStream_t s) {
+  if (count > batch_cap_)
+    throw std::invalid_argument("more pixels than the labeller was sized for");
+  Batch b;
+  b.nframes = 1;
+  b.lists = list;
+  b.one_count = count;
+  b.one_z = z;
+  b.most = carried + count;
+  enqueue_batch(b, s);
+}
+
+void DeviceLabeller::enqueue_rest(uint64_t carried, cudaStream_t s) {
+  Batch b;
+  b.close_all = true;
+  b.most = carried;
+  enqueue_batch(b, s);
+}
+
+void DeviceLabeller::enqueue_batch(const Batch &b, cudaStream_t s) {
+  const int nframes = b.nframes;
   if (nframes > frame_cap_)
     throw std::invalid_argument("more frames than the labeller was sized for");
   if (live_cap_ == 0)
@@ -1850,18 +2001,20 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   a.width = width_;
   a.wdiv = DivU32::of(static_cast<uint32_t>(width_));
   a.nframes = nframes;
-  a.close_all = close_all ? 1 : 0;
+  a.close_all = b.close_all ? 1 : 0;
   a.two_d = opt_.two_d ? 1 : 0;
   a.min_size = opt_.min_spot_size;
   a.max_size = opt_.max_spot_size;
   a.max_sep = opt_.max_separation;
   a.live_cap = live_cap_;
   a.spot_cap = spot_cap_;
-  a.lists = lists;
-  a.offs = offs;
-  a.counts = counts;
-  a.count_map = count_map;
-  a.caps = caps;
+  a.lists = b.lists;
+  a.offs = b.offs ? b.offs : &sc_->zero;
+  a.counts = b.counts;
+  a.count_map = b.count_map;
+  a.caps = b.caps;
+  a.one_count = b.one_count;
+  a.one_z = b.one_z;
   const Live &cur = live_[cur_];
   const Live &nxt = live_[cur_ ^ 1];
   a.fr = cur.frame;
@@ -1904,7 +2057,18 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   a.nblk = nblk_;
   a.sc = sc_;
   a.report = report_;
+  a.head = head_;
 
+  if (b.most <= kSmallPixels) {
+    lab_small_open<<<1, kThreads, 0, s>>>(a);
+    lab_accept<kCompCap><<<grid_ / 8, kCompWarps * 32, kCompWarps * warp_comp_bytes<kCompCap>(),
+                           s>>>(a, 0u, 0xffffffffu, 0);
+    lab_small_close<<<1, kThreads, 0, s>>>(a);
+    check(cudaGetLastError(), "launching the labeller");
+    cur_ ^= 1;
+    return;
+  }
+  create_streams();
   const unsigned grid = grid_;
   LabelScalars *sc = sc_;
   lab_setup<<<grid, kThreads, 0, s>>>(a);

@@ -69,6 +69,7 @@ struct LabelScalars {
   uint64_t kept_total; // pixels of accepted spots so far (Spot::first base)
   int32_t status;      // nonzero: a capacity was exceeded
   int32_t pad1;
+  uint64_t zero; // the offset of a batch's only list
 };
 
 enum : int32_t {
@@ -76,6 +77,16 @@ enum : int32_t {
   kLabelLiveOverflow = 1,
   kLabelSpotOverflow = 2,
   kLabelWaitTimeout = 3, // a tile's wait for the tiles before it gave up
+};
+
+// Page-locked host memory in which a small batch leaves its results, so that
+// the host has them with its scalars, without copies of their own (two of them
+// and a second wait were 30 us of each frame added). As far as they fit here:
+// much more than a frame of a few thousand pixels finishes, and little to lock.
+struct LabelHead {
+  static constexpr uint64_t kSpots = 128, kPixels = 1536;
+  Spot spots[kSpots];
+  Pixel pixels[kPixels];
 };
 
 // What a component's root holds, in one 16-byte word at its position.
@@ -113,6 +124,17 @@ public:
                const uint32_t *counts, const int32_t *count_map, const uint32_t *caps,
                bool close_all, cudaStream_t s);
 
+  // The same for one frame, number z, of `count` records at `list`, where the
+  // caller knows how many pixels the last batch left (`carried`); nothing but
+  // the list is read from device memory.
+  void enqueue_frame(int64_t z, const SignalPixel *list, uint32_t count, uint64_t carried,
+                     cudaStream_t s);
+  // ... and for finishing what is left.
+  void enqueue_rest(uint64_t carried, cudaStream_t s);
+  // Whether those two, with `pixels` carried and added, leave the batch's spots
+  // and pixels in the head that head_to() gave, as far as they fit there.
+  static bool takes_head(uint64_t pixels);
+
   // Sets batch_z0 for the next enqueue (an asynchronous copy from pinned
   // host memory; the labeller keeps the staging word until the next call).
   void set_next_frame(int64_t z, cudaStream_t s);
@@ -127,6 +149,7 @@ public:
   // Page-locked host memory that each batch leaves a copy of the scalars in
   // (there once its stream has passed); set before the first one.
   void report_to(LabelScalars *host) { report_ = host; }
+  void head_to(LabelHead *host) { head_ = host; }
   Spot *batch_spots() const { return spots_out_; }
   Pixel *batch_pixels() const { return kept_out_; }
   uint64_t spot_capacity() const { return spot_cap_; }
@@ -137,6 +160,20 @@ public:
   const GroupOptions &options() const { return opt_; }
 
 private:
+  struct Batch {
+    int nframes = 0;
+    const SignalPixel *lists = nullptr;
+    const uint64_t *offs = nullptr;
+    const uint32_t *counts = nullptr;
+    const int32_t *count_map = nullptr;
+    const uint32_t *caps = nullptr;
+    uint32_t one_count = 0; // without counts: of the only frame
+    int64_t one_z = 0;      // and its number
+    bool close_all = false;
+    uint64_t most = 0; // pixels, carried ones too, that it can hold
+  };
+  void enqueue_batch(const Batch &b, cudaStream_t s);
+  void create_streams();
   void release();
   bool allocate(uint64_t batch_pixels, int frames, uint64_t carry_pixels);
 
@@ -182,6 +219,7 @@ private:
   unsigned grid_ = 0;
   LabelScalars *sc_ = nullptr;
   LabelScalars *report_ = nullptr;
+  LabelHead *head_ = nullptr;
   cudaStream_t aux_ = nullptr;  // the large components' spot pass
   cudaStream_t aux2_ = nullptr; // the middle-sized components' spot pass
   cudaEvent_t fork_ = nullptr, join_ = nullptr, join2_ = nullptr;
