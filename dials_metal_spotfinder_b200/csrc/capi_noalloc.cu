@@ -82,9 +82,9 @@ Layout plan_layout(uint64_t height, uint64_t width) {
   L.max_blocks = device_sm_count() * std::min(occ, kBlocksPerSm);
   const uint64_t resident = static_cast<uint64_t>(L.max_blocks) * kWarpsPerBlock;
 
-  const uint64_t strips = (width + kStripOut - 1) / kStripOut;
+  const uint64_t strips = (width + strip_out(2) - 1) / strip_out(2);
   // 232 output columns per 256-column strip; rows start on 128-byte lines
-  L.pitch = align_up(strips * kStripOut + (kStripCols - kStripOut), 64);
+  L.pitch = align_up(strips * strip_out(2) + (strip_cols(2) - strip_out(2)), 64);
   L.rows = height + 2 * kMarginRows;
 
   // Output rows per task: fewest waves x (rows + 20 rows of halo).

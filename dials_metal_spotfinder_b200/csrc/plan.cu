@@ -56,8 +56,8 @@ uint64_t round_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 // 35 -> 27 us (4 rows).
 constexpr uint64_t kRowBase = 5, kRowLeast = 12;
 constexpr int kMinSeg = 4;
-int choose_seg_rows(const std::vector<ThresholdPlan::Shape> &shapes, uint64_t sms, int wpc,
-                    int blocks_per_sm) {
+int choose_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, uint64_t sms,
+                    int wpc, int blocks_per_sm) {
   int max_h = 1;
   for (const auto &s : shapes)
     max_h = std::max(max_h, s.height);
@@ -66,7 +66,7 @@ int choose_seg_rows(const std::vector<ThresholdPlan::Shape> &shapes, uint64_t sm
   for (int seg = std::min(kMinSeg, max_h); seg <= max_h; seg++) {
     uint64_t tasks = 0;
     for (const auto &s : shapes) {
-      const uint64_t strips = (s.width + kStripOut - 1) / kStripOut;
+      const uint64_t strips = (s.width + strip_out(elem_bytes) - 1) / strip_out(elem_bytes);
       tasks += strips * ((s.height + seg - 1) / seg);
     }
     const uint64_t per_block = static_cast<uint64_t>(wpc);
@@ -95,14 +95,14 @@ int model_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shap
     throw DeviceError("the threshold kernel does not fit on this device");
   if (blocks_per_sm > 0)
     occ = std::min(occ, blocks_per_sm);
-  return choose_seg_rows(shapes, static_cast<uint64_t>(device_sm_count()), wpc, occ);
+  return choose_seg_rows(elem_bytes, shapes, static_cast<uint64_t>(device_sm_count()), wpc, occ);
 }
 
 void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes, uint64_t pitch_elems,
                       uint64_t rows) {
   const cuuint64_t dims[2] = {pitch_elems, rows};
   const cuuint64_t strides[1] = {pitch_elems * static_cast<uint64_t>(elem_bytes)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kStripCols),
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(strip_cols(elem_bytes)),
                              static_cast<cuuint32_t>(kBoxRows)};
   const cuuint32_t estride[2] = {1, 1};
   const CUtensorMapDataType dt =
@@ -141,25 +141,27 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     throw std::invalid_argument("a plan needs at least one frame");
   if (slots < 1)
     throw std::invalid_argument("a plan needs at least one slot");
-  // 16-bit pixels: 7 two-warp blocks per SM; 32-bit: each warp's shared
-  // memory is twice the size, so one-warp blocks fill the SM best
+  // eight two-warp blocks an SM
   if (tuning_.warps_per_block == 0)
-    tuning_.warps_per_block = elem_bytes == 2 ? 2 : 1;
+    tuning_.warps_per_block = 2;
   const int wpc = tuning_.warps_per_block;
   if (wpc != 1 && wpc != 2 && wpc != 4)
     throw std::invalid_argument("warps_per_block must be 1, 2 or 4");
 
+  const int out_cols = strip_out(elem_bytes);
   int32_t max_strips = 0;
   for (const Shape &s : shapes) {
     if (s.height < 1 || s.width < 1)
       throw std::invalid_argument("frame with no pixels");
     if (static_cast<uint64_t>(s.height) * s.width > 0x7fffffffull)
       throw std::invalid_argument("frame larger than INT32_MAX pixels");
-    max_strips = std::max(max_strips, (s.width + kStripOut - 1) / kStripOut);
+    max_strips = std::max(max_strips, (s.width + out_cols - 1) / out_cols);
   }
-  // Every strip reads 256 columns from a multiple of 232; the pitch is a
-  // multiple of 128 bytes so each arena row starts on a TMA-friendly line.
-  pitch_ = round_up(static_cast<uint64_t>(max_strips) * kStripOut + (kStripCols - kStripOut),
+  // Every strip reads its columns from a multiple of its output columns; the
+  // pitch is a multiple of 128 bytes so each arena row starts on a TMA-friendly
+  // line.
+  pitch_ = round_up(static_cast<uint64_t>(max_strips) * out_cols +
+                        (strip_cols(elem_bytes) - out_cols),
                     128 / elem_bytes);
 
   const int occ = elem_bytes == 2 ? threshold_occupancy<uint16_t>(wpc)
@@ -170,7 +172,7 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
   sms_ = device_sm_count();
   max_blocks_ = sms_ * per_sm;
   if (tuning_.seg_rows <= 0)
-    tuning_.seg_rows = choose_seg_rows(shapes, static_cast<uint64_t>(sms_), wpc, per_sm);
+    tuning_.seg_rows = choose_seg_rows(elem_bytes, shapes, static_cast<uint64_t>(sms_), wpc, per_sm);
 
   uint64_t row = 0, tile = 0, out = 0;
   uint32_t task = 0;
@@ -180,7 +182,7 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     d.row0 = static_cast<int64_t>(row + kMarginRows);
     d.height = s.height;
     d.width = s.width;
-    d.strips = (s.width + kStripOut - 1) / kStripOut;
+    d.strips = (s.width + out_cols - 1) / out_cols;
     d.seg_rows = std::min(tuning_.seg_rows, s.height);
     d.segments = (s.height + d.seg_rows - 1) / d.seg_rows;
     d.task_begin = task;

@@ -21,15 +21,29 @@ struct SignalPixel {
 };
 static_assert(sizeof(SignalPixel) == 16, "SignalPixel must be 16 bytes");
 
-// Geometry of the streaming threshold. A warp owns a strip of 256 pixel
-// columns (8 per lane); the outer 10 on each side are halo, 4 more on the
-// right are padding, so a strip produces 232 output columns. Strips start at
-// multiples of 232 elements in a buffer whose frame sits 10 columns in from
-// the left, which keeps every strip's first column 16-byte aligned for TMA.
-constexpr int kLaneCols = 8;
-constexpr int kStripCols = 32 * kLaneCols; // 256
+// Geometry of the streaming threshold. A warp owns a strip of pixel columns;
+// the outer 10 on each side are halo. Strips start at multiples of their
+// output columns in a buffer whose frame sits 10 columns in from the left, and
+// those are a multiple of 16 bytes, which keeps every strip's first column
+// aligned for TMA.
 constexpr int kHalo = 10;                  // 3 (7x7) + 2 (5x5) + 5 (11x11)
-constexpr int kStripOut = 232;             // outputs per strip
+template <typename T> struct Strip;
+template <> struct Strip<uint16_t> {
+  static constexpr int kLane = 8;          // columns a lane
+  static constexpr int kCols = 32 * kLane; // 256
+  static constexpr int kOut = 232;         // output columns; 4 more are padding
+};
+template <> struct Strip<uint32_t> {
+  static constexpr int kLane = 4;
+  static constexpr int kCols = 32 * kLane; // 128
+  static constexpr int kOut = 108;
+};
+constexpr int strip_cols(int elem_bytes) {
+  return elem_bytes == 2 ? Strip<uint16_t>::kCols : Strip<uint32_t>::kCols;
+}
+constexpr int strip_out(int elem_bytes) {
+  return elem_bytes == 2 ? Strip<uint16_t>::kOut : Strip<uint32_t>::kOut;
+}
 constexpr int kMarginLeft = kHalo;         // frame column 0 at buffer column 10
 constexpr int kMarginRows = kHalo;         // rows of fill above and below
 constexpr int kRingRows = 20;              // rows of a strip held in smem
@@ -39,7 +53,7 @@ constexpr uint32_t kChunkRecords = 1024;   // staging pool allocation unit
 // The most records a warp stages at once (two output rows of a strip); a
 // staging chunk is abandoned when that many might not fit, so each chunk
 // wastes fewer than this.
-constexpr uint32_t kMaxStaged = 2 * kStripOut;
+constexpr uint32_t kMaxStaged = 2 * Strip<uint16_t>::kOut;
 
 // Limits of the word in which the threshold's warps share a task's rows (row
 // numbers of kSharedRowBits bits, task numbers of the 22 bits above two): plans
@@ -62,7 +76,6 @@ template <> struct Traits<uint16_t> {
   static constexpr uint32_t kMasked = 0xfffeu; // pixels >= this are masked
   static constexpr int kShift7 = 22;  // 49 * 65533 < 2^22, count <= 49 < 2^6
   static constexpr int kShift11 = 23; // 121 * 65533 < 2^23, count <= 121 < 2^7
-  static constexpr int kRowVecs = 1;  // uint4 loads per lane per row
 };
 
 template <> struct Traits<uint32_t> {
@@ -70,7 +83,6 @@ template <> struct Traits<uint32_t> {
   static constexpr uint32_t kMasked = 0xfffffffeu;
   static constexpr int kShift7 = 40;  // 49 * 2^32 < 2^40
   static constexpr int kShift11 = 40; // 121 * 2^32 < 2^40, count < 2^7
-  static constexpr int kRowVecs = 2;
 };
 
 // One frame of a batch as the device sees it. The arena is a single pitched
@@ -83,7 +95,7 @@ struct FrameDesc {
   int64_t row0;         // arena row of frame row 0
   int32_t height;
   int32_t width;
-  int32_t strips;       // ceil(width / kStripOut)
+  int32_t strips;       // ceil(width / strip_out())
   int32_t segments;     // ceil(height / seg_rows)
   int32_t seg_rows;     // output rows per task
   uint32_t task_begin;  // first task of this frame

@@ -2,14 +2,15 @@
 // reference (dispersion test, erode, masked background, Poisson test, emit),
 // as one streaming kernel per batch of frames.
 //
-// Decomposition. A task is one strip of 256 buffer columns (232 output
-// columns plus halo) by one segment of output rows of one frame. A warp owns
+// Decomposition. A task is one strip of buffer columns (256 of 16-bit pixels,
+// of which 232 are output and the rest halo; 128 of 32-bit ones, 108 output) by
+// one segment of output rows of one frame. A warp owns
 // a task at a time and walks down it row by row; one that has nothing left
 // takes rows from another's task (see pack_range), but none waits for
 // another. Each warp has a ring of 20 rows of its strip in shared memory, fed
 // 2 rows at a time by TMA (one elected lane issues, an mbarrier per stage).
 //
-// Per input row r entering at the bottom of the ring, each lane (8 columns)
+// Per input row r entering at the bottom of the ring, each lane (8 or 4 columns)
 // updates, all in registers:
 //   - vertical 7-row running sums of the valid count+sum (packed) and of the
 //     sum of squares, from rows r and r-7;
@@ -17,7 +18,7 @@
 //     for the 3 neighbour columns each side), and the dispersion test there
 //     -> one bit per pixel (masked pixels are 1, src/dext.cc:113);
 //   - the 5 x 5 erode at row r-5 on those bits (vertical AND of five
-//     8-bit rows, then horizontal AND with 2 shuffled neighbour bits);
+//     rows' bits, then horizontal AND with 2 shuffled neighbour bits);
 //   - vertical 11-row running sums of the count+sum of pixels that are valid
 //     and not kept by the erode, from rows r-5 and r-16;
 //   - at row r-10, for the pixels that are candidates (value > 0 and kept
@@ -38,6 +39,13 @@
 // after it, one masked test a pair of rows (956 -> 897 us for 16 frames). Not
 // kept: high halves by a high multiply (927), and additions as multiply-adds
 // in the vertical (926) or the horizontal sums (910), which cost two each.
+// 32-bit pixels: 8 columns a lane take 220 registers, which leaves an SM 8
+// warps, too few to hide the latency of their 64-bit sums and doubles (each
+// scheduler issued 0.54 a cycle); 4 columns a lane fit 16 warps, and though
+// their rows cost 24 % more instructions, 8 frames of 4362 x 4148 uint32 take
+// 878 us where they took 976 (1.3 TB/s of their own bytes), one of 1062 x 1028
+// 38 where it took 45. Not kept: doubles from integers by exponent bits and an
+// addition (905).
 //
 // Cost. The running sums are updated as if every pixel entering and leaving
 // were valid -- then the packed counts cancel and an update is one add of
@@ -174,13 +182,14 @@ __device__ __forceinline__ uint32_t dispersion_bits49(const uint32_t (&hs)[8],
   return bits;
 }
 
-// The same with R = double, for 32-bit pixels (count << 40 | sum).
-__device__ __forceinline__ uint32_t dispersion_bits(const uint64_t (&hs)[8],
-                                                    const uint64_t (&hq)[8],
+// The same with R = double, for the 4 columns of a lane of 32-bit pixels
+// (count << 40 | sum).
+__device__ __forceinline__ uint32_t dispersion_bits(const uint64_t (&hs)[4],
+                                                    const uint64_t (&hq)[4],
                                                     const double *sq) {
   uint32_t bits = 0;
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < 4; k++) {
     const uint32_t m = static_cast<uint32_t>(hs[k] >> 40);
     const double md = __uint2double_rn(m);
     const double sd = __ull2double_rn(hs[k] & ((1ull << 40) - 1));
@@ -214,7 +223,7 @@ __device__ __forceinline__ bool poisson(uint32_t p, uint64_t m, uint64_t s,
 // Row access
 // --------------------------------------------------------------------------
 
-// The lane's 8 pixels of one ring row, and whether any is masked.
+// The lane's pixels of one ring row, and whether any is masked.
 template <typename T> struct LaneRow;
 
 template <> struct LaneRow<uint16_t> {
@@ -251,30 +260,28 @@ template <> struct LaneRow<uint16_t> {
 };
 
 template <> struct LaneRow<uint32_t> {
-  uint4 a, b;
+  uint4 v;
   __device__ __forceinline__ void load(const uint32_t *row, int lane) {
-    const uint4 *v = reinterpret_cast<const uint4 *>(row + 8 * lane);
-    a = v[0];
-    b = v[1];
+    v = reinterpret_cast<const uint4 *>(row)[lane];
   }
-  __device__ __forceinline__ void unpack(uint32_t (&p)[8], uint32_t) const {
-    p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w;
-    p[4] = b.x; p[5] = b.y; p[6] = b.z; p[7] = b.w;
+  __device__ __forceinline__ void unpack(uint32_t (&p)[4], uint32_t) const {
+    p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
   }
   __device__ __forceinline__ uint32_t masked_bits() const {
     const uint32_t m = Traits<uint32_t>::kMasked;
-    return (a.x >= m ? 1u : 0u) | (a.y >= m ? 2u : 0u) | (a.z >= m ? 4u : 0u) |
-           (a.w >= m ? 8u : 0u) | (b.x >= m ? 16u : 0u) | (b.y >= m ? 32u : 0u) |
-           (b.z >= m ? 64u : 0u) | (b.w >= m ? 128u : 0u);
+    return (v.x >= m ? 1u : 0u) | (v.y >= m ? 2u : 0u) | (v.z >= m ? 4u : 0u) |
+           (v.w >= m ? 8u : 0u);
   }
   static __device__ __forceinline__ bool any_masked(const LaneRow &r, const LaneRow &s) {
-    return (r.masked_bits() | s.masked_bits()) != 0;
+    const uint32_t m = max(max(max(r.v.x, r.v.y), max(r.v.z, r.v.w)),
+                           max(max(s.v.x, s.v.y), max(s.v.z, s.v.w)));
+    return m >= Traits<uint32_t>::kMasked;
   }
 };
 
 template <typename T>
-__device__ __forceinline__ void load_pixels(const T *row, int lane, uint32_t (&p)[8],
-                                            uint32_t down) {
+__device__ __forceinline__ void load_pixels(const T *row, int lane,
+                                            uint32_t (&p)[Strip<T>::kLane], uint32_t down) {
   LaneRow<T> r;
   r.load(row, lane);
   r.unpack(p, down);
@@ -293,28 +300,29 @@ __device__ __forceinline__ uint64_t shfl_down(uint64_t v) {
   return (static_cast<uint64_t>(hi) << 32) | lo;
 }
 
-// Horizontal sums of width 2R+1 over the lane's 8 columns, given the lane's
+// Horizontal sums of width 2R+1 over the lane's C columns, given the lane's
 // own vertical sums v[0..8) and the neighbouring lanes' by shuffle. The edge
 // lanes see no neighbour; their edge columns are halo and never used.
-template <int R, typename A>
-__device__ __forceinline__ void hsum(const A (&v)[8], A (&h)[8], A from = 0) {
-  A e[8 + 2 * R];
+template <int R, int C, typename A>
+__device__ __forceinline__ void hsum(const A (&v)[C], A (&h)[C], A from = 0) {
+  static_assert(R <= C, "a window reaches the next lane at most");
+  A e[C + 2 * R];
 #pragma unroll
   for (int i = 0; i < R; i++)
-    e[i] = shfl_up(v[8 - R + i]);
+    e[i] = shfl_up(v[C - R + i]);
 #pragma unroll
-  for (int i = 0; i < 8; i++)
+  for (int i = 0; i < C; i++)
     e[R + i] = v[i];
 #pragma unroll
   for (int i = 0; i < R; i++)
-    e[R + 8 + i] = shfl_down(v[i]);
+    e[R + C + i] = shfl_down(v[i]);
   A run = from;
 #pragma unroll
   for (int i = 0; i < 2 * R + 1; i++)
     run += e[i];
   h[0] = run;
 #pragma unroll
-  for (int k = 1; k < 8; k++) {
+  for (int k = 1; k < C; k++) {
     run += e[k + 2 * R] - e[k - 1];
     h[k] = run;
   }
@@ -326,29 +334,31 @@ __device__ __forceinline__ void hsum(const A (&v)[8], A (&h)[8], A from = 0) {
 // bit is in `ng`, is changed to take its count back and add nothing.
 template <typename T> using GroundWord = typename Traits<T>::Acc;
 template <typename T>
-__device__ __forceinline__ void load_ground(const T *row, int lane, GroundWord<T> (&g)[8],
-                                            uint32_t down) {
-  uint32_t p[8];
+__device__ __forceinline__ void load_ground(const T *row, int lane,
+                                            GroundWord<T> (&g)[Strip<T>::kLane], uint32_t down) {
+  uint32_t p[Strip<T>::kLane];
   load_pixels<T>(row, lane, p, down);
 #pragma unroll
-  for (int k = 0; k < 8; k++)
+  for (int k = 0; k < Strip<T>::kLane; k++)
     g[k] = p[k];
 }
 template <typename T>
-__device__ __forceinline__ void only_ground(GroundWord<T> (&in)[8], GroundWord<T> (&out)[8],
+__device__ __forceinline__ void only_ground(GroundWord<T> (&in)[Strip<T>::kLane],
+                                            GroundWord<T> (&out)[Strip<T>::kLane],
                                             uint32_t ng_in, uint32_t ng_out) {
   constexpr GroundWord<T> kNot = GroundWord<T>(0) - (GroundWord<T>(1) << Traits<T>::kShift11);
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < Strip<T>::kLane; k++) {
     in[k] = (ng_in >> k) & 1u ? kNot : in[k];
     out[k] = (ng_out >> k) & 1u ? kNot : out[k];
   }
 }
 template <typename T>
-__device__ __forceinline__ void add_rows(GroundWord<T> (&sum)[8], const GroundWord<T> (&in)[8],
-                                         const GroundWord<T> (&out)[8]) {
+__device__ __forceinline__ void add_rows(GroundWord<T> (&sum)[Strip<T>::kLane],
+                                         const GroundWord<T> (&in)[Strip<T>::kLane],
+                                         const GroundWord<T> (&out)[Strip<T>::kLane]) {
 #pragma unroll
-  for (int k = 0; k < 8; k++)
+  for (int k = 0; k < Strip<T>::kLane; k++)
     sum[k] += in[k] - out[k];
 }
 
@@ -396,7 +406,7 @@ __device__ __forceinline__ int find_frame(const FrameDesc *frames, int n,
 // some, strips differ in masked columns and candidates): without this, 12.9
 // of the 16 warps an SM holds were active on average, and 16 frames of
 // 4362 x 4148 uint16 took 1104 us (958 with it), 16 of 2162 x 2068 327 (304),
-// 8 of 4362 x 4148 uint32 1103 (995). Halves down to kLeastShare rows are
+// 8 of 4362 x 4148 uint32, then 8 warps an SM, 1103 (995). Halves down to kLeastShare rows are
 // worth the 20 rows of halo they cost again: at least 64 gave 976 and 329
 // us, 24 the same as 32; claims of 8 rows the same as of 16.
 constexpr uint32_t kQuantum = 16;
@@ -476,10 +486,9 @@ __device__ __forceinline__ int back_slot(int slot, int back) {
   return s < 0 ? s + kRingRows : s;
 }
 
-// Warps per SM the registers allow: 16 for 16-bit pixels, 8 for 32-bit
-// (whose ring and 11-row sums, 24 KB a warp, also fill the shared memory;
-// 16-bit pixels take 12.1 KB a warp).
-template <typename T> constexpr int kWarpsPerSm = sizeof(T) == 2 ? 16 : 8;
+// Warps per SM the registers allow (their rings and 11-row sums take 12.1 KB a
+// warp).
+constexpr int kWarpsPerSm = 16;
 
 // The rows before a task's first are read as zeros: 16 rows, the farthest
 // back any row's sums reach (the 11-row window's leaving row, 16 above).
@@ -494,30 +503,32 @@ static_assert(kQuantum % 2 == 0 && kQuantum / kBoxRows >= 2, "claims go in pairs
 // Per-warp shared memory (the square-root table is static).
 template <typename T> struct WarpSmem {
   using A = typename Traits<T>::Acc;
-  static constexpr uint32_t kRing = kStripCols * sizeof(T) * kRingRows;
-  static constexpr uint32_t kWin = 2 * kStripCols * sizeof(A);
+  static constexpr uint32_t kRing = Strip<T>::kCols * sizeof(T) * kRingRows;
+  static constexpr uint32_t kWin = 2 * Strip<T>::kCols * sizeof(A);
   static constexpr uint32_t kBars = kRingStages * sizeof(uint64_t);
   static constexpr uint32_t kTotal = kRing + kWin + kBars;
 };
 
 template <typename T, int WPC>
-__global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsPerSm<T> / WPC : 1)
+__global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     threshold_kernel(const __grid_constant__ CUtensorMap arena, ThresholdArgs args) {
   using Tr = Traits<T>;
+  constexpr int C = Strip<T>::kLane;
+  constexpr uint32_t kLaneBits = (1u << C) - 1; // a bit a column
   using A = typename Tr::Acc;
   using Rl = typename Real<T>::type;
   using Sm = WarpSmem<T>;
-  constexpr uint32_t kRowBytes = kStripCols * sizeof(T);
+  constexpr uint32_t kRowBytes = Strip<T>::kCols * sizeof(T);
   constexpr uint32_t kBoxBytes = kRowBytes * kBoxRows;
   constexpr A C7 = A(1) << Tr::kShift7;   // one valid pixel's count in a 7 x 7 sum
   constexpr A C11 = A(1) << Tr::kShift11; // ... in an 11 x 11 sum
-  constexpr int kVecs = kStripCols * sizeof(T) / (32 * 16); // 16-byte words per lane per row
+  constexpr int kVecs = Strip<T>::kCols * sizeof(T) / (32 * 16); // 16-byte words per lane per row
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ Rl sqrt_tab[64];
-  // for each 8-bit mask, the positions of its set bits in ascending order,
-  // four bits each
-  __shared__ uint32_t bit_pos[256];
+  // for each mask of a lane's columns, the positions of its set bits in
+  // ascending order, four bits each
+  __shared__ uint32_t bit_pos[1 << C];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   unsigned char *at = smem_raw;
@@ -529,9 +540,9 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
 
   for (int m = threadIdx.x; m < 64; m += blockDim.x)
     sqrt_tab[m] = sqrt_term(m, Rl(0));
-  for (int m = threadIdx.x; m < 256; m += blockDim.x) {
+  for (int m = threadIdx.x; m < 1 << C; m += blockDim.x) {
     uint32_t v = 0, n = 0;
-    for (int k = 0; k < 8; k++)
+    for (int k = 0; k < C; k++)
       if ((m >> k) & 1) {
         v |= static_cast<uint32_t>(k) << (4 * n);
         n++;
@@ -588,16 +599,16 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
     const int rs = r0 - kHalo;       // first input row (frame coordinates)
     int nrows = static_cast<int>(limit - from) + 2 * kHalo;
     int nboxes = (nrows + kBoxRows - 1) / kBoxRows;
-    const int32_t tma_x = strip * kStripOut;
+    const int32_t tma_x = strip * Strip<T>::kOut;
     const int64_t tma_y0 = fd.row0 + rs;
 
     // Output columns of this lane: ring columns [10, 242) inside the frame.
     uint32_t outmask = 0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int j = 8 * lane + k;
-      const int col = strip * kStripOut + j - kHalo;
-      if (j >= kHalo && j < kHalo + kStripOut && col < fd.width)
+    for (int k = 0; k < C; k++) {
+      const int j = C * lane + k;
+      const int col = strip * Strip<T>::kOut + j - kHalo;
+      if (j >= kHalo && j < kHalo + Strip<T>::kOut && col < fd.width)
         outmask |= 1u << k;
     }
 
@@ -611,7 +622,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
     // writes before they are last read.
 #pragma unroll 1
     for (int i = 0; i < kPreRows; i++) {
-      uint4 *row = reinterpret_cast<uint4 *>(ring + (kRingRows - kPreRows + i) * kStripCols);
+      uint4 *row = reinterpret_cast<uint4 *>(ring + (kRingRows - kPreRows + i) * Strip<T>::kCols);
 #pragma unroll
       for (int v = 0; v < kVecs; v++)
         row[kVecs * lane + v] = make_uint4(0, 0, 0, 0);
@@ -624,14 +635,14 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       for (int b = 0; b < 2 && b < nboxes; b++) {
         const int st = b % kRingStages;
         mbar_expect_tx(&bars[st], kBoxBytes);
-        tma_load_2d(ring + st * kBoxRows * kStripCols, &arena, &bars[st], tma_x,
+        tma_load_2d(ring + st * kBoxRows * Strip<T>::kCols, &arena, &bars[st], tma_x,
                     static_cast<int32_t>(tma_y0 + b * kBoxRows));
       }
     }
 
-    A vs[8], vq[8], vg[8];
+    A vs[C], vq[C], vg[C];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < C; k++) {
       vs[k] = 7 * C7;
       vq[k] = 0;
       vg[k] = 11 * C11;
@@ -646,7 +657,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
     uint32_t dirty = 0;     // warp-uniform: bit i = the pair of row r-1-i holds a masked pixel
     uint32_t gdirty = 0;    // warp-uniform: bit i = row r-6-i holds a non-g pixel
 
-    auto row_at = [&](int slot) { return ring + slot * kStripCols; };
+    auto row_at = [&](int slot) { return ring + slot * Strip<T>::kCols; };
 
     // Rows r = rr and r+1 of the task (ring slots `slot`, slot+1) enter.
     // Row r's sums are completed before row r+1's; the stages of the two
@@ -676,12 +687,12 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       }
 
       // ---- 7-row sums: + rows r, r+1, - rows r-7, r-6 ------------------
-      uint32_t p[8], q[8];
-      A vsA[8], vqA[8];
+      uint32_t p[C], q[C];
+      A vsA[C], vqA[C];
       nA.unpack(p, down);
       lA.unpack(q, down);
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
+      for (int k = 0; k < C; k++) {
         vsA[k] = vs[k] + static_cast<A>(p[k]) - static_cast<A>(q[k]);
         vqA[k] = static_cast<A>(p[k]) * static_cast<A>(p[k]) -
                  (static_cast<A>(q[k]) * static_cast<A>(q[k]) - vq[k]);
@@ -690,7 +701,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
         const uint32_t mk7 = static_cast<uint32_t>(hist_mk >> 48) & 0xffu; // row r-7
         if (mkA | mk7) {
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
+          for (int k = 0; k < C; k++) {
             if ((mkA >> k) & 1u) {
               vsA[k] -= static_cast<A>(p[k]) + C7;
               vqA[k] -= static_cast<A>(p[k]) * static_cast<A>(p[k]);
@@ -705,7 +716,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       nB.unpack(p, down);
       lB.unpack(q, down);
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
+      for (int k = 0; k < C; k++) {
         vs[k] = vsA[k] + static_cast<A>(p[k]) - static_cast<A>(q[k]);
         vq[k] = static_cast<A>(p[k]) * static_cast<A>(p[k]) -
                 (static_cast<A>(q[k]) * static_cast<A>(q[k]) - vqA[k]);
@@ -714,7 +725,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
         const uint32_t mk6 = static_cast<uint32_t>(hist_mk >> 40) & 0xffu; // row r-6
         if (mkB | mk6) {
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
+          for (int k = 0; k < C; k++) {
             if ((mkB >> k) & 1u) {
               vs[k] -= static_cast<A>(p[k]) + C7;
               vq[k] -= static_cast<A>(p[k]) * static_cast<A>(p[k]);
@@ -737,7 +748,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
       const bool wdB = ((dirty & 0x1fu) | (flags & 3u)) != 0;
       uint32_t s0A, s0B;
       {
-        A hs[8], hq[8];
+        A hs[C], hq[C];
         hsum<3>(vsA, hs, wdA ? A(0) : kClean);
         hsum<3>(vqA, hq);
         if constexpr (sizeof(T) == 2)
@@ -746,7 +757,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
           s0A = dispersion_bits(hs, hq, sqrt_tab);
       }
       {
-        A hs[8], hq[8];
+        A hs[C], hq[C];
         hsum<3>(vs, hs, wdB ? A(0) : kClean);
         hsum<3>(vq, hq);
         if constexpr (sizeof(T) == 2)
@@ -759,35 +770,37 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
 
       // ---- erode at rows b = r-5 and b+1 -------------------------------
       // row b: dispersion rows r-7 .. r-3; row b+1: r-6 .. r-2. Both rows'
-      // bits travel in one word (row b in bits 0-7, b+1 in 16-23).
+      // bits travel in one word (row b in the low half, b+1 in the high one).
       const uint32_t vA = s0A & hist_s0 & (hist_s0 >> 8) & (hist_s0 >> 16) & (hist_s0 >> 24);
       const uint32_t vB = s0B & s0A & hist_s0 & (hist_s0 >> 8) & (hist_s0 >> 16);
       hist_s0 = (hist_s0 << 16) | (s0A << 8) | s0B;
-      const uint32_t v2 = (vA & 0xffu) | ((vB & 0xffu) << 16);
+      const uint32_t v2 = (vA & kLaneBits) | ((vB & kLaneBits) << 16);
+      constexpr uint32_t kBoth = kLaneBits | kLaneBits << 16;
       const uint32_t vl = shfl_up(v2), vr = shfl_down(v2);
-      const uint32_t w2 = ((vl >> 6) & 0x00030003u) | (v2 << 2) | ((vr << 10) & 0x0c000c00u);
-      const uint32_t hv2 = w2 & (w2 >> 1) & (w2 >> 2) & (w2 >> 3) & (w2 >> 4) & 0x00ff00ffu;
+      const uint32_t w2 = ((vl >> (C - 2)) & 0x00030003u) | (v2 << 2) |
+                          ((vr << (C + 2)) & (0x00030003u << (C + 2)));
+      const uint32_t hv2 = w2 & (w2 >> 1) & (w2 >> 2) & (w2 >> 3) & (w2 >> 4) & kBoth;
       const uint32_t mkb2 = (static_cast<uint32_t>(hist_mk >> 32) & 0xffu) |      // row r-5
                             ((static_cast<uint32_t>(hist_mk >> 24) & 0xffu) << 16); // r-4
       const uint32_t s1 = hv2 | mkb2;                 // scr1, src/dext.cc:117-142
-      const uint32_t gv2 = ~s1 & 0x00ff00ffu;         // valid and not kept
-      const uint32_t cs2 = s1 & ~mkb2 & 0x00ff00ffu;  // kept and not masked
+      const uint32_t gv2 = ~s1 & kBoth;               // valid and not kept
+      const uint32_t cs2 = s1 & ~mkb2 & kBoth;        // kept and not masked
       const uint32_t gvA = gv2 & 0xffu, gvB = gv2 >> 16;
       const uint32_t gflags =
-          __reduce_or_sync(kFull, (gvA != 0xffu ? 1u : 0u) | (gvB != 0xffu ? 2u : 0u));
+          __reduce_or_sync(kFull, (gvA != kLaneBits ? 1u : 0u) | (gvB != kLaneBits ? 2u : 0u));
 
       // ---- 11-row sums at rows b, b+1: + rows r-5, r-4, - rows r-16, r-15
-      const uint32_t ng16 = ~(gv_hi >> 16) & 0xffu; // row r-16
-      const uint32_t ng15 = ~(gv_hi >> 8) & 0xffu;  // row r-15
-      GroundWord<T> gp[8], gq[8];
+      const uint32_t ng16 = ~(gv_hi >> 16) & kLaneBits; // row r-16
+      const uint32_t ng15 = ~(gv_hi >> 8) & kLaneBits;  // row r-15
+      GroundWord<T> gp[C], gq[C];
       load_ground<T>(row_at(back_slot(slot, 5)), lane, gp, down);
       load_ground<T>(row_at(back_slot(slot, 16)), lane, gq, down);
       if ((gflags & 1u) | ((gdirty >> 10) & 1u))
         only_ground<T>(gp, gq, ~gvA, ng16);
       add_rows<T>(vg, gp, gq);
-      A vgA[8];
+      A vgA[C];
 #pragma unroll
-      for (int k = 0; k < 8; k++)
+      for (int k = 0; k < C; k++)
         vgA[k] = vg[k];
       load_ground<T>(row_at(back_slot(slot, 4)), lane, gp, down);
       load_ground<T>(row_at(back_slot(slot, 15)), lane, gq, down);
@@ -811,17 +824,17 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
         // for one division and one square root: a prefix count over the
         // lanes, and each lane finds its candidate by itself.
         if constexpr (sizeof(A) == 4) {
-          uint4 *w0 = reinterpret_cast<uint4 *>(win + 8 * lane);
-          uint4 *w1 = reinterpret_cast<uint4 *>(win + kStripCols + 8 * lane);
+          uint4 *w0 = reinterpret_cast<uint4 *>(win + C * lane);
+          uint4 *w1 = reinterpret_cast<uint4 *>(win + Strip<T>::kCols + C * lane);
           w0[0] = make_uint4(vgA[0], vgA[1], vgA[2], vgA[3]);
           w0[1] = make_uint4(vgA[4], vgA[5], vgA[6], vgA[7]);
           w1[0] = make_uint4(vg[0], vg[1], vg[2], vg[3]);
           w1[1] = make_uint4(vg[4], vg[5], vg[6], vg[7]);
         } else {
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
-            win[8 * lane + k] = vgA[k];
-            win[kStripCols + 8 * lane + k] = vg[k];
+          for (int k = 0; k < C; k++) {
+            win[C * lane + k] = vgA[k];
+            win[Strip<T>::kCols + C * lane + k] = vg[k];
           }
         }
         const uint32_t cntA = __popc(csA), cntB = __popc(csB);
@@ -856,7 +869,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
         const uint32_t start = chunk + fill;
         const int c = rs + rr - kHalo; // frame row of row c
         const uint32_t index0 = static_cast<uint32_t>(c) * static_cast<uint32_t>(fd.width) +
-                                static_cast<uint32_t>(strip * kStripOut - kHalo);
+                                static_cast<uint32_t>(strip * Strip<T>::kOut - kHalo);
         uint32_t foundA = 0, foundB = 0;
         for (uint32_t base = 0; base < total; base += 32) {
           const uint32_t i = base + lane;
@@ -883,9 +896,9 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
           SignalPixel px;
           if (i < total) {
             const uint32_t j = t - ((exL >> sh) & 0xffffu);
-            const uint32_t col = 8 * L + ((pL >> (4 * j)) & 0xfu); // an output column
+            const uint32_t col = C * L + ((pL >> (4 * j)) & 0xfu); // an output column
             const T *prow = row_at(back_slot(slot, rowB ? 9 : 10));
-            const A *w = win + (rowB ? kStripCols : 0);
+            const A *w = win + (rowB ? Strip<T>::kCols : 0);
             const uint32_t pv = prow[col];
             A h = 0;
 #pragma unroll
@@ -957,7 +970,7 @@ __global__ void __launch_bounds__(WPC * 32, (kWarpsPerSm<T> / WPC) > 0 ? kWarpsP
         const int nst = (b + 1) % kRingStages;
         fence_proxy_async_smem();
         mbar_expect_tx(&bars[nst], kBoxBytes);
-        tma_load_2d(ring + nst * kBoxRows * kStripCols, &arena, &bars[nst], tma_x,
+        tma_load_2d(ring + nst * kBoxRows * Strip<T>::kCols, &arena, &bars[nst], tma_x,
                     static_cast<int32_t>(tma_y0 + (b + 1) * kBoxRows));
       }
       const bool ok = mbar_wait_bounded(&bars[st], (phase >> st) & 1u, args.wait_limit);
