@@ -82,9 +82,9 @@ Layout plan_layout(uint64_t height, uint64_t width) {
   L.max_blocks = device_sm_count() * std::min(occ, kBlocksPerSm);
   const uint64_t resident = static_cast<uint64_t>(L.max_blocks) * kWarpsPerBlock;
 
-  const uint64_t strips = (width + strip_out(2) - 1) / strip_out(2);
+  const uint64_t strips = (width + strip_out(2, 8) - 1) / strip_out(2, 8);
   // 232 output columns per 256-column strip; rows start on 128-byte lines
-  L.pitch = align_up(strips * strip_out(2) + (strip_cols(2) - strip_out(2)), 64);
+  L.pitch = align_up(strips * strip_out(2, 8) + (strip_cols(8) - strip_out(2, 8)), 64);
   L.rows = height + 2 * kMarginRows;
 
   // Output rows per task: fewest waves x (rows + 20 rows of halo).
@@ -221,7 +221,7 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
         "copying the frame to the device");
 
   CUtensorMap map;
-  encode_arena_map(&map, arena, 2, L.pitch, L.rows);
+  encode_arena_map(&map, arena, 2, L.pitch, L.rows, 8);
   ThresholdLaunch T;
   T.frames = frames;
   T.nframes = 1;
@@ -237,6 +237,7 @@ int find_noalloc(const uint16_t *image, size_t height, size_t width, SignalPixel
   T.status = run_status;
   T.wait_limit = 1u << 22;
   T.warps_per_block = kWarpsPerBlock;
+  T.lane_cols = 8;
   T.max_blocks = L.max_blocks;
   check(launch_threshold<uint16_t>(map, T, s), "launching the threshold");
 

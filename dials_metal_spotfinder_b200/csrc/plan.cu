@@ -43,30 +43,44 @@ constexpr uint64_t kLinearUpload = 512 * 1024;
 
 uint64_t round_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 
-// Output rows per task. A task costs its rows plus the 20 rows of halo it
-// re-reads; how long a row takes depends on the warps that share the SM: as
-// 5 + w for w of them, and no less than for 7, when a warp waits on itself
-// (16-bit pixels, one frame of each of several sizes over many heights; 0.08
-// us a unit). So the height with the least (rows + 20) x (5 + w), an SM's w
-// taken as the most that any has when the blocks are dealt out, in as many
-// rounds as they need; no shorter than kMinSeg rows, below which the halo is
-// most of the work and the gain is in the noise. The threshold of one frame:
-// 2162 x 2068 uint16 59 -> 52 us (17 rows; 16, the least there was, put a
-// tenth warp on some SMs), 1062 x 1028 44 -> 36 us (6 rows), 256 x 384
-// 35 -> 27 us (4 rows).
-constexpr uint64_t kRowBase = 5, kRowLeast = 12;
+// Output rows per task, and what the launch then costs. A task costs its rows
+// plus the 20 rows of halo it re-reads; how long a row takes depends on the
+// warps that share the SM: as 5 + w for w of them, and no less than for 7, when
+// a warp waits on itself (16-bit pixels, one frame of each of several sizes
+// over many heights; 0.08 us a unit). So the height with the least
+// (rows + 20) x (5 + w), an SM's w taken as the most that any has when the
+// blocks are dealt out, in as many rounds as they need; no shorter than kMinSeg
+// rows, below which the halo is most of the work and the gain is in the noise.
+// The threshold of one frame: 2162 x 2068 uint16 59 -> 52 us (17 rows; 16, the
+// least there was, put a tenth warp on some SMs), 1062 x 1028 44 -> 36 us
+// (6 rows), 256 x 384 35 -> 27 us (4 rows).
+//
+// Strips of 4 columns a lane have 2.2 times the tasks of 8, but a row of theirs
+// takes 8.2 + 0.4 w units, no less than 9.5: a small frame, whose warps have an
+// SM's schedulers nearly to themselves, is done sooner (256 x 384 uint16
+// 25 -> 22 us, 700 x 900 30 -> 28, 1062 x 1028 34.5 -> 32.5; 2162 x 2068 would
+// take 51 for 48). The two costs decide.
+struct Heights {
+  int rows;
+  uint64_t cost; // tenths of a unit
+};
 constexpr int kMinSeg = 4;
-int choose_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, uint64_t sms,
-                    int wpc, int blocks_per_sm) {
+Heights choose_seg_rows(int elem_bytes, int lane_cols,
+                        const std::vector<ThresholdPlan::Shape> &shapes, uint64_t sms, int wpc,
+                        int blocks_per_sm) {
+  const bool narrow = elem_bytes == 2 && lane_cols == 4;
+  auto row_cost = [&](uint64_t w) {
+    return narrow ? std::max<uint64_t>(95, 82 + 4 * w) : std::max<uint64_t>(120, 50 + 10 * w);
+  };
+  const uint64_t out_cols = strip_out(elem_bytes, lane_cols);
   int max_h = 1;
   for (const auto &s : shapes)
     max_h = std::max(max_h, s.height);
-  int best = max_h;
-  uint64_t best_cost = ~0ull;
+  Heights best{max_h, ~0ull};
   for (int seg = std::min(kMinSeg, max_h); seg <= max_h; seg++) {
     uint64_t tasks = 0;
     for (const auto &s : shapes) {
-      const uint64_t strips = (s.width + strip_out(elem_bytes) - 1) / strip_out(elem_bytes);
+      const uint64_t strips = (s.width + out_cols - 1) / out_cols;
       tasks += strips * ((s.height + seg - 1) / seg);
     }
     const uint64_t per_block = static_cast<uint64_t>(wpc);
@@ -74,13 +88,10 @@ int choose_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &sha
     const uint64_t per_sm = (blocks + sms - 1) / sms * per_block;
     const uint64_t fit = static_cast<uint64_t>(blocks_per_sm) * per_block;
     const uint64_t rest = per_sm % fit;
-    const uint64_t row = per_sm / fit * std::max(kRowLeast, kRowBase + fit) +
-                         (rest ? std::max(kRowLeast, kRowBase + rest) : 0);
+    const uint64_t row = per_sm / fit * row_cost(fit) + (rest ? row_cost(rest) : 0);
     const uint64_t cost = row * static_cast<uint64_t>(std::min(seg, max_h) + 2 * kHalo);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = seg;
-    }
+    if (cost < best.cost)
+      best = Heights{seg, cost};
   }
   return best;
 }
@@ -95,14 +106,16 @@ int model_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shap
     throw DeviceError("the threshold kernel does not fit on this device");
   if (blocks_per_sm > 0)
     occ = std::min(occ, blocks_per_sm);
-  return choose_seg_rows(elem_bytes, shapes, static_cast<uint64_t>(device_sm_count()), wpc, occ);
+  return choose_seg_rows(elem_bytes, elem_bytes == 2 ? 8 : 4, shapes,
+                         static_cast<uint64_t>(device_sm_count()), wpc, occ)
+      .rows;
 }
 
 void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes, uint64_t pitch_elems,
-                      uint64_t rows) {
+                      uint64_t rows, int lane_cols) {
   const cuuint64_t dims[2] = {pitch_elems, rows};
   const cuuint64_t strides[1] = {pitch_elems * static_cast<uint64_t>(elem_bytes)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(strip_cols(elem_bytes)),
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(strip_cols(lane_cols)),
                              static_cast<cuuint32_t>(kBoxRows)};
   const cuuint32_t estride[2] = {1, 1};
   const CUtensorMapDataType dt =
@@ -148,21 +161,12 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
   if (wpc != 1 && wpc != 2 && wpc != 4)
     throw std::invalid_argument("warps_per_block must be 1, 2 or 4");
 
-  const int out_cols = strip_out(elem_bytes);
-  int32_t max_strips = 0;
   for (const Shape &s : shapes) {
     if (s.height < 1 || s.width < 1)
       throw std::invalid_argument("frame with no pixels");
     if (static_cast<uint64_t>(s.height) * s.width > 0x7fffffffull)
       throw std::invalid_argument("frame larger than INT32_MAX pixels");
-    max_strips = std::max(max_strips, (s.width + out_cols - 1) / out_cols);
   }
-  // Every strip reads its columns from a multiple of its output columns; the
-  // pitch is a multiple of 128 bytes so each arena row starts on a TMA-friendly
-  // line.
-  pitch_ = round_up(static_cast<uint64_t>(max_strips) * out_cols +
-                        (strip_cols(elem_bytes) - out_cols),
-                    128 / elem_bytes);
 
   const int occ = elem_bytes == 2 ? threshold_occupancy<uint16_t>(wpc)
                                   : threshold_occupancy<uint32_t>(wpc);
@@ -171,8 +175,30 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
   const int per_sm = tuning_.blocks_per_sm > 0 ? std::min(tuning_.blocks_per_sm, occ) : occ;
   sms_ = device_sm_count();
   max_blocks_ = sms_ * per_sm;
-  if (tuning_.seg_rows <= 0)
-    tuning_.seg_rows = choose_seg_rows(elem_bytes, shapes, static_cast<uint64_t>(sms_), wpc, per_sm);
+  lane_cols_ = elem_bytes == 2 ? 8 : 4;
+  if (tuning_.seg_rows <= 0) {
+    const uint64_t sms = static_cast<uint64_t>(sms_);
+    Heights h = choose_seg_rows(elem_bytes, lane_cols_, shapes, sms, wpc, per_sm);
+    if (elem_bytes == 2) {
+      const Heights narrow = choose_seg_rows(elem_bytes, 4, shapes, sms, wpc, per_sm);
+      if (narrow.cost < h.cost) {
+        h = narrow;
+        lane_cols_ = 4;
+      }
+    }
+    tuning_.seg_rows = h.rows;
+  }
+
+  const int out_cols = strip_out(elem_bytes, lane_cols_);
+  int32_t max_strips = 0;
+  for (const Shape &s : shapes)
+    max_strips = std::max(max_strips, (s.width + out_cols - 1) / out_cols);
+  // Every strip reads its columns from a multiple of its output columns; the
+  // pitch is a multiple of 128 bytes so each arena row starts on a TMA-friendly
+  // line.
+  pitch_ = round_up(static_cast<uint64_t>(max_strips) * out_cols +
+                        (strip_cols(lane_cols_) - out_cols),
+                    128 / elem_bytes);
 
   uint64_t row = 0, tile = 0, out = 0;
   uint32_t task = 0;
@@ -257,7 +283,7 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
             "cudaMalloc frame counts");
       sl.status = reinterpret_cast<int *>(sl.frame_count + nf);
       check(cudaMemset(sl.frame_count, 0, (nf + 1) * 4), "clearing frame counts");
-      encode_arena_map(&sl.map, sl.arena, elem_bytes_, pitch_, arena_rows_);
+      encode_arena_map(&sl.map, sl.arena, elem_bytes_, pitch_, arena_rows_, lane_cols_);
     }
     // The fills above ran on the legacy stream; the plan's users work on
     // non-blocking streams that do not wait for it.
@@ -351,6 +377,7 @@ void ThresholdPlan::enqueue(int slot, cudaStream_t stream, cudaEvent_t mid, Host
   L.status = run_status_;
   L.wait_limit = 1u << 22;
   L.warps_per_block = tuning_.warps_per_block;
+  L.lane_cols = lane_cols_;
   L.max_blocks = max_blocks_;
   if (elem_bytes_ == 2)
     check(launch_threshold<uint16_t>(sl.map, L, stream), "launching the threshold");

@@ -27,23 +27,13 @@ static_assert(sizeof(SignalPixel) == 16, "SignalPixel must be 16 bytes");
 // those are a multiple of 16 bytes, which keeps every strip's first column
 // aligned for TMA.
 constexpr int kHalo = 10;                  // 3 (7x7) + 2 (5x5) + 5 (11x11)
-template <typename T> struct Strip;
-template <> struct Strip<uint16_t> {
-  static constexpr int kLane = 8;          // columns a lane
-  static constexpr int kCols = 32 * kLane; // 256
-  static constexpr int kOut = 232;         // output columns; 4 more are padding
-};
-template <> struct Strip<uint32_t> {
-  static constexpr int kLane = 4;
-  static constexpr int kCols = 32 * kLane; // 128
-  static constexpr int kOut = 108;
-};
-constexpr int strip_cols(int elem_bytes) {
-  return elem_bytes == 2 ? Strip<uint16_t>::kCols : Strip<uint32_t>::kCols;
+// With `lane_cols` columns a lane: 8 or 4 of 16-bit pixels (256 columns for 232
+// of output, 128 for 104), 4 of 32-bit ones (128 for 108).
+__host__ __device__ constexpr int strip_cols(int lane_cols) { return 32 * lane_cols; }
+__host__ __device__ constexpr int strip_out(int elem_bytes, int lane_cols) {
+  return (32 * lane_cols - 2 * kHalo) / (16 / elem_bytes) * (16 / elem_bytes);
 }
-constexpr int strip_out(int elem_bytes) {
-  return elem_bytes == 2 ? Strip<uint16_t>::kOut : Strip<uint32_t>::kOut;
-}
+static_assert(strip_out(2, 8) == 232 && strip_out(2, 4) == 104 && strip_out(4, 4) == 108);
 constexpr int kMarginLeft = kHalo;         // frame column 0 at buffer column 10
 constexpr int kMarginRows = kHalo;         // rows of fill above and below
 constexpr int kRingRows = 20;              // rows of a strip held in smem
@@ -53,7 +43,7 @@ constexpr uint32_t kChunkRecords = 1024;   // staging pool allocation unit
 // The most records a warp stages at once (two output rows of a strip); a
 // staging chunk is abandoned when that many might not fit, so each chunk
 // wastes fewer than this.
-constexpr uint32_t kMaxStaged = 2 * Strip<uint16_t>::kOut;
+constexpr uint32_t kMaxStaged = 2 * strip_out(2, 8);
 
 // Limits of the word in which the threshold's warps share a task's rows (row
 // numbers of kSharedRowBits bits, task numbers of the 22 bits above two): plans

@@ -45,13 +45,13 @@ struct ThresholdLaunch {
   int *status;
   uint32_t wait_limit;
   int warps_per_block;
+  int lane_cols; // columns a lane: 8 or 4 for 16-bit pixels, 4 for 32-bit ones
   int max_blocks; // 0: one warp per task
 };
 
 template <typename T>
 cudaError_t launch_threshold(const CUtensorMap &map, const ThresholdLaunch &L,
                              cudaStream_t stream);
-template <typename T> size_t threshold_smem_bytes(int wpc);
 template <typename T> int threshold_occupancy(int wpc);
 
 // What a one-frame batch leaves in page-locked host memory besides its list on
@@ -101,7 +101,7 @@ void repitch(const uint8_t *src, size_t height, size_t row_bytes, void *dst, siz
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
 // library needs no link against libcuda.
 void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes,
-                      uint64_t pitch_elems, uint64_t rows);
+                      uint64_t pitch_elems, uint64_t rows, int lane_cols);
 
 int device_sm_count();
 
@@ -191,6 +191,7 @@ private:
   uint64_t ntiles_ = 0, total_capacity_ = 0;
   uint32_t pool_cap_ = 0;
   int max_blocks_ = 0, grid_blocks_ = 0, sms_ = 0;
+  int lane_cols_ = 8; // columns a lane (ThresholdLaunch)
   uint64_t device_bytes_ = 0;
 
   std::vector<Slot> slots_;

@@ -3,8 +3,9 @@
 // as one streaming kernel per batch of frames.
 //
 // Decomposition. A task is one strip of buffer columns (256 of 16-bit pixels,
-// of which 232 are output and the rest halo; 128 of 32-bit ones, 108 output) by
-// one segment of output rows of one frame. A warp owns
+// of which 232 are output and the rest halo, or 128 and 104 for small frames;
+// 128 and 108 of 32-bit ones) by one segment of output rows of one frame. A
+// warp owns
 // a task at a time and walks down it row by row; one that has nothing left
 // takes rows from another's task (see pack_range), but none waits for
 // another. Each warp has a ring of 20 rows of its strip in shared memory, fed
@@ -68,8 +69,8 @@
 //
 // Output order. Records for the tile (row, strip) land contiguously in the
 // staging pool; the tile's count and start go to two small arrays. The
-// placement kernels (place.cu) then scan the counts in row-major tile order,
-// which is ascending pixel index, and copy each tile's records to the final
+// placement (place.cu) then scans the counts in row-major tile order,
+// which is ascending pixel index, and copies each tile's records to the final
 // list -- so the list comes out sorted by index with no sort.
 
 #include <math_constants.h>
@@ -116,18 +117,19 @@ __device__ __forceinline__ uint32_t push_sign(uint32_t bits, float x) {
 // The two tests, in the reference's arithmetic.
 // --------------------------------------------------------------------------
 
-// src/dext.cc:97-110 with R = float, for the 8 columns of a lane: window
+// src/dext.cc:97-110 with R = float, for the columns of a lane: window
 // count+sum packed in hs (count << 22 | sum), sum of squares in hq. `sq` is
 // the per-count table (sqrt_term). Bit k set where the window is dispersed.
-__device__ __forceinline__ uint32_t dispersion_bits(const uint32_t (&hs)[8],
-                                                    const uint32_t (&hq)[8],
+template <int C>
+__device__ __forceinline__ uint32_t dispersion_bits(const uint32_t (&hs)[C],
+                                                    const uint32_t (&hq)[C],
                                                     const float *sq) {
   const float2 magic = make_float2(-8388608.0f, -8388608.0f);
   const float2 neg1 = make_float2(-1.0f, -1.0f);
   const float2 six = make_float2(6.0f, 6.0f);
   uint32_t bits = 0;
 #pragma unroll
-  for (int k = 6; k >= 0; k -= 2) {
+  for (int k = C - 2; k >= 0; k -= 2) {
     const uint32_t m0 = hs[k] >> 22, m1 = hs[k + 1] >> 22;
     const float2 S = __fadd2_rn(make_float2(magic_bits(hs[k] & 0x3fffffu),
                                             magic_bits(hs[k + 1] & 0x3fffffu)),
@@ -155,8 +157,9 @@ __device__ __forceinline__ uint32_t dispersion_bits(const uint32_t (&hs)[8],
 // scaling by a power of two is exact and commutes with rounding, so
 // fl(s * 48) = 8 fl(s * 6), and t3 - fl(s * 48) is one fused operation on
 // the already rounded fl(s * 6), which the right side needs anyway.
-__device__ __forceinline__ uint32_t dispersion_bits49(const uint32_t (&hs)[8],
-                                                      const uint32_t (&hq)[8], float sq49) {
+template <int C>
+__device__ __forceinline__ uint32_t dispersion_bits49(const uint32_t (&hs)[C],
+                                                      const uint32_t (&hq)[C], float sq49) {
   const float2 magic = make_float2(-8388608.0f, -8388608.0f);
   const float2 neg1 = make_float2(-1.0f, -1.0f);
   const float2 neg8 = make_float2(-8.0f, -8.0f);
@@ -165,7 +168,7 @@ __device__ __forceinline__ uint32_t dispersion_bits49(const uint32_t (&hs)[8],
   const float2 R = make_float2(sq49, sq49);
   uint32_t bits = 0;
 #pragma unroll
-  for (int k = 6; k >= 0; k -= 2) {
+  for (int k = C - 2; k >= 0; k -= 2) {
     const float2 S = __fadd2_rn(make_float2(__uint_as_float(hs[k]), __uint_as_float(hs[k + 1])),
                                 magic);
     const float2 Q = make_float2(__uint2float_rn(hq[k]), __uint2float_rn(hq[k + 1]));
@@ -224,9 +227,9 @@ __device__ __forceinline__ bool poisson(uint32_t p, uint64_t m, uint64_t s,
 // --------------------------------------------------------------------------
 
 // The lane's pixels of one ring row, and whether any is masked.
-template <typename T> struct LaneRow;
+template <typename T, int C> struct LaneRow;
 
-template <> struct LaneRow<uint16_t> {
+template <> struct LaneRow<uint16_t, 8> {
   uint4 v;
   __device__ __forceinline__ void load(const uint16_t *row, int lane) {
     v = reinterpret_cast<const uint4 *>(row)[lane];
@@ -259,7 +262,29 @@ template <> struct LaneRow<uint16_t> {
   }
 };
 
-template <> struct LaneRow<uint32_t> {
+template <> struct LaneRow<uint16_t, 4> {
+  uint2 v;
+  __device__ __forceinline__ void load(const uint16_t *row, int lane) {
+    v = reinterpret_cast<const uint2 *>(row)[lane];
+  }
+  __device__ __forceinline__ void unpack(uint32_t (&p)[4], uint32_t down) const {
+    p[1] = v.x >> 16;
+    p[0] = p[1] * down + v.x;
+    p[3] = v.y >> 16;
+    p[2] = p[3] * down + v.y;
+  }
+  static __device__ __forceinline__ bool any_masked(const LaneRow &r, const LaneRow &s) {
+    const uint32_t m = __vmaxu2(__vmaxu2(r.v.x, r.v.y), __vmaxu2(s.v.x, s.v.y));
+    return (m & 0xffffu) >= 0xfffeu || m >= 0xfffe0000u;
+  }
+  __device__ __forceinline__ uint32_t masked_bits() const {
+    const uint32_t x = (__vcmpgeu2(v.x, 0xfffefffeu) & 0x00010001u) |
+                       ((__vcmpgeu2(v.y, 0xfffefffeu) & 0x00010001u) << 2);
+    return (x | (x >> 15)) & 0xfu;
+  }
+};
+
+template <> struct LaneRow<uint32_t, 4> {
   uint4 v;
   __device__ __forceinline__ void load(const uint32_t *row, int lane) {
     v = reinterpret_cast<const uint4 *>(row)[lane];
@@ -279,10 +304,10 @@ template <> struct LaneRow<uint32_t> {
   }
 };
 
-template <typename T>
+template <typename T, int C>
 __device__ __forceinline__ void load_pixels(const T *row, int lane,
-                                            uint32_t (&p)[Strip<T>::kLane], uint32_t down) {
-  LaneRow<T> r;
+                                            uint32_t (&p)[C], uint32_t down) {
+  LaneRow<T, C> r;
   r.load(row, lane);
   r.unpack(p, down);
 }
@@ -333,32 +358,32 @@ __device__ __forceinline__ void hsum(const A (&v)[C], A (&h)[C], A from = 0) {
 // that enters and the one that leaves), and one that is masked or kept, whose
 // bit is in `ng`, is changed to take its count back and add nothing.
 template <typename T> using GroundWord = typename Traits<T>::Acc;
-template <typename T>
+template <typename T, int C>
 __device__ __forceinline__ void load_ground(const T *row, int lane,
-                                            GroundWord<T> (&g)[Strip<T>::kLane], uint32_t down) {
-  uint32_t p[Strip<T>::kLane];
+                                            GroundWord<T> (&g)[C], uint32_t down) {
+  uint32_t p[C];
   load_pixels<T>(row, lane, p, down);
 #pragma unroll
-  for (int k = 0; k < Strip<T>::kLane; k++)
+  for (int k = 0; k < C; k++)
     g[k] = p[k];
 }
-template <typename T>
-__device__ __forceinline__ void only_ground(GroundWord<T> (&in)[Strip<T>::kLane],
-                                            GroundWord<T> (&out)[Strip<T>::kLane],
+template <typename T, int C>
+__device__ __forceinline__ void only_ground(GroundWord<T> (&in)[C],
+                                            GroundWord<T> (&out)[C],
                                             uint32_t ng_in, uint32_t ng_out) {
   constexpr GroundWord<T> kNot = GroundWord<T>(0) - (GroundWord<T>(1) << Traits<T>::kShift11);
 #pragma unroll
-  for (int k = 0; k < Strip<T>::kLane; k++) {
+  for (int k = 0; k < C; k++) {
     in[k] = (ng_in >> k) & 1u ? kNot : in[k];
     out[k] = (ng_out >> k) & 1u ? kNot : out[k];
   }
 }
-template <typename T>
-__device__ __forceinline__ void add_rows(GroundWord<T> (&sum)[Strip<T>::kLane],
-                                         const GroundWord<T> (&in)[Strip<T>::kLane],
-                                         const GroundWord<T> (&out)[Strip<T>::kLane]) {
+template <typename T, int C>
+__device__ __forceinline__ void add_rows(GroundWord<T> (&sum)[C],
+                                         const GroundWord<T> (&in)[C],
+                                         const GroundWord<T> (&out)[C]) {
 #pragma unroll
-  for (int k = 0; k < Strip<T>::kLane; k++)
+  for (int k = 0; k < C; k++)
     sum[k] += in[k] - out[k];
 }
 
@@ -501,28 +526,29 @@ static_assert(kBoxRows == 2 && kRingRows % kBoxRows == 0, "a box is a pair of ro
 static_assert(kQuantum % 2 == 0 && kQuantum / kBoxRows >= 2, "claims go in pairs of rows");
 
 // Per-warp shared memory (the square-root table is static).
-template <typename T> struct WarpSmem {
+template <typename T, int C> struct WarpSmem {
   using A = typename Traits<T>::Acc;
-  static constexpr uint32_t kRing = Strip<T>::kCols * sizeof(T) * kRingRows;
-  static constexpr uint32_t kWin = 2 * Strip<T>::kCols * sizeof(A);
+  static constexpr int kCols = strip_cols(C);
+  static constexpr uint32_t kRing = kCols * sizeof(T) * kRingRows;
+  static constexpr uint32_t kWin = 2 * kCols * sizeof(A);
   static constexpr uint32_t kBars = kRingStages * sizeof(uint64_t);
   static constexpr uint32_t kTotal = kRing + kWin + kBars;
 };
 
-template <typename T, int WPC>
+template <typename T, int WPC, int C>
 __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     threshold_kernel(const __grid_constant__ CUtensorMap arena, ThresholdArgs args) {
   using Tr = Traits<T>;
-  constexpr int C = Strip<T>::kLane;
+  constexpr int kCols = strip_cols(C), kOut = strip_out(sizeof(T), C);
   constexpr uint32_t kLaneBits = (1u << C) - 1; // a bit a column
   using A = typename Tr::Acc;
   using Rl = typename Real<T>::type;
-  using Sm = WarpSmem<T>;
-  constexpr uint32_t kRowBytes = Strip<T>::kCols * sizeof(T);
+  using Sm = WarpSmem<T, C>;
+  constexpr uint32_t kRowBytes = kCols * sizeof(T);
   constexpr uint32_t kBoxBytes = kRowBytes * kBoxRows;
   constexpr A C7 = A(1) << Tr::kShift7;   // one valid pixel's count in a 7 x 7 sum
   constexpr A C11 = A(1) << Tr::kShift11; // ... in an 11 x 11 sum
-  constexpr int kVecs = Strip<T>::kCols * sizeof(T) / (32 * 16); // 16-byte words per lane per row
+  constexpr int kZeros = kPreRows * kCols * sizeof(T) / (32 * 16); // 16-byte words a lane
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ Rl sqrt_tab[64];
@@ -599,7 +625,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     const int rs = r0 - kHalo;       // first input row (frame coordinates)
     int nrows = static_cast<int>(limit - from) + 2 * kHalo;
     int nboxes = (nrows + kBoxRows - 1) / kBoxRows;
-    const int32_t tma_x = strip * Strip<T>::kOut;
+    const int32_t tma_x = strip * kOut;
     const int64_t tma_y0 = fd.row0 + rs;
 
     // Output columns of this lane: ring columns [10, 242) inside the frame.
@@ -607,8 +633,8 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
 #pragma unroll
     for (int k = 0; k < C; k++) {
       const int j = C * lane + k;
-      const int col = strip * Strip<T>::kOut + j - kHalo;
-      if (j >= kHalo && j < kHalo + Strip<T>::kOut && col < fd.width)
+      const int col = strip * kOut + j - kHalo;
+      if (j >= kHalo && j < kHalo + kOut && col < fd.width)
         outmask |= 1u << k;
     }
 
@@ -620,13 +646,10 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     // windows reach 10 rows up, and the first output row is the task's
     // 11th. They live in the ring slots of rows -16 .. -1, which no TMA box
     // writes before they are last read.
-#pragma unroll 1
-    for (int i = 0; i < kPreRows; i++) {
-      uint4 *row = reinterpret_cast<uint4 *>(ring + (kRingRows - kPreRows + i) * Strip<T>::kCols);
-#pragma unroll
-      for (int v = 0; v < kVecs; v++)
-        row[kVecs * lane + v] = make_uint4(0, 0, 0, 0);
-    }
+    uint4 *zeros = reinterpret_cast<uint4 *>(ring + (kRingRows - kPreRows) * kCols);
+#pragma unroll 4
+    for (int i = 0; i < kZeros; i++)
+      zeros[32 * i + lane] = make_uint4(0, 0, 0, 0);
     fence_proxy_async_smem(); // these writes before any later TMA write of the slots
     __syncwarp();
 
@@ -635,7 +658,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
       for (int b = 0; b < 2 && b < nboxes; b++) {
         const int st = b % kRingStages;
         mbar_expect_tx(&bars[st], kBoxBytes);
-        tma_load_2d(ring + st * kBoxRows * Strip<T>::kCols, &arena, &bars[st], tma_x,
+        tma_load_2d(ring + st * kBoxRows * kCols, &arena, &bars[st], tma_x,
                     static_cast<int32_t>(tma_y0 + b * kBoxRows));
       }
     }
@@ -657,7 +680,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     uint32_t dirty = 0;     // warp-uniform: bit i = the pair of row r-1-i holds a masked pixel
     uint32_t gdirty = 0;    // warp-uniform: bit i = row r-6-i holds a non-g pixel
 
-    auto row_at = [&](int slot) { return ring + slot * Strip<T>::kCols; };
+    auto row_at = [&](int slot) { return ring + slot * kCols; };
 
     // Rows r = rr and r+1 of the task (ring slots `slot`, slot+1) enter.
     // Row r's sums are completed before row r+1's; the stages of the two
@@ -665,7 +688,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     // work to interleave.
     auto process_pair = [&](int rr, int slot) {
       // ---- loads, masks, and the pair's warp-wide flags -----------------
-      LaneRow<T> nA, nB, lA, lB;
+      LaneRow<T, C> nA, nB, lA, lB;
       nA.load(row_at(slot), lane);
       nB.load(row_at(slot + 1), lane);
       lA.load(row_at(back_slot(slot, 7)), lane);
@@ -678,7 +701,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
       // bits 0 and 1: a masked pixel in row r, r+1 (in either: the pair is
       // tested as one); bit 2: a candidate
       const uint32_t flags =
-          __reduce_or_sync(kFull, (LaneRow<T>::any_masked(nA, nB) ? 3u : 0u) |
+          __reduce_or_sync(kFull, (LaneRow<T, C>::any_masked(nA, nB) ? 3u : 0u) |
                                       ((csA | csB) ? 4u : 0u));
       uint32_t mkA = 0, mkB = 0;
       if (flags & 3u) {
@@ -825,16 +848,17 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
         // lanes, and each lane finds its candidate by itself.
         if constexpr (sizeof(A) == 4) {
           uint4 *w0 = reinterpret_cast<uint4 *>(win + C * lane);
-          uint4 *w1 = reinterpret_cast<uint4 *>(win + Strip<T>::kCols + C * lane);
-          w0[0] = make_uint4(vgA[0], vgA[1], vgA[2], vgA[3]);
-          w0[1] = make_uint4(vgA[4], vgA[5], vgA[6], vgA[7]);
-          w1[0] = make_uint4(vg[0], vg[1], vg[2], vg[3]);
-          w1[1] = make_uint4(vg[4], vg[5], vg[6], vg[7]);
+          uint4 *w1 = reinterpret_cast<uint4 *>(win + kCols + C * lane);
+#pragma unroll
+          for (int k = 0; k < C; k += 4) {
+            w0[k / 4] = make_uint4(vgA[k], vgA[k + 1], vgA[k + 2], vgA[k + 3]);
+            w1[k / 4] = make_uint4(vg[k], vg[k + 1], vg[k + 2], vg[k + 3]);
+          }
         } else {
 #pragma unroll
           for (int k = 0; k < C; k++) {
             win[C * lane + k] = vgA[k];
-            win[Strip<T>::kCols + C * lane + k] = vg[k];
+            win[kCols + C * lane + k] = vg[k];
           }
         }
         const uint32_t cntA = __popc(csA), cntB = __popc(csB);
@@ -869,7 +893,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
         const uint32_t start = chunk + fill;
         const int c = rs + rr - kHalo; // frame row of row c
         const uint32_t index0 = static_cast<uint32_t>(c) * static_cast<uint32_t>(fd.width) +
-                                static_cast<uint32_t>(strip * Strip<T>::kOut - kHalo);
+                                static_cast<uint32_t>(strip * kOut - kHalo);
         uint32_t foundA = 0, foundB = 0;
         for (uint32_t base = 0; base < total; base += 32) {
           const uint32_t i = base + lane;
@@ -898,7 +922,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
             const uint32_t j = t - ((exL >> sh) & 0xffffu);
             const uint32_t col = C * L + ((pL >> (4 * j)) & 0xfu); // an output column
             const T *prow = row_at(back_slot(slot, rowB ? 9 : 10));
-            const A *w = win + (rowB ? Strip<T>::kCols : 0);
+            const A *w = win + (rowB ? kCols : 0);
             const uint32_t pv = prow[col];
             A h = 0;
 #pragma unroll
@@ -970,7 +994,7 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
         const int nst = (b + 1) % kRingStages;
         fence_proxy_async_smem();
         mbar_expect_tx(&bars[nst], kBoxBytes);
-        tma_load_2d(ring + nst * kBoxRows * Strip<T>::kCols, &arena, &bars[nst], tma_x,
+        tma_load_2d(ring + nst * kBoxRows * kCols, &arena, &bars[nst], tma_x,
                     static_cast<int32_t>(tma_y0 + (b + 1) * kBoxRows));
       }
       const bool ok = mbar_wait_bounded(&bars[st], (phase >> st) & 1u, args.wait_limit);
@@ -1004,18 +1028,13 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
 // Host side
 // --------------------------------------------------------------------------
 
-template <typename T>
-size_t threshold_smem_bytes(int wpc) {
-  return static_cast<size_t>(wpc) * WarpSmem<T>::kTotal;
-}
-
-template <typename T, int WPC>
+template <typename T, int WPC, int C>
 static cudaError_t launch_wpc(const CUtensorMap &map, const ThresholdLaunch &L,
                               cudaStream_t stream) {
-  const size_t smem = threshold_smem_bytes<T>(WPC);
+  const size_t smem = static_cast<size_t>(WPC) * WarpSmem<T, C>::kTotal;
   static bool configured = false; // per instantiation; setting it twice is harmless
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(threshold_kernel<T, WPC>,
+    cudaError_t e = cudaFuncSetAttribute(threshold_kernel<T, WPC, C>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess)
@@ -1042,18 +1061,20 @@ static cudaError_t launch_wpc(const CUtensorMap &map, const ThresholdLaunch &L,
     blocks = static_cast<uint32_t>(L.max_blocks);
   if (blocks == 0)
     return cudaSuccess;
-  threshold_kernel<T, WPC><<<blocks, WPC * 32, smem, stream>>>(map, a);
+  threshold_kernel<T, WPC, C><<<blocks, WPC * 32, smem, stream>>>(map, a);
   return cudaGetLastError();
 }
 
+// Of the widest strips; narrower ones fit as often.
 template <typename T, int WPC> static int occupancy_wpc() {
-  const size_t smem = threshold_smem_bytes<T>(WPC);
-  if (cudaFuncSetAttribute(threshold_kernel<T, WPC>,
+  constexpr int C = sizeof(T) == 2 ? 8 : 4;
+  const size_t smem = static_cast<size_t>(WPC) * WarpSmem<T, C>::kTotal;
+  if (cudaFuncSetAttribute(threshold_kernel<T, WPC, C>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return 0;
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, threshold_kernel<T, WPC>, WPC * 32,
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, threshold_kernel<T, WPC, C>, WPC * 32,
                                                     smem) != cudaSuccess)
     return 0;
   return n;
@@ -1068,23 +1089,32 @@ template <typename T> int threshold_occupancy(int wpc) {
   }
 }
 
+template <typename T, int C>
+static cudaError_t launch_cols(const CUtensorMap &map, const ThresholdLaunch &L,
+                               cudaStream_t stream) {
+  switch (L.warps_per_block) {
+  case 1: return launch_wpc<T, 1, C>(map, L, stream);
+  case 2: return launch_wpc<T, 2, C>(map, L, stream);
+  case 4: return launch_wpc<T, 4, C>(map, L, stream);
+  default: return cudaErrorInvalidValue;
+  }
+}
+
 template <typename T>
 cudaError_t launch_threshold(const CUtensorMap &map, const ThresholdLaunch &L,
                              cudaStream_t stream) {
-  switch (L.warps_per_block) {
-  case 1: return launch_wpc<T, 1>(map, L, stream);
-  case 2: return launch_wpc<T, 2>(map, L, stream);
-  case 4: return launch_wpc<T, 4>(map, L, stream);
-  default: return cudaErrorInvalidValue;
-  }
+  if (L.lane_cols == 4)
+    return launch_cols<T, 4>(map, L, stream);
+  if constexpr (sizeof(T) == 2)
+    if (L.lane_cols == 8)
+      return launch_cols<T, 8>(map, L, stream);
+  return cudaErrorInvalidValue;
 }
 
 template cudaError_t launch_threshold<uint16_t>(const CUtensorMap &, const ThresholdLaunch &,
                                                 cudaStream_t);
 template cudaError_t launch_threshold<uint32_t>(const CUtensorMap &, const ThresholdLaunch &,
                                                 cudaStream_t);
-template size_t threshold_smem_bytes<uint16_t>(int);
-template size_t threshold_smem_bytes<uint32_t>(int);
 template int threshold_occupancy<uint16_t>(int);
 template int threshold_occupancy<uint32_t>(int);
 

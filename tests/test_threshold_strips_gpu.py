@@ -51,3 +51,30 @@ def test_widths_around_strips(gpu_lib, dtype, widths, large):
                 assert got_status == (0 if found <= img.nbytes // 16 else -2)
                 if got_status == 0:
                     assert got.tobytes() == want.tobytes(), (shapes[f], warps)
+
+
+@pytest.mark.parametrize("large", [False, True])
+@pytest.mark.parametrize("w", [1, 3, 4, 5, 103, 104, 105, 127, 128, 129, 207, 208, 209, 384, 521])
+def test_narrow_strips_of_small_frames(gpu_lib, w, large):
+    """One small 16-bit frame: strips of 104 output columns, 4 a lane, where
+    the task height is not given; and the same frame with it given, in strips
+    of 232. Through sf_find too, which leaves it open."""
+    import dials_metal_spotfinder_b200 as sf
+    from dials_metal_spotfinder_b200.engine import Engine
+    for h in (1, 10, 67, 256):
+        img = edges(np.uint16, w, h, large)
+        _, want, found = O.dext(img)
+        fits = found <= img.nbytes // 16
+        for seg in (0, 4):
+            with Engine([(h, w)], np.uint16, seg_rows=seg) as eng:
+                info = eng.info()
+                strips = -(-w // (232 if seg else 104))
+                assert info["tasks"] == strips * -(-h // info["seg_rows"])
+                eng.upload(0, 0, img)
+                eng.run(0)
+                eng.synchronize()
+                status, got = eng.signal_status(0, 0)
+                assert status == (0 if fits else -2)
+                assert not fits or got.tobytes() == want.tobytes()
+        if fits:
+            assert sf.find(img).tobytes() == want.tobytes()
