@@ -98,3 +98,38 @@ def test_a_series_that_crosses_the_edge_both_ways(gpu_lib):
     check(signals)
     check(signals, frames=[2 * k + (k > 4) for k in range(len(sizes))])
     check(signals, two_d=True, min_spot_size=2, max_spot_size=9)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("nframes", [1, 3])
+def test_an_engine_small_enough(gpu_lib, nframes, graph):
+    """An engine whose lists and carry hold no more than the edge takes the
+    one-block launches too, replayed from graphs as well."""
+    from dials_metal_spotfinder_b200._lib import PIXEL, SPOT
+    from dials_metal_spotfinder_b200.engine import Engine
+    h, w, runs = 90, 110, 5
+    rng = np.random.default_rng(61)
+    frames = []
+    for _ in range(nframes * runs):
+        img = rng.poisson(1.0, (h, w)).astype(np.uint16)
+        for y, x in zip(rng.integers(2, h - 3, 12), rng.integers(2, w - 3, 12)):
+            img[y:y + 3, x:x + 3] += np.uint16(rng.integers(40, 900))
+        frames.append(img)
+    want = O.group([O.dext(f)[1] for f in frames], h, w)
+    spots, pixels = [], []
+    with Engine([(h, w)] * nframes, np.uint16) as eng:
+        eng.enable_grouping(carry_capacity=300)
+        eng.use_graph(graph)
+        for r in range(runs):
+            for f in range(nframes):
+                eng.upload(0, f, frames[r * nframes + f])
+            eng.run(0)
+            spots.append(eng.spots())
+            pixels.append(eng.pixels())
+        eng.finish()
+        spots.append(eng.spots())
+        pixels.append(eng.pixels())
+        counts, _ = eng.group_counts()
+    assert counts == want.counts
+    same_spots(np.concatenate(spots).astype(SPOT), want.spots)
+    assert np.concatenate(pixels).astype(PIXEL).tobytes() == want.pixels.tobytes()
