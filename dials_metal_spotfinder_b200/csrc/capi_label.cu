@@ -62,10 +62,10 @@ struct HostLabeller {
     }
   }
 
-  // Before a batch of `pixels`: whether its results will be in the head, if
-  // they fit there.
-  bool want_head(uint64_t pixels) {
-    if (!DeviceLabeller::takes_head(pixels))
+  // Before a batch: whether its results will be in the head, if they fit
+  // there.
+  bool want_head(uint64_t pixels, int nframes) {
+    if (!dev->one_block(pixels, nframes))
       return false;
     if (!head) {
       check(cudaMallocHost(&head, sizeof(LabelHead)), "cudaMallocHost");
@@ -114,7 +114,7 @@ struct HostLabeller {
     if (n)
       check(cudaMemcpyAsync(list, sig, n * sizeof(SignalPixel), cudaMemcpyHostToDevice, stream),
             "copying the signal list");
-    const bool in_head = want_head(carry + n);
+    const bool in_head = want_head(carry + n, 1);
     dev->enqueue_frame(frame, list, static_cast<uint32_t>(n), carry, stream);
     collect(in_head);
     started = true;
@@ -125,7 +125,7 @@ struct HostLabeller {
     if (!started)
       return;
     dev->reserve(1, 1, carry + 1, true);
-    const bool in_head = want_head(carry);
+    const bool in_head = want_head(carry, 0);
     dev->enqueue_rest(carry, stream);
     collect(in_head);
   }

@@ -69,12 +69,20 @@ constexpr int kThreads = kTileThreads;
 // launches with larger buffers.
 constexpr uint32_t kSmallCap = 256;
 constexpr uint32_t kMidCap = 512;
-// Batches of up to this many pixels, carried ones too, take the launches of
-// one block (lab_small_open, lab_small_close), where the host knows how many
-// there are: a frame added to a series and its results read took 186 us with
-// the launches of many and takes 124 at 1.1 k pixels, 143 at 2.6 k and 157 at
-// 3.2 k on average (their most 1.9 k, 4.4 k and 5.3 k); the two meet at 7 k.
+// Small batches take the launches of one block (lab_small_open,
+// lab_small_close), where the host knows how many pixels there are: up to
+// kSmallPixels of them, carried ones too. A frame added to a 256 x 384 or
+// 512 x 512 series and its results read takes 67 us against 130 with the
+// launches of many at 0.75 k pixels, 98 against 138 at 3.3 k; the two meet at 5
+// to 6 k (at 2.2 k where every few pixels are a spot of their own: 192 us
+// against 159 at 3 k).
+// The frames' block tables, a word per 64 pixels of their area, are cleared
+// and copied too, by the one block at 0.8 to 1.7 ns a word, so kSmallTable
+// words count as a pixel, which costs 18 to 53 ns. With the pixels alone in the
+// rule, 500 new pixels took 571 us a 4362 x 4148 frame (many blocks: 221), 197
+// a 2162 x 2068 one (153) and 135 at 1500 x 1500 (143).
 constexpr uint64_t kSmallPixels = 4096;
+constexpr uint64_t kSmallTable = 16;
 constexpr int kGatherFrames = 4; // see lab_gather
 // 32-position words a warp of lab_scatter takes at a time.
 constexpr int kScatterWords = 4;
@@ -1771,8 +1779,7 @@ DeviceLabeller::DeviceLabeller(int height, int width, const GroupOptions &option
   check(cudaStreamSynchronize(cudaStreamLegacy), "clearing labeller scalars");
 }
 
-// The streams beside the caller's, which only batches of more than kSmallPixels
-// need.
+// The streams beside the caller's, which only batches of many blocks need.
 void DeviceLabeller::create_streams() {
   if (join2_)
     return;
@@ -1969,7 +1976,9 @@ void DeviceLabeller::enqueue(int nframes, const SignalPixel *lists, const uint64
   enqueue_batch(b, s);
 }
 
-bool DeviceLabeller::takes_head(uint64_t pixels) { return pixels <= kSmallPixels; }
+bool DeviceLabeller::one_block(uint64_t pixels, int nframes) const {
+  return pixels + static_cast<uint64_t>(nframes) * nblk_ / kSmallTable <= kSmallPixels;
+}
 
 void DeviceLabeller::enqueue_frame(int64_t z, const SignalPixel *list, uint32_t count,
                                    uint64_t carried, cudaStream_t s) {
@@ -2059,7 +2068,7 @@ void DeviceLabeller::enqueue_batch(const Batch &b, cudaStream_t s) {
   a.report = report_;
   a.head = head_;
 
-  if (b.most <= kSmallPixels) {
+  if (one_block(b.most, nframes)) {
     lab_small_open<<<1, kThreads, 0, s>>>(a);
     lab_accept<kCompCap><<<grid_ / 8, kCompWarps * 32, kCompWarps * warp_comp_bytes<kCompCap>(),
                            s>>>(a, 0u, 0xffffffffu, 0);

@@ -131,9 +131,11 @@ public:
                      cudaStream_t s);
   // ... and for finishing what is left.
   void enqueue_rest(uint64_t carried, cudaStream_t s);
-  // Whether those two, with `pixels` carried and added, leave the batch's spots
-  // and pixels in the head that head_to() gave, as far as they fit there.
-  static bool takes_head(uint64_t pixels);
+  // Whether a batch of `nframes` frames with `pixels` pixels, carried and added,
+  // takes the launches of one block. Those of the two calls above leave the
+  // batch's spots and pixels in the head that head_to() gave, as far as they
+  // fit there.
+  bool one_block(uint64_t pixels, int nframes) const;
 
   // Sets batch_z0 for the next enqueue (an asynchronous copy from pinned
   // host memory; the labeller keeps the staging word until the next call).
