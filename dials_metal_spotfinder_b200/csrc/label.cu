@@ -89,8 +89,12 @@ constexpr int kScatterWords = 4;
 // The spots' scan packs pixels above rows, neither of which reaches 2^31.
 constexpr int kPackShift = 31;
 constexpr uint64_t kPackLow = (1ull << kPackShift) - 1;
-// The least a growing labeller makes room for: 16 Ki pixels, 3 MB.
+// The least batch a growing labeller makes room for, which with the carry's four
+// times as much is 16 MB (a pixel takes 195 bytes of buffers); and the most
+// room: the kRoomShare-th part of the memory that is free on the device, so that
+// what a labeller does not need yet is there for others.
 constexpr uint64_t kRoomPixels = 16384;
+constexpr uint64_t kRoomShare = 16;
 
 // Quotients by one divisor fixed for a whole launch (the frame width), by a
 // multiply-high and two shifts: Granlund and Montgomery, "Division by
@@ -1863,16 +1867,19 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
   batch_cap_ = carry_cap_ = live_cap_ = spot_cap_ = 0;
   frame_cap_ = 0;
   // With room: half as much again for the batch, a few such batches for the
-  // carry, and at least kRoomPixels, where that fits.
+  // carry (a series of noisy frames comes to hold five), and at least
+  // kRoomPixels, where that is within the share and fits.
   bool done = false;
   if (room) {
     const uint64_t rb = std::max<uint64_t>(
         bc, std::min(std::max(bc + bc / 2, kRoomPixels),
                      static_cast<uint64_t>(height_) * static_cast<uint64_t>(width_)));
     const uint64_t rc = std::max(2 * cc, 4 * rb);
-    done = rb + rc < 0x7fffffffull && allocate(rb, fc, rc);
+    size_t free_bytes = 0, total_bytes = 0;
+    check(cudaMemGetInfo(&free_bytes, &total_bytes), "cudaMemGetInfo");
+    done = rb + rc < 0x7fffffffull && allocate(rb, fc, rc, free_bytes / kRoomShare);
   }
-  if (!done && !allocate(bc, fc, cc))
+  if (!done && !allocate(bc, fc, cc, UINT64_MAX))
     throw DeviceError("CUDA: cudaMalloc labeller buffers: out of memory");
   if (host.carry_n) {
     const Live &c = live_[cur_];
@@ -1884,8 +1891,8 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
 }
 
 // The buffers for these capacities, in one allocation; false (and nothing
-// held) where it does not fit.
-bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
+// held) where that is more than `most` bytes or does not fit.
+bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc, uint64_t most) {
   const uint64_t live = bc + cc;
   const uint64_t nwmax = live / 32 + 1;
   const uint64_t spot_cap = live / opt_.min_spot_size + 1;
@@ -1934,6 +1941,8 @@ bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc) {
   uint64_t total = 0;
   for (const Part &q : parts)
     total += (q.bytes + 255) / 256 * 256;
+  if (total > most)
+    return false;
   if (cudaMalloc(reinterpret_cast<void **>(&arena_), total) != cudaSuccess) {
     cudaGetLastError();
     arena_ = nullptr;
