@@ -1841,11 +1841,15 @@ void DeviceLabeller::release() {
 
 void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t carry_pixels,
                              bool room) {
-  if (batch_pixels <= batch_cap_ && max_frames <= frame_cap_ && carry_pixels <= carry_cap_)
-    return;
-  const uint64_t bc = std::max(batch_pixels, batch_cap_);
+  // what it was ever asked for, which leaves out the room it was given with it
+  const uint64_t bc = std::max(batch_pixels, batch_asked_);
   const int fc = std::max(max_frames, frame_cap_);
-  const uint64_t cc = std::max(carry_pixels, carry_cap_);
+  const uint64_t cc = std::max(carry_pixels, carry_asked_);
+  if (batch_pixels <= batch_cap_ && max_frames <= frame_cap_ && carry_pixels <= carry_cap_) {
+    batch_asked_ = bc;
+    carry_asked_ = cc;
+    return;
+  }
   if (bc + cc >= 0x7fffffffull)
     throw std::invalid_argument("labelling batch too large");
   // Growing keeps the carry: copy it across after reallocating.
@@ -1881,6 +1885,8 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
   }
   if (!done && !allocate(bc, fc, cc, UINT64_MAX))
     throw DeviceError("CUDA: cudaMalloc labeller buffers: out of memory");
+  batch_asked_ = bc;
+  carry_asked_ = cc;
   if (host.carry_n) {
     const Live &c = live_[cur_];
     check(cudaMemcpy(c.frame, fr.data(), host.carry_n * 4, cudaMemcpyHostToDevice), "carry");

@@ -185,6 +185,7 @@ private:
   unsigned char *arena_ = nullptr; // every buffer below but the scalars and the carry's table
 
   uint64_t batch_cap_ = 0, carry_cap_ = 0, live_cap_ = 0, spot_cap_ = 0;
+  uint64_t batch_asked_ = 0, carry_asked_ = 0; // of the capacities: what reserve() was asked for
   int frame_cap_ = 0;
   int cur_ = 0; // which live buffer holds the carry
 

@@ -42,3 +42,22 @@ def test_room_is_a_share_of_the_free_memory(gpu_lib):
     counts = lab.counts()
     lab.close()
     assert counts["signal_pixels"] == counts["groups"] == counts["too_small"] == n
+
+
+def test_room_is_not_asked_for_again(gpu_lib):
+    """Where a batch leaves no room, the labeller grows to what it was asked
+    for, not to that and the room it once had."""
+    from dials_metal_spotfinder_b200.labeller import Labeller
+    first, second = SIDE * SIDE // 16, SIDE * SIDE // 4
+    free = free_bytes()
+    if 7.5 * second * (BYTES - 20) < free / 16 or 7.5 * first * BYTES > free / 16:
+        pytest.skip("a device on which both batches have room, or neither")
+    lab = Labeller(SIDE, SIDE)
+    lab.add(0, lone(first))
+    lab.add(1, lone(second))
+    used = free - free_bytes()
+    assert lab.live() == first + second  # joined across the frames, or new
+    assert used < (first + second) * BYTES + second * LIST + (64 << 20)
+    lab.finish()
+    assert lab.counts()["groups"] == second
+    lab.close()
