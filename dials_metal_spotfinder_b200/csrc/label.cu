@@ -92,9 +92,12 @@ constexpr uint64_t kPackLow = (1ull << kPackShift) - 1;
 // The least batch a growing labeller makes room for, which with the carry's four
 // times as much is 16 MB (a pixel takes 195 bytes of buffers); and the most
 // room: the kRoomShare-th part of the memory that is free on the device, so that
-// what a labeller does not need yet is there for others.
+// what a labeller does not need yet is there for others. Buffers of up to
+// kRoomAlways bytes are not held against that (asking for what is free costs a
+// small series 40 of its 2550 us).
 constexpr uint64_t kRoomPixels = 16384;
 constexpr uint64_t kRoomShare = 16;
+constexpr uint64_t kRoomAlways = 64 << 20;
 
 // Quotients by one divisor fixed for a whole launch (the frame width), by a
 // multiply-high and two shifts: Granlund and Montgomery, "Division by
@@ -1879,11 +1882,9 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
         bc, std::min(std::max(bc + bc / 2, kRoomPixels),
                      static_cast<uint64_t>(height_) * static_cast<uint64_t>(width_)));
     const uint64_t rc = std::max(2 * cc, 4 * rb);
-    size_t free_bytes = 0, total_bytes = 0;
-    check(cudaMemGetInfo(&free_bytes, &total_bytes), "cudaMemGetInfo");
-    done = rb + rc < 0x7fffffffull && allocate(rb, fc, rc, free_bytes / kRoomShare);
+    done = rb + rc < 0x7fffffffull && allocate(rb, fc, rc, true);
   }
-  if (!done && !allocate(bc, fc, cc, UINT64_MAX))
+  if (!done && !allocate(bc, fc, cc, false))
     throw DeviceError("CUDA: cudaMalloc labeller buffers: out of memory");
   batch_asked_ = bc;
   carry_asked_ = cc;
@@ -1897,8 +1898,8 @@ void DeviceLabeller::reserve(uint64_t batch_pixels, int max_frames, uint64_t car
 }
 
 // The buffers for these capacities, in one allocation; false (and nothing
-// held) where that is more than `most` bytes or does not fit.
-bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc, uint64_t most) {
+// held) where it does not fit or, with `share`, is past kRoomShare's part.
+bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc, bool share) {
   const uint64_t live = bc + cc;
   const uint64_t nwmax = live / 32 + 1;
   const uint64_t spot_cap = live / opt_.min_spot_size + 1;
@@ -1947,8 +1948,12 @@ bool DeviceLabeller::allocate(uint64_t bc, int fc, uint64_t cc, uint64_t most) {
   uint64_t total = 0;
   for (const Part &q : parts)
     total += (q.bytes + 255) / 256 * 256;
-  if (total > most)
-    return false;
+  if (share && total > kRoomAlways) {
+    size_t free_bytes = 0, all_bytes = 0;
+    check(cudaMemGetInfo(&free_bytes, &all_bytes), "cudaMemGetInfo");
+    if (total > free_bytes / kRoomShare)
+      return false;
+  }
   if (cudaMalloc(reinterpret_cast<void **>(&arena_), total) != cudaSuccess) {
     cudaGetLastError();
     arena_ = nullptr;

@@ -177,7 +177,7 @@ private:
   void enqueue_batch(const Batch &b, cudaStream_t s);
   void create_streams();
   void release();
-  bool allocate(uint64_t batch_pixels, int frames, uint64_t carry_pixels, uint64_t most);
+  bool allocate(uint64_t batch_pixels, int frames, uint64_t carry_pixels, bool share);
 
   int height_, width_;
   GroupOptions opt_;

@@ -1,5 +1,5 @@
 """How much device memory a labeller takes for pixels it has not been given
-yet: never more than a sixteenth of what is free."""
+yet: never more than a sixteenth of what is free, small buffers aside."""
 
 import numpy as np
 import pytest
