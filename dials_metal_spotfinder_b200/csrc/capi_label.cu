@@ -78,7 +78,7 @@ struct HostLabeller {
     check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     const LabelScalars &sc = *host_sc;
     if (sc.status != kLabelOk)
-      throw DeviceError("labeller capacity exceeded (status " + std::to_string(sc.status) + ")");
+      throw DeviceError(label_error("labeller", sc.status));
     const uint64_t ns = sc.batch_spots, np = sc.batch_pixels;
     if (in_head && ns <= LabelHead::kSpots && np <= LabelHead::kPixels) {
       spots.insert(spots.end(), head->spots, head->spots + ns);

@@ -47,11 +47,12 @@ struct ServerSeries;
 // What a run leaves for the host, in page-locked memory the device writes.
 struct SinkHeader {
   uint32_t nsig;      // the frame's signal pixels
-  int32_t status;     // 0, or what failed (kSink* bits)
+  int32_t status;     // 0, or what failed (kSink* bits, and the labeller's status above them)
   uint64_t nspots, npixels;
   uint64_t counts[6]; // running grouping counts
 };
 enum : int32_t { kSinkPlan = 1, kSinkDecode = 2, kSinkLabel = 4, kSinkOverflow = 8 };
+constexpr int kSinkLabelShift = 8;
 
 struct SlotState {
   ServerSeries *series = nullptr;
@@ -81,7 +82,7 @@ __global__ void sink_results(const LabelScalars *sc, const Spot *spots, const Pi
     if (decode_err && *decode_err)
       st |= kSinkDecode;
     if (sc->status)
-      st |= kSinkLabel;
+      st |= kSinkLabel | sc->status << kSinkLabelShift;
     if (ns > cap_spots || np > cap_pixels)
       st |= kSinkOverflow;
     sink->nsig = frame_count[0];
@@ -456,7 +457,7 @@ struct Server {
                              std::to_string(se.cap_spots) + ", " + std::to_string(se.cap_pixels) +
                              ")"
                    : h.status & kSinkDecode ? "an uploaded chunk held a malformed LZ4 block"
-                   : h.status & kSinkLabel  ? "grouping capacity exceeded"
+                   : h.status & kSinkLabel  ? label_error("grouping", h.status >> kSinkLabelShift)
                                             : "a threshold wait gave up";
       if (!h.status) {
         for (const Spot &s : sp) {

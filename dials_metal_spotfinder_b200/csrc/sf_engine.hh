@@ -385,7 +385,7 @@ struct Engine {
     check(cudaStreamSynchronize(group), "cudaStreamSynchronize");
     const LabelScalars &sc = host_sc[k];
     if (sc.status != kLabelOk)
-      throw DeviceError("grouping capacity exceeded (status " + std::to_string(sc.status) + ")");
+      throw DeviceError(label_error("grouping", sc.status));
     return sc;
   }
 

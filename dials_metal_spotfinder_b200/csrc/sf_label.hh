@@ -78,6 +78,12 @@ enum : int32_t {
   kLabelSpotOverflow = 2,
   kLabelWaitTimeout = 3, // a tile's wait for the tiles before it gave up
 };
+// What to tell the caller of `what` ("grouping") that ended with a status.
+inline std::string label_error(const char *what, int32_t status) {
+  return what + std::string(status == kLabelWaitTimeout ? ": a wait on the device gave up"
+                                                        : " capacity exceeded") +
+         " (status " + std::to_string(status) + ")";
+}
 
 // Page-locked host memory in which a small batch leaves its results, so that
 // the host has them with its scalars, without copies of their own (two of them
