@@ -322,18 +322,19 @@ void *ThresholdPlan::frame_origin(int slot, int f) const {
 }
 
 bool ThresholdPlan::linear_copy() {
-  if (!linear_) {
+  if (!linear_ && !linear_refused_) {
     uint64_t most = 0;
     for (const Shape &s : shapes_)
       most = std::max(most, static_cast<uint64_t>(s.height) * s.width * elem_bytes_);
     if (cudaMalloc(&linear_, most) != cudaSuccess) {
-      cudaGetLastError(); // no room: the pitched copy needs none
+      cudaGetLastError(); // no room: the pitched copy needs none, of this plan's frames
       linear_ = nullptr;
+      linear_refused_ = true;
       return false;
     }
     device_bytes_ += most;
   }
-  return true;
+  return linear_ != nullptr;
 }
 
 void ThresholdPlan::upload(int slot, int f, const void *host, cudaStream_t stream) {

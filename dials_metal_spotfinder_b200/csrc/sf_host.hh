@@ -208,6 +208,7 @@ private:
   uint32_t *tile_start_ = nullptr;
   SignalPixel *pool_ = nullptr;
   uint8_t *linear_ = nullptr; // upload()'s contiguous copy
+  bool linear_refused_ = false; // there was no room for it
 };
 
 // The cost model's task height (plan.cu) for these shapes at `wpc` warps per
