@@ -57,9 +57,15 @@ uint64_t round_up(uint64_t v, uint64_t m) { return (v + m - 1) / m * m; }
 //
 // Strips of 4 columns a lane have 2.2 times the tasks of 8, but a row of theirs
 // takes 8.2 + 0.4 w units, no less than 9.5: a small frame, whose warps have an
-// SM's schedulers nearly to themselves, is done sooner (256 x 384 uint16
-// 25 -> 22 us, 700 x 900 30 -> 28, 1062 x 1028 34.5 -> 32.5; 2162 x 2068 would
-// take 51 for 48). The two costs decide.
+// SM's schedulers nearly to themselves, is done sooner. Between the two forms
+// the costs are not quite alike: over 40 shapes of one to 64 frames, both
+// forms timed at their best heights, strips of 4 were the slower only above 1.07
+// times the cost of 8 (wide, narrow us: 256 x 384 uint16 25.9, 24.2; 700 x 900
+// 32.5, 28.1 at 1.03 times; 1062 x 1028 34.9, 30.8 at 1.06; 64 frames of
+// 128 x 128 38.7, 40.9 at 1.07; 32 of 256 x 384 47.0, 48.9 at 1.09; 1500 x 1500
+// 40.7, 42.9 at 1.13; 2162 x 2068 49.3, 53.7 at 1.18), so they are taken up
+// to there.
+constexpr uint64_t kNarrowPercent = 107;
 struct Heights {
   int rows;
   uint64_t cost; // tenths of a unit
@@ -181,7 +187,7 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
     Heights h = choose_seg_rows(elem_bytes, lane_cols_, shapes, sms, wpc, per_sm);
     if (elem_bytes == 2) {
       const Heights narrow = choose_seg_rows(elem_bytes, 4, shapes, sms, wpc, per_sm);
-      if (narrow.cost < h.cost) {
+      if (100 * narrow.cost < kNarrowPercent * h.cost) {
         h = narrow;
         lane_cols_ = 4;
       }
