@@ -19,8 +19,8 @@
 //      previous batch's grouping kernels, which run beside it on the other
 //      stream, instead of holding them until it ends.
 //
-// The tuner file holds one line per (pixel bytes, height, width, SM count,
-// device name): frames per launch, warps per block, the task-height ratio,
+// The tuner file holds one line per (kernel version, pixel bytes, height, width,
+// SM count, device name): frames per launch, warps per block, the task-height ratio,
 // the measured time per frame. Results never depend on the tuning (every
 // tuple gives byte-identical lists); only the time does.
 
@@ -56,9 +56,15 @@ std::string device_name() {
   return s;
 }
 
+// What the entries were measured with: a new number for a change of the
+// threshold or of the model that the ratios are relative to, so that entries
+// from before it are not read (one for 32-bit pixels could hold a kernel that
+// fits 16 warps an SM to the 8 that the one before it fitted).
+constexpr int kThresholdVersion = 2;
+
 std::string make_key(int elem_bytes, int height, int width) {
   std::ostringstream k;
-  k << "u" << 8 * elem_bytes << ":" << height << "x" << width << ":sm" << device_sm_count()
+  k << "k" << kThresholdVersion << ":u" << 8 * elem_bytes << ":" << height << "x" << width << ":sm" << device_sm_count()
     << ":" << device_name();
   return k.str();
 }

@@ -318,8 +318,8 @@ SF_API int sf_engine_stage_totals(sf_engine *engine, double out4[4]);
  * leave room on every SM for the grouping running beside it), on the
  * caller's sample frames (host, row-major, cycled into the
  * batches), with CUDA events. The best tuple is appended to a tuner file,
- * keyed by pixel type, shape, SM count and device name; engines created
- * without explicit tuning read it. Results never depend on the tuning, only
+ * keyed by kernel version, pixel type, shape, SM count and device name;
+ * engines created without explicit tuning read it. Results never depend on the tuning, only
  * the time does. The reference chooses its stage windows by measurement
  * the same way (src/dext_gpu.cc:18-37, tests/bench_dext_gpu.cc:242-337). */
 typedef struct sf_tune_options {
