@@ -94,12 +94,9 @@ int sf_engine_create(int elem_bytes, int nframes, const int32_t *heights,
     const bool from_cache = automatic && uniform &&
                             sf::tune_lookup(elem_bytes, shapes[0].height, shapes[0].width,
                                             nullptr, &tuned);
-    if (from_cache) {
-      t.warps_per_block = tuned.warps_per_block;
-      t.blocks_per_sm = tuned.blocks_per_sm;
-      t.seg_rows = sf::tune_seg_rows(elem_bytes, shapes, tuned.warps_per_block, tuned.seg_ratio,
-                                     tuned.blocks_per_sm);
-    }
+    if (from_cache)
+      t = sf::tuned_plan(elem_bytes, shapes, tuned.warps_per_block, tuned.seg_ratio,
+                         tuned.blocks_per_sm);
     auto e = sf::make_engine(elem_bytes, shapes, t, slots);
     e->tuned_from_cache = from_cache;
     *out = reinterpret_cast<sf_engine *>(e.release());

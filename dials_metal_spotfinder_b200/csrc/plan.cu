@@ -102,19 +102,31 @@ Heights choose_seg_rows(int elem_bytes, int lane_cols,
   return best;
 }
 
+// The form and height of a batch's tasks.
+TaskShape choose_task(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
+                      int blocks_per_sm) {
+  const uint64_t sms = static_cast<uint64_t>(device_sm_count());
+  const int wide = elem_bytes == 2 ? 8 : 4;
+  const Heights h = choose_seg_rows(elem_bytes, wide, shapes, sms, wpc, blocks_per_sm);
+  if (elem_bytes == 2) {
+    const Heights narrow = choose_seg_rows(elem_bytes, 4, shapes, sms, wpc, blocks_per_sm);
+    if (100 * narrow.cost < kNarrowPercent * h.cost)
+      return TaskShape{narrow.rows, 4};
+  }
+  return TaskShape{h.rows, wide};
+}
+
 } // namespace
 
-int model_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
-                   int blocks_per_sm) {
+TaskShape model_task(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
+                     int blocks_per_sm) {
   int occ = elem_bytes == 2 ? threshold_occupancy<uint16_t>(wpc)
                             : threshold_occupancy<uint32_t>(wpc);
   if (occ < 1)
     throw DeviceError("the threshold kernel does not fit on this device");
   if (blocks_per_sm > 0)
     occ = std::min(occ, blocks_per_sm);
-  return choose_seg_rows(elem_bytes, elem_bytes == 2 ? 8 : 4, shapes,
-                         static_cast<uint64_t>(device_sm_count()), wpc, occ)
-      .rows;
+  return choose_task(elem_bytes, shapes, wpc, occ);
 }
 
 void encode_arena_map(CUtensorMap *map, void *base, int elem_bytes, uint64_t pitch_elems,
@@ -181,19 +193,12 @@ ThresholdPlan::ThresholdPlan(int elem_bytes, const std::vector<Shape> &shapes,
   const int per_sm = tuning_.blocks_per_sm > 0 ? std::min(tuning_.blocks_per_sm, occ) : occ;
   sms_ = device_sm_count();
   max_blocks_ = sms_ * per_sm;
-  lane_cols_ = elem_bytes == 2 ? 8 : 4;
   if (tuning_.seg_rows <= 0) {
-    const uint64_t sms = static_cast<uint64_t>(sms_);
-    Heights h = choose_seg_rows(elem_bytes, lane_cols_, shapes, sms, wpc, per_sm);
-    if (elem_bytes == 2) {
-      const Heights narrow = choose_seg_rows(elem_bytes, 4, shapes, sms, wpc, per_sm);
-      if (100 * narrow.cost < kNarrowPercent * h.cost) {
-        h = narrow;
-        lane_cols_ = 4;
-      }
-    }
-    tuning_.seg_rows = h.rows;
+    const TaskShape t = choose_task(elem_bytes, shapes, wpc, per_sm);
+    tuning_.seg_rows = t.rows;
+    tuning_.lane_cols = t.lane_cols;
   }
+  lane_cols_ = tuning_.lane_cols == 4 || elem_bytes != 2 ? 4 : 8;
 
   const int out_cols = strip_out(elem_bytes, lane_cols_);
   int32_t max_strips = 0;

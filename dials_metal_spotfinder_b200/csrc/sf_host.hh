@@ -111,7 +111,8 @@ cudaStream_t create_stream(int rank);
 
 // Launch geometry of the threshold for one batch shape.
 struct PlanTuning {
-  int seg_rows = 0;        // output rows per task; 0 picks by frame count
+  int seg_rows = 0;        // output rows per task; 0 picks them and lane_cols by the cost model
+  int lane_cols = 0;       // with seg_rows, for 16-bit pixels: 4 for narrow strips, else wide ones
   int warps_per_block = 0; // 1, 2 or 4; 0: 2
   int blocks_per_sm = 0;   // 0: as many as fit
 };
@@ -211,10 +212,13 @@ private:
   bool linear_refused_ = false; // there was no room for it
 };
 
-// The cost model's task height (plan.cu) for these shapes at `wpc` warps per
-// block and as many blocks per SM as fit.
-int model_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
-                   int blocks_per_sm = 0);
+// The tasks of the cost model (plan.cu) for these shapes at `wpc` warps per
+// block and as many blocks per SM as fit: their height and columns a lane.
+struct TaskShape {
+  int rows, lane_cols;
+};
+TaskShape model_task(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
+                     int blocks_per_sm = 0);
 
 // The autotuner (tune.cu). An entry is what a search measured best for one
 // frame shape on one kind of device: frames per launch, warps per block, the
@@ -239,8 +243,9 @@ struct TuneResult {
 };
 std::string tune_cache_path(const char *given);
 bool tune_lookup(int elem_bytes, int height, int width, const char *cache_path, TuneEntry *out);
-int tune_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
-                  double ratio, int blocks_per_sm = 0);
+// What a batch of these shapes runs with by an entry.
+PlanTuning tuned_plan(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
+                      double ratio, int blocks_per_sm = 0);
 TuneResult tune_search(int elem_bytes, int height, int width, const void *const *sample,
                        int nsample, const TuneOptions &options);
 

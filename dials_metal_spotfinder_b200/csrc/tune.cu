@@ -163,14 +163,23 @@ bool tune_lookup(int elem_bytes, int height, int width, const char *cache_path,
   return read_entry(tune_cache_path(cache_path), make_key(elem_bytes, height, width), out);
 }
 
-int tune_seg_rows(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
-                  double ratio, int blocks_per_sm) {
-  const int base = model_seg_rows(elem_bytes, shapes, wpc, blocks_per_sm);
+// The model's tasks for these shapes, their height times the ratio: at a ratio
+// of 1 what an untuned engine of as many warps a block runs with. (Heights
+// below 16 rows are half halo and more: a ratio goes there only from a model's
+// height that is there already.)
+PlanTuning tuned_plan(int elem_bytes, const std::vector<ThresholdPlan::Shape> &shapes, int wpc,
+                      double ratio, int blocks_per_sm) {
+  const TaskShape base = model_task(elem_bytes, shapes, wpc, blocks_per_sm);
   int max_h = 1;
   for (const auto &s : shapes)
     max_h = std::max(max_h, s.height);
-  const int seg = static_cast<int>(std::lround(base * ratio));
-  return std::max(16, std::min(seg, max_h));
+  const int seg = static_cast<int>(std::lround(base.rows * ratio));
+  PlanTuning t;
+  t.warps_per_block = wpc;
+  t.blocks_per_sm = blocks_per_sm;
+  t.seg_rows = std::max(std::min(16, base.rows), std::min(seg, max_h));
+  t.lane_cols = base.lane_cols;
+  return t;
 }
 
 TuneResult tune_search(int elem_bytes, int height, int width, const void *const *sample,
@@ -203,9 +212,7 @@ TuneResult tune_search(int elem_bytes, int height, int width, const void *const 
       continue;
     int last_seg = -1;
     for (double ratio : {0.5, 0.75, 1.0, 1.5, 2.0}) {
-      PlanTuning t;
-      t.warps_per_block = wpc;
-      t.seg_rows = tune_seg_rows(elem_bytes, shapes1, wpc, ratio);
+      const PlanTuning t = tuned_plan(elem_bytes, shapes1, wpc, ratio);
       if (t.seg_rows == last_seg)
         continue;
       last_seg = t.seg_rows;
@@ -228,9 +235,7 @@ TuneResult tune_search(int elem_bytes, int height, int width, const void *const 
         engine_bytes(elem_bytes, height, width, F) > budget)
       continue;
     const std::vector<ThresholdPlan::Shape> shapes(F, ThresholdPlan::Shape{height, width});
-    PlanTuning t;
-    t.warps_per_block = best_wpc;
-    t.seg_rows = tune_seg_rows(elem_bytes, shapes, best_wpc, best_ratio);
+    const PlanTuning t = tuned_plan(elem_bytes, shapes, best_wpc, best_ratio);
     const double ms =
         time_engine(elem_bytes, height, width, F, t, o.grouping, sample, nsample, o.steps);
     r.candidates++;
@@ -254,10 +259,7 @@ TuneResult tune_search(int elem_bytes, int height, int width, const void *const 
       if (bps < 1 || bps >= last)
         continue;
       last = bps;
-      PlanTuning t;
-      t.warps_per_block = best_wpc;
-      t.blocks_per_sm = bps;
-      t.seg_rows = tune_seg_rows(elem_bytes, shapes, best_wpc, best_ratio, bps);
+      const PlanTuning t = tuned_plan(elem_bytes, shapes, best_wpc, best_ratio, bps);
       const double ms = time_engine(elem_bytes, height, width, best_f, t, o.grouping, sample,
                                     nsample, o.steps);
       r.candidates++;
@@ -308,8 +310,9 @@ extern "C" int sf_tune(int elem_bytes, int height, int width, const void *const 
         r.entry.frames, sf::ThresholdPlan::Shape{height, width});
     out->frames_per_launch = r.entry.frames;
     out->warps_per_block = r.entry.warps_per_block;
-    out->seg_rows = sf::tune_seg_rows(elem_bytes, shapes, r.entry.warps_per_block,
-                                      r.entry.seg_ratio, r.entry.blocks_per_sm);
+    out->seg_rows = sf::tuned_plan(elem_bytes, shapes, r.entry.warps_per_block,
+                                   r.entry.seg_ratio, r.entry.blocks_per_sm)
+                        .seg_rows;
     out->blocks_per_sm = r.entry.blocks_per_sm;
     out->from_cache = r.from_cache ? 1 : 0;
     out->candidates = r.candidates;
