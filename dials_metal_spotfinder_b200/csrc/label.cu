@@ -83,7 +83,7 @@ constexpr uint32_t kMidCap = 512;
 // a 2162 x 2068 one (153) and 135 at 1500 x 1500 (143).
 constexpr uint64_t kSmallPixels = 4096;
 constexpr uint64_t kSmallTable = 16;
-constexpr int kGatherFrames = 4; // see lab_gather
+constexpr uint64_t kGatherArea = 1 << 24; // see lab_gather
 // 32-position words a warp of lab_scatter takes at a time.
 constexpr int kScatterWords = 4;
 // The spots' scan packs pixels above rows, neither of which reaches 2^31.
@@ -390,9 +390,12 @@ __device__ __forceinline__ const uint32_t *table_of(const LabArgs &a, int s, int
 // joined by lab_link at the chunk's first position.
 // A warp takes kGatherWords chunks at a time, all their records read before
 // any is used. Four: a quarter of the run list's claims, block-wide waits and
-// segment lookups (16 frames of 4362 x 4148 142 -> 133 us for 460 MB moved); one
-// for batches of fewer than kGatherFrames frames, which four leave with too
-// few warps (one frame of 2162 x 2068 11 us; 13 with four).
+// segment lookups (16 frames of 4362 x 4148 142 -> 133 us for 460 MB moved). One
+// where four would leave too few warps, which is a matter of pixels, and they
+// of the frames' area, all that the host knows: the grouping of 8 frames of
+// 256 x 384 takes 104 us with one and 109 with four, of 16 of 2162 x 2068 408
+// and 388; from 4 Mi to 18 Mi frame pixels the two are within 1 %. And one for
+// a single frame (2162 x 2068 11 us, 13 with four; 4362 x 4148 the same).
 template <int kGatherWords>
 __device__ __forceinline__ void gather_step(const LabArgs &a) {
   LabelScalars *sc = a.sc;
@@ -2101,7 +2104,7 @@ void DeviceLabeller::enqueue_batch(const Batch &b, cudaStream_t s) {
   const unsigned grid = grid_;
   LabelScalars *sc = sc_;
   lab_setup<<<grid, kThreads, 0, s>>>(a);
-  if (nframes >= kGatherFrames)
+  if (nframes > 1 && static_cast<uint64_t>(nframes) * height_ * width_ >= kGatherArea)
     lab_gather<4><<<grid, kThreads, 0, s>>>(a);
   else
     lab_gather<1><<<grid, kThreads, 0, s>>>(a);
