@@ -33,11 +33,12 @@
 //
 // Bound: instruction issue (2.7 of 4 a cycle) and the integer pipe (74 % busy)
 // at the 16 warps an SM holds for 16-bit pixels; 4362 x 4148 uint16 takes
-// 56 us a frame in a batch, 810 GB/s of its own bytes. Integer work is
+// 55 us a frame in a batch, 850 GB/s of its own bytes. Integer work is
 // therefore moved or saved where that costs no more instructions: low halves
 // by a multiply-add, float bits formed by the sums themselves, what the
 // 11-row sums leave out selected before the addition instead of corrected
-// after it, one masked test a pair of rows (956 -> 897 us for 16 frames). Not
+// after it, one masked test a pair of rows (956 -> 899 us for 16 frames, and
+// 882 since). Not
 // kept: high halves by a high multiply (927), and additions as multiply-adds
 // in the vertical (926) or the horizontal sums (910), which cost two each.
 // 32-bit pixels: 8 columns a lane take 220 registers, which leaves an SM 8
@@ -326,7 +327,7 @@ __device__ __forceinline__ uint64_t shfl_down(uint64_t v) {
 }
 
 // Horizontal sums of width 2R+1 over the lane's C columns, given the lane's
-// own vertical sums v[0..8) and the neighbouring lanes' by shuffle. The edge
+// own vertical sums v[0..C) and the neighbouring lanes' by shuffle. The edge
 // lanes see no neighbour; their edge columns are halo and never used.
 template <int R, int C, typename A>
 __device__ __forceinline__ void hsum(const A (&v)[C], A (&h)[C], A from = 0) {
@@ -430,7 +431,7 @@ __device__ __forceinline__ int find_frame(const FrameDesc *frames, int n,
 // Warps of equal tasks do not finish together (an SM's schedulers favour
 // some, strips differ in masked columns and candidates): without this, 12.9
 // of the 16 warps an SM holds were active on average, and 16 frames of
-// 4362 x 4148 uint16 took 1104 us (958 with it), 16 of 2162 x 2068 327 (304),
+// 4362 x 4148 uint16 took 1104 us (956 with it), 16 of 2162 x 2068 327 (304),
 // 8 of 4362 x 4148 uint32, then 8 warps an SM, 1103 (995). Halves down to kLeastShare rows are
 // worth the 20 rows of halo they cost again: at least 64 gave 976 and 329
 // us, 24 the same as 32; claims of 8 rows the same as of 16.
@@ -628,7 +629,8 @@ __global__ void __launch_bounds__(WPC * 32, kWarpsPerSm / WPC)
     const int32_t tma_x = strip * kOut;
     const int64_t tma_y0 = fd.row0 + rs;
 
-    // Output columns of this lane: ring columns [10, 242) inside the frame.
+    // Output columns of this lane: ring columns [kHalo, kHalo + kOut) inside the
+    // frame.
     uint32_t outmask = 0;
 #pragma unroll
     for (int k = 0; k < C; k++) {
